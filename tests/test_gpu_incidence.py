@@ -306,3 +306,34 @@ def test_role_bit_form_against_the_oracle(d, n_univ, monkeypatch):
                 probe = rng.choice(n_cand, 53)
                 assert np.array_equal(b.ball_gather(probe, t),
                                       o.ball_gather(probe, t)), (step, t)
+
+
+@pytest.mark.parametrize("v,k,t", [(24, 6, 3), (18, 9, 4), (20, 12, 2),
+                                   (23, 4, 3), (17, 16, 5), (26, 7, 1),
+                                   (19, 18, 2), (14, 7, 7)])
+def test_design_fields_by_levels_against_the_rows(v, k, t):
+    """A design's fields equal the same rows served as explicit incidence:
+    one level and many, byte and 16-bit levels, more block than half the
+    points, sizes that end inside a run, and the sizes the row form keeps."""
+    from coldcore_b200.incidence import GpuCoveringDesignBackend
+    with GpuCoveringDesignBackend(v, k, t, mu=2) as b:
+        rows = b.rows()
+        rng = np.random.default_rng(v)
+        sols = [rng.choice(b.n_cand, m, replace=False)
+                for m in (0, min(40, b.n_cand // 3))]
+        got = []
+        for sol in sols:
+            b.recount(sol)
+            for fld in (b.gain_map, b.loss_map):
+                fld()
+                got.append(b.map_all())
+        n_univ = b.n_univ
+    o = IncidenceOracle(rows, n_univ, mu=2)
+    want = []
+    for sol in sols:
+        o.recount(sol)
+        for fld in (o.gain_map, o.loss_map):
+            fld()
+            want.append(o.map.copy())
+    for a, w in zip(got, want):
+        assert np.array_equal(a, w)
