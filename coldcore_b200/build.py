@@ -46,6 +46,7 @@ def build(verbose=False, extra=()):
     os.makedirs(OBJ, exist_ok=True)
     srcs = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
     headers = sorted(glob.glob(os.path.join(CSRC, "*.h")) +
+                     glob.glob(os.path.join(CSRC, "*.cuh")) +
                      glob.glob(os.path.join(ROOT, "include", "*", "*.h")))
     with concurrent.futures.ThreadPoolExecutor(len(srcs)) as ex:
         res = list(ex.map(lambda s: _compile(s, headers, list(extra)), srcs))

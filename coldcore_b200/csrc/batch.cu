@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstring>
+#include <map>
 #include <unordered_map>
 #include <vector>
 
@@ -39,6 +40,8 @@ struct Cell {
   long long *dcode = nullptr, *bounds = nullptr;
   long long nbounds = 0;
   int first_pass = 0, npass = 0;     // global pass range (small cells)
+  int kid = -1;                      // register kernel of a small cell's passes
+  bool regs = false;                 // one axis size, with a register kernel
   bool big = false;                  // own register-blocked launches
   int side = 0;                      // its side stream (big cells)
   bool tuned = false;                // fast[] tuned (big cells)
@@ -80,15 +83,18 @@ __global__ void k_batch_bounds(const BoundsJob *jobs) {
 // register-blocked kernel run as their own launches (captured on forked
 // streams of the same graph); smaller cells share the persistent kernel.
 // (CC_BATCH_BIG: log2 of that threshold; CC_BATCH_ITEM: the words of one
-// work item of the persistent kernel, at least)
+// work item of the persistent kernels, at least)
 long long big_cell_words() {
   const char *e = getenv("CC_BATCH_BIG");
   const int lg = e ? atoi(e) : 16;
   return 1LL << (lg < 8 ? 8 : lg > 40 ? 40 : lg);
 }
-long long item_words() {
+// (register kernels: a step of 256 cells of 10^3..10^5 words took 0.95 ms
+// with items of 2,048 words, 0.99 with 4,096, 1.33 with 8,192, 1.89 with
+// 16,384: one tile an item keeps the most CTAs busy)
+long long item_words(bool regs) {
   const char *e = getenv("CC_BATCH_ITEM");
-  const long long w = e ? atoll(e) : 32768;
+  const long long w = e ? atoll(e) : regs ? 2048 : 32768;
   return w < 256 ? 256 : w;
 }
 // side streams the big cells are spread over (CC_BATCH_STREAMS, 1..16,
@@ -101,17 +107,30 @@ int side_streams() {
   return n < 1 ? 1 : n > kSideStreams ? kSideStreams : n;
 }
 
+// one persistent launch: the small cells one kernel serves (kid -1: the
+// runtime-size tiles)
+struct Group {
+  int kid = -1;
+  long long item0 = 0, nitems = 0;   // its range of the item table
+  size_t smem = 0;
+  int grid = 1;
+  int side = -1;                     // side stream, -1 the main stream
+};
+
 struct Batch {
   std::vector<Cell> cells;
   bool built = false;
   char *arena = nullptr;
   size_t arena_bytes = 0;
-  std::vector<GroupArgs> passes;
+  std::vector<GroupPlan> passes;
   std::vector<int> dep;
   std::vector<unsigned> need;
+  std::vector<int> pass_cell;
+  std::vector<Group> groups;         // persistent launches, one a kernel
   GroupArgs *d_passes = nullptr;
   int *d_dep = nullptr;
   unsigned *d_need = nullptr;
+  int *d_pass_cell = nullptr;
   int4 *d_items = nullptr;
   long long nitems = 0;
   unsigned *d_done = nullptr;
@@ -130,7 +149,6 @@ struct Batch {
   long long ext_cap = 0;
   long long *d_count = nullptr;
   size_t tile_budget = 48 * 1024;
-  size_t smem = 0;
   int grid = 0;
   cudaStream_t stream = nullptr;
   cudaStream_t side[kSideStreams] = {nullptr};
@@ -138,7 +156,7 @@ struct Batch {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   float tuned_ms = 0;
-  int nside = 4;                     // side streams in use
+  int nside = 4;                     // side streams of the big cells
 };
 
 std::unordered_map<long long, Batch *> g_batches;
@@ -236,6 +254,7 @@ void release(Batch *b) {
   b->graph = nullptr;
   auto F = [](void *p) { if (p) cudaFree(p); };
   F(b->arena); F(b->d_passes); F(b->d_dep); F(b->d_need); F(b->d_items);
+  F(b->d_pass_cell);
   F(b->d_done); F(b->d_next); F(b->d_err); F(b->d_scal); F(b->d_bounds);
   F(b->d_ncode); F(b->d_jobs); F(b->d_words); F(b->d_out); F(b->d_ext);
   F(b->d_extv); F(b->d_count);
@@ -245,6 +264,7 @@ void release(Batch *b) {
   b->d_count = nullptr; b->ext_cap = 0;
   b->d_bounds = nullptr;
   b->bounds_cap = 0;
+  b->d_pass_cell = nullptr;
   b->arena = nullptr; b->d_passes = nullptr; b->d_dep = nullptr;
   b->d_need = nullptr; b->d_items = nullptr; b->d_done = nullptr;
   b->d_next = nullptr; b->d_err = nullptr; b->d_scal = nullptr;
@@ -324,8 +344,10 @@ int make_schedule(Batch *b) {
   b->passes.clear();
   b->dep.clear();
   b->need.clear();
-  std::vector<std::vector<int>> by_level;
-  size_t smem = 0;
+  b->pass_cell.clear();
+  b->groups.clear();
+  // per kernel (-1 first): its passes by level
+  std::map<int, std::vector<std::vector<int>>> by_kid;
   const char *tma_env = getenv("CC_TMA");
   const bool streams_off = tma_env && atoi(tma_env) == 0;
   for (size_t i = 0; i < b->cells.size(); i++) {
@@ -373,11 +395,41 @@ int make_schedule(Batch *b) {
       }
       continue;
     }
-    const std::vector<GroupArgs> groups = plan_cell(c, b->tile_budget);
-    const int G = (int)groups.size();
+    // a small cell: three transforms of the same groups on one kernel
+    std::vector<std::vector<GroupPlan>> plans(3);
+    c.kid = -1;
+    if (c.regs) {
+      const long long ball = ball_cardinality(c.g);
+      for (int t = 0; t < 3; t++) {
+        Knobs kn{b->tile_budget, 0};
+        kn.half = c.R1 >= 2 && (t == 0 || ball <= 65535) ? 1 : 0;
+        PlanPtrs ptr{c.layers, c.plane, c.cnt, c.dcode,
+                     (long long)c.code.size(), t == 1 ? c.gain : c.loss};
+        ptr.layers16 = reinterpret_cast<uint16_t *>(c.layers + c.plane);
+        plans[t] = plan_groups(transform_geometry(c.g), c.R1, ptr,
+                               t == 0 ? kSrcCode : kSrcCnt,
+                               t == 0 ? kDstCnt : kDstMap, kn);
+        if (plans[t].empty()) return -1;
+      }
+      c.kid = plans[0][0].kernel;
+    } else {
+      for (const GroupArgs &ga : plan_cell(c, b->tile_budget)) {
+        GroupPlan p;
+        p.a = ga;
+        p.kernel = -1;
+        p.threads = 256;
+        p.smem = group_smem_bytes(ga, c.R1);
+        p.grid = (int)std::min<long long>(ga.ntiles,
+                                          (long long)sm_count() * 4);
+        for (auto &v : plans) v.push_back(p);
+      }
+    }
+    auto &by_level = by_kid[c.kid];
     for (int t = 0; t < 3; t++) {            // recount, gain, loss
+      const int G = (int)plans[t].size();
       for (int k = 0; k < G; k++) {
-        GroupArgs a = groups[k];
+        GroupPlan p = plans[t][k];
+        GroupArgs &a = p.a;
         const bool first = k == 0, last = k == G - 1;
         a.src = !first ? kSrcLayers : t == 0 ? kSrcCode : kSrcCnt;
         a.dst = !last ? kDstLayers : t == 0 ? kDstCnt : kDstMap;
@@ -390,14 +442,15 @@ int make_schedule(Batch *b) {
         a.map = t == 1 ? c.gain : c.loss;
         a.red = b->d_scal + 3 * i + t;
         a.red_mode = last ? (t == 0 ? 1 : 2) : 0;
+        if (prepare_group(p)) return -1;
         const int pid = (int)b->passes.size();
-        b->passes.push_back(a);
+        b->passes.push_back(p);
+        b->pass_cell.push_back((int)i);
         b->dep.push_back(pid == c.first_pass ? -1 : pid - 1);
         b->need.push_back((unsigned)a.ntiles);
         const int level = pid - c.first_pass;
         if ((int)by_level.size() <= level) by_level.resize(level + 1);
         by_level[level].push_back(pid);
-        smem = std::max(smem, group_smem_bytes(a, c.R1));
       }
     }
     c.npass = (int)b->passes.size() - c.first_pass;
@@ -432,7 +485,8 @@ int make_schedule(Batch *b) {
   }
   // tile slices of each cell's code for this schedule's first groups
   auto first_tiles = [&](const Cell &c) {
-    return c.big ? c.fast[0][0].a.ntiles : b->passes[c.first_pass].ntiles;
+    return c.big ? c.fast[0][0].a.ntiles
+                 : b->passes[c.first_pass].a.ntiles;
   };
   long long nb = 0;
   for (const Cell &c : b->cells) nb += first_tiles(c) + 1;
@@ -448,7 +502,7 @@ int make_schedule(Batch *b) {
     c.nbounds = first_tiles(c) + 1;
     nb += c.nbounds;
     for (int p = c.first_pass; p < c.first_pass + c.npass; p++)
-      b->passes[p].code_bounds = c.bounds;
+      b->passes[p].a.code_bounds = c.bounds;
     if (c.big)
       for (int t = 0; t < 3; t++)
         for (auto &gp : c.fast[t]) gp.a.code_bounds = c.bounds;
@@ -469,8 +523,8 @@ int make_schedule(Batch *b) {
       j.tile_words = (long long)a0.Bo * a0.mid * a0.inner;
       j.ntiles = a0.ntiles;
     } else {
-      const GroupArgs &a0 = b->passes[c.first_pass];
-      j.tile_words = (long long)a0.Bo * a0.mid;
+      const GroupArgs &a0 = b->passes[c.first_pass].a;
+      j.tile_words = (long long)a0.Bo * a0.mid * a0.inner;
       j.ntiles = a0.ntiles;
     }
     jobs.push_back(j);
@@ -483,38 +537,87 @@ int make_schedule(Batch *b) {
     CC_CK(cudaMemcpyAsync(b->d_jobs, jobs.data(),
                           jobs.size() * sizeof(BoundsJob),
                           cudaMemcpyHostToDevice, b->stream));
+  // the work items: per kernel, level by level; largest passes first inside
+  // a level (long tails start early).  A cell all of whose passes are single
+  // tiles is one chained item of its first level (register kernels).
   std::vector<int4> items;
-  for (auto &lv : by_level) {
-    // largest passes first inside a level: long tails start early
-    std::stable_sort(lv.begin(), lv.end(), [&](int x, int y) {
-      return b->passes[x].ntiles > b->passes[y].ntiles;
-    });
-    for (int pid : lv) {
-      const GroupArgs &a = b->passes[pid];
-      const long long tw = (long long)a.Bo * a.mid * a.W;
-      const long long per = std::max<long long>(1, item_words() / tw);
-      for (long long t = 0; t < a.ntiles; t += per)
-        items.push_back(make_int4(pid, (int)t,
-                                  (int)std::min<long long>(per, a.ntiles - t),
-                                  0));
+  for (auto &kv : by_kid) {
+    Group gr;
+    gr.kid = kv.first;
+    gr.item0 = (long long)items.size();
+    long long most = 1;                   // items of the widest level
+    for (auto &lv : kv.second) {
+      std::stable_sort(lv.begin(), lv.end(), [&](int x, int y) {
+        return b->passes[x].a.ntiles > b->passes[y].a.ntiles;
+      });
+      const long long before = (long long)items.size();
+      for (int pid : lv) {
+        const GroupArgs &a = b->passes[pid].a;
+        const Cell &c = b->cells[b->pass_cell[pid]];
+        gr.smem = std::max(gr.smem, b->passes[pid].smem);
+        if (gr.kid >= 0) {
+          bool single = true;
+          for (int p = c.first_pass; p < c.first_pass + c.npass; p++)
+            single = single && b->passes[p].a.ntiles == 1;
+          if (single) {
+            if (pid == c.first_pass)
+              items.push_back(make_int4(pid, 0, 1, c.npass));
+            continue;
+          }
+        }
+        const long long tw = (long long)a.Bo * a.mid * a.W;
+        const long long per = std::max<long long>(
+            1, item_words(gr.kid >= 0) / tw);
+        for (long long t = 0; t < a.ntiles; t += per)
+          items.push_back(make_int4(
+              pid, (int)t, (int)std::min<long long>(per, a.ntiles - t), 1));
+      }
+      most = std::max(most, (long long)items.size() - before);
     }
+    gr.nitems = (long long)items.size() - gr.item0;
+    gr.grid = gr.kid < 0 ? batch_grid(gr.smem)
+                         : (int)std::min<long long>(
+                               batch_groups_grid(gr.kid, gr.smem), most);
+    b->groups.push_back(gr);
+  }
+  // the register kernels' launches onto the streams the big cells leave,
+  // most items first
+  {
+    std::vector<size_t> order;
+    for (size_t k = 0; k < b->groups.size(); k++)
+      if (b->groups[k].kid >= 0) order.push_back(k);
+    std::sort(order.begin(), order.end(), [&](size_t x, size_t y) {
+      return b->groups[x].nitems > b->groups[y].nitems;
+    });
+    const int first = b->nside < kSideStreams ? b->nside : 0;
+    for (size_t k = 0; k < order.size(); k++)
+      b->groups[order[k]].side =
+          first + (int)(k % (size_t)(kSideStreams - first));
   }
   b->nitems = (long long)items.size();
-  b->smem = smem;
-  b->grid = batch_grid(smem);
+  b->grid = 0;
+  for (const Group &gr : b->groups) b->grid += gr.grid;
   auto F = [](void *p) { if (p) cudaFree(p); };
   F(b->d_passes); F(b->d_dep); F(b->d_need); F(b->d_items); F(b->d_done);
+  F(b->d_pass_cell); F(b->d_next);
   const size_t np = b->passes.size();
   const size_t npa = std::max<size_t>(1, np);
   CC_CK(cudaMalloc(&b->d_passes, npa * sizeof(GroupArgs)));
   CC_CK(cudaMalloc(&b->d_dep, npa * sizeof(int)));
   CC_CK(cudaMalloc(&b->d_need, npa * sizeof(unsigned)));
   CC_CK(cudaMalloc(&b->d_done, npa * sizeof(unsigned)));
+  CC_CK(cudaMalloc(&b->d_pass_cell, npa * sizeof(int)));
+  CC_CK(cudaMalloc(&b->d_next, std::max<size_t>(1, b->groups.size()) * 8));
   CC_CK(cudaMalloc(&b->d_items, std::max<size_t>(1, items.size()) *
                                     sizeof(int4)));
+  std::vector<GroupArgs> args;
+  for (const GroupPlan &p : b->passes) args.push_back(p.a);
   if (np) {
-    CC_CK(cudaMemcpyAsync(b->d_passes, b->passes.data(),
+    CC_CK(cudaMemcpyAsync(b->d_passes, args.data(),
                           np * sizeof(GroupArgs), cudaMemcpyHostToDevice,
+                          b->stream));
+    CC_CK(cudaMemcpyAsync(b->d_pass_cell, b->pass_cell.data(),
+                          np * sizeof(int), cudaMemcpyHostToDevice,
                           b->stream));
     CC_CK(cudaMemcpyAsync(b->d_dep, b->dep.data(), np * sizeof(int),
                           cudaMemcpyHostToDevice, b->stream));
@@ -559,6 +662,18 @@ int run_big_cell(Batch *b, size_t i, cudaStream_t s) {
   return 0;
 }
 
+// persistent launch k of the batch on its stream (nullptr active: every
+// cell's items run)
+int launch_items(Batch *b, size_t k, const int *active) {
+  const Group &gr = b->groups[k];
+  if (!gr.nitems) return 0;
+  BatchLaunch L{b->d_passes, b->d_dep, b->d_need, b->d_items + gr.item0,
+                gr.nitems, b->d_done, b->d_next + k, b->d_err, gr.smem,
+                gr.grid, gr.kid, b->d_pass_cell, active};
+  cudaStream_t s = gr.side < 0 ? b->stream : b->side[gr.side];
+  return gr.kid < 0 ? launch_batch(L, s) : launch_batch_groups(L, s);
+}
+
 int capture_graph(Batch *b) {
   if (b->exec) { cudaGraphExecDestroy(b->exec); b->exec = nullptr; }
   if (b->graph) { cudaGraphDestroy(b->graph); b->graph = nullptr; }
@@ -572,7 +687,8 @@ int capture_graph(Batch *b) {
       rc = -(100 + (int)e);
     }
   };
-  ck(cudaMemsetAsync(b->d_next, 0, 8, b->stream), "memset next");
+  ck(cudaMemsetAsync(b->d_next, 0, std::max<size_t>(1, b->groups.size()) * 8,
+                     b->stream), "memset next");
   ck(cudaMemsetAsync(b->d_err, 0, 4, b->stream), "memset err");
   ck(cudaMemsetAsync(b->d_done, 0, np * sizeof(unsigned), b->stream),
      "memset done");
@@ -582,20 +698,22 @@ int capture_graph(Batch *b) {
   k_batch_bounds<<<(unsigned)b->cells.size(), 256, 0, b->stream>>>(
       b->d_jobs);
   ck(cudaGetLastError(), "bounds launch");
-  // big cells fork onto side streams, small cells share one persistent
-  // launch on the main stream, and everything joins before the end
+  // big cells and the register kernels' small cells fork onto side streams,
+  // the runtime-size tiles run on the main stream, and everything joins
+  // before the end
   ck(cudaEventRecord(b->fork, b->stream), "fork record");
-  for (int k = 0; k < b->nside; k++)
-    ck(cudaStreamWaitEvent(b->side[k], b->fork, 0), "fork wait");
+  bool used[kSideStreams] = {false};
+  for (const Cell &c : b->cells) if (c.big) used[c.side] = true;
+  for (const Group &gr : b->groups) if (gr.side >= 0) used[gr.side] = true;
+  for (int k = 0; k < kSideStreams; k++)
+    if (used[k]) ck(cudaStreamWaitEvent(b->side[k], b->fork, 0), "fork wait");
+  for (size_t k = 0; k < b->groups.size() && !rc; k++)
+    rc = launch_items(b, k, nullptr);
   for (size_t i = 0; i < b->cells.size() && !rc; i++)
     if (b->cells[i].big)
       rc = run_big_cell(b, i, b->side[b->cells[i].side]);
-  if (!rc && b->nitems) {
-    BatchLaunch L{b->d_passes, b->d_dep, b->d_need, b->d_items, b->nitems,
-                  b->d_done, b->d_next, b->d_err, b->smem, b->grid};
-    rc = launch_batch(L, b->stream);
-  }
-  for (int k = 0; k < b->nside; k++) {
+  for (int k = 0; k < kSideStreams; k++) {
+    if (!used[k]) continue;
     ck(cudaEventRecord(b->join[k], b->side[k]), "join record");
     ck(cudaStreamWaitEvent(b->stream, b->join[k], 0), "join wait");
   }
@@ -638,14 +756,7 @@ int run_per_pass(Batch *b) {
       continue;
     }
     for (int p = c.first_pass; p < c.first_pass + c.npass; p++) {
-      GroupPlan gp;
-      gp.a = b->passes[p];
-      gp.kernel = -1;
-      gp.threads = 256;
-      gp.smem = group_smem_bytes(gp.a, c.R1);
-      gp.grid = (int)std::min<long long>(gp.a.ntiles,
-                                         (long long)sm_count() * 4);
-      const int rc = launch_group(gp, b->stream);
+      const int rc = launch_group(b->passes[p], b->stream);
       if (rc) return rc;
     }
   }
@@ -719,6 +830,8 @@ int dct_batch_add(long long h, int problem, int n, const int *ax, int R,
   bool homog = true;
   for (int i = 1; i < n; i++) homog &= ax[i] == ax[0];
   int bm = 0;
+  c.regs = homog && pick_group_kernel(transform_geometry(c.g).prob, ax[0],
+                                      c.R1, &bm) >= 0;
   c.big = c.g.space >= big_cell_words() && homog &&
           pick_group_kernel(problem, ax[0], c.R1, &bm) >= 0;
   b->cells.push_back(std::move(c));
@@ -746,7 +859,6 @@ int dct_batch_build(long long h, int tile_kb) {
   }
   CC_CK(cudaMalloc(&b->arena, total));
   b->arena_bytes = total;
-  CC_CK(cudaMalloc(&b->d_next, 8));
   CC_CK(cudaMalloc(&b->d_err, 4));
   CC_CK(cudaMalloc(&b->d_scal, b->cells.size() * 3 * 8));
   CC_CK(cudaMalloc(&b->d_ncode, b->cells.size() * 8));
@@ -884,7 +996,7 @@ int dct_batch_info(long long h, long long *out, int cap) {
         }
     } else {
       for (int p = c.first_pass; p < c.first_pass + c.npass; p++) {
-        GroupArgs a = b->passes[p];
+        GroupArgs a = b->passes[p].a;
         a.ncode = (long long)c.code.size();
         cb += group_bytes(a);
       }

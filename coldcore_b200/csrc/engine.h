@@ -229,21 +229,30 @@ int launch_code_bounds(const long long *code, long long ncode,
                        long long tile_words, long long ntiles,
                        long long *bounds, cudaStream_t s);
 
-// batched engine: one persistent launch over (pass, tile) work items
+// batched engine: persistent launches over (pass, tile) work items
 struct BatchLaunch {
   const GroupArgs *passes;
   const int *dep;
   const unsigned *need;
-  const int4 *items;            // (pass, first tile, tiles, 0)
+  // (pass, first tile, tiles, chain): chain > 1 runs the item's pass and the
+  // chain - 1 after it (single-tile passes of one cell) in the same CTA
+  const int4 *items;
   long long nitems;
   unsigned *done;
   unsigned long long *next;
   int *err;
   size_t smem;
   int grid;
+  int kernel;                   // -1 the runtime-size tiles, else a kernel id
+  const int *pass_cell;         // cell of each pass
+  const int *active;            // per cell: its items run (nullptr: all do)
 };
 int launch_batch(const BatchLaunch &b, cudaStream_t s);
 int batch_grid(size_t smem);
+// the register-blocked kernel `kernel` over work items (batch_groups.cu)
+int launch_batch_groups(const BatchLaunch &b, cudaStream_t s);
+// resident CTAs of that kernel over the whole GPU, opted in to `smem` bytes
+int batch_groups_grid(int kernel, size_t smem);
 
 // window pass (torus / grid) over one axis, any width, out of place
 struct WindowArgs {

@@ -93,3 +93,41 @@ def test_campaign_of_256_cells_against_golden_digests():
                 assert digest(b.loss(i).astype("<i4")) == g["loss"], (mode, i)
                 assert tuple(sc[i]) == (g["deficit"], g["gain_max"],
                                         g["loss_max"]), (mode, i)
+
+
+@pytest.mark.parametrize("mu", [1, 2])
+@pytest.mark.parametrize("tile_kb", [16, 96])
+def test_every_register_kernel_in_the_persistent_launches(tile_kb, mu):
+    """One chained single-tile cell and one of several passes per kernel of
+    the persistent launches: Hamming q = 2..6, Lee q = 4..7, the torus
+    windows, R = 1..4; codes with repeated words."""
+    cells = []
+    rng = np.random.default_rng(tile_kb + mu)
+    for R in (1, 2, 3, 4):
+        for p, q, ns in (("hamming", 2, (6, 13)), ("hamming", 3, (5, 9)),
+                         ("hamming", 4, (4, 7)), ("hamming", 5, (4, 6)),
+                         ("hamming", 6, (4, 5)), ("lee", 4, (4, 7)),
+                         ("lee", 5, (4, 6)), ("lee", 6, (4, 5)),
+                         ("lee", 7, (4, 5))):
+            for n in ns:
+                cells.append((p, (q,) * n, R))
+    cells += [("torus_linf", (3,) * 4, 1), ("torus_linf", (4,) * 7, 1),
+              ("torus_linf", (5,) * 6, 2)]
+    codes = [np.concatenate([c, c[:2]]) for c in
+             (rng.integers(0, int(np.prod(a)), size=9) for _p, a, _R in cells)]
+    with BatchEngine() as b:
+        for (p, a, R), code in zip(cells, codes):
+            b.add(p, a, R, code, mu)
+        b.build(tile_kb)
+        b.run(0)
+        sc = b.scalars()
+        for i, ((p, a, R), code) in enumerate(zip(cells, codes)):
+            o = OracleBackend(list(a), R, problem=p, mu=mu)
+            o.recount(code)
+            assert np.array_equal(b.cnt(i), o.read_cnt()), (i, p, a, R)
+            o.gain_map()
+            assert np.array_equal(b.gain(i), o.map), (i, p, a, R)
+            gmax = o.map_max()
+            o.loss_map()
+            assert np.array_equal(b.loss(i), o.map), (i, p, a, R)
+            assert tuple(sc[i]) == (o.uncovered(), gmax, o.map_max())
