@@ -41,6 +41,8 @@ struct Cell {
   long long nbounds = 0;
   int first_pass = 0, npass = 0;     // global pass range (small cells)
   int kid = -1;                      // register kernel of a small cell's passes
+  int gain_pass = 0, ngain = 0;      // its gain transform alone (greedy)
+  double gain_us = 0;                // estimate of that transform's time
   bool regs = false;                 // one axis size, with a register kernel
   bool big = false;                  // own register-blocked launches
   int side = 0;                      // its side stream (big cells)
@@ -51,7 +53,10 @@ struct Cell {
   long long code_cap = 0;
   long long *dncode = nullptr;
   // support table for the cell's walks (dct_batch_set_table), SoA slots
-  int32_t *dtbl = nullptr;
+  int32_t *dtbl_base = nullptr, *dtbl = nullptr;
+  uint32_t *dpk = nullptr;           // its packed form (pack_walk)
+  int4 *dent = nullptr;
+  int noff = 0;
   int slots = 0;
   long long tlen = 0;
 };
@@ -115,6 +120,7 @@ struct Group {
   size_t smem = 0;
   int grid = 1;
   int side = -1;                     // side stream, -1 the main stream
+  int next = 0;                      // its claim counter
 };
 
 struct Batch {
@@ -122,11 +128,14 @@ struct Batch {
   bool built = false;
   char *arena = nullptr;
   size_t arena_bytes = 0;
-  std::vector<GroupPlan> passes;
+  std::vector<GroupPlan> passes;     // the step's nstep, then gain alone
+  int nstep = 0;
   std::vector<int> dep;
   std::vector<unsigned> need;
   std::vector<int> pass_cell;
   std::vector<Group> groups;         // persistent launches, one a kernel
+  // the gain transforms alone, without reductions: the greedy's rebuilds
+  std::vector<Group> gain_groups;
   GroupArgs *d_passes = nullptr;
   int *d_dep = nullptr;
   unsigned *d_need = nullptr;
@@ -148,6 +157,12 @@ struct Batch {
   int32_t *d_extv = nullptr;
   long long ext_cap = 0;
   long long *d_count = nullptr;
+  // the greedy's workspace, grown to the largest call, and its state ring
+  char *d_greedy = nullptr;
+  size_t greedy_cap = 0;
+  char *h_greedy = nullptr;
+  size_t h_greedy_cap = 0;
+  cudaEvent_t ev_greedy[2] = {nullptr};
   size_t tile_budget = 48 * 1024;
   int grid = 0;
   cudaStream_t stream = nullptr;
@@ -157,6 +172,7 @@ struct Batch {
   cudaGraphExec_t exec = nullptr;
   float tuned_ms = 0;
   int nside = 4;                     // side streams of the big cells
+  int nnext = 0;                     // claim counters of d_next
 };
 
 std::unordered_map<long long, Batch *> g_batches;
@@ -257,8 +273,18 @@ void release(Batch *b) {
   F(b->d_pass_cell);
   F(b->d_done); F(b->d_next); F(b->d_err); F(b->d_scal); F(b->d_bounds);
   F(b->d_ncode); F(b->d_jobs); F(b->d_words); F(b->d_out); F(b->d_ext);
-  F(b->d_extv); F(b->d_count);
-  for (Cell &c : b->cells) { F(c.dtbl); c.dtbl = nullptr; }
+  F(b->d_extv); F(b->d_count); F(b->d_greedy);
+  if (b->h_greedy) cudaFreeHost(b->h_greedy);
+  for (auto &ev : b->ev_greedy) {
+    if (ev) cudaEventDestroy(ev);
+    ev = nullptr;
+  }
+  b->d_greedy = b->h_greedy = nullptr;
+  b->greedy_cap = b->h_greedy_cap = 0;
+  for (Cell &c : b->cells) {
+    F(c.dtbl_base);
+    c.dtbl_base = c.dtbl = nullptr; c.dpk = nullptr; c.dent = nullptr;
+  }
   b->d_ncode = nullptr; b->d_jobs = nullptr; b->d_words = nullptr;
   b->d_out = nullptr; b->d_ext = nullptr; b->d_extv = nullptr;
   b->d_count = nullptr; b->ext_cap = 0;
@@ -346,8 +372,10 @@ int make_schedule(Batch *b) {
   b->need.clear();
   b->pass_cell.clear();
   b->groups.clear();
+  b->gain_groups.clear();
   // per kernel (-1 first): its passes by level
-  std::map<int, std::vector<std::vector<int>>> by_kid;
+  typedef std::map<int, std::vector<std::vector<int>>> ByKid;
+  ByKid by_kid, gain_by_kid;
   const char *tma_env = getenv("CC_TMA");
   const bool streams_off = tma_env && atoi(tma_env) == 0;
   for (size_t i = 0; i < b->cells.size(); i++) {
@@ -455,6 +483,31 @@ int make_schedule(Batch *b) {
     }
     c.npass = (int)b->passes.size() - c.first_pass;
   }
+  b->nstep = (int)b->passes.size();
+  // the gain transforms again, on their own
+  for (size_t i = 0; i < b->cells.size(); i++) {
+    Cell &c = b->cells[i];
+    double bytes = 0;
+    if (c.big)
+      for (const auto &gp : c.fast[1]) bytes += group_bytes(gp.a);
+    const int G = c.npass / 3;
+    c.gain_pass = (int)b->passes.size();
+    c.ngain = G;
+    for (int k = 0; k < G; k++) {
+      GroupPlan p = b->passes[c.first_pass + G + k];
+      p.a.red_mode = 0;
+      bytes += group_bytes(p.a);
+      const int pid = (int)b->passes.size();
+      b->passes.push_back(p);
+      b->pass_cell.push_back((int)i);
+      b->dep.push_back(k == 0 ? -1 : pid - 1);
+      b->need.push_back((unsigned)p.a.ntiles);
+      auto &by_level = gain_by_kid[c.kid];
+      if ((int)by_level.size() <= k) by_level.resize(k + 1);
+      by_level[k].push_back(pid);
+    }
+    c.gain_us = 1.0 + bytes / 1.8e6;
+  }
   // big cells onto the side streams: largest (algorithmic bytes) first,
   // each onto the least loaded stream
   {
@@ -541,60 +594,64 @@ int make_schedule(Batch *b) {
   // a level (long tails start early).  A cell all of whose passes are single
   // tiles is one chained item of its first level (register kernels).
   std::vector<int4> items;
-  for (auto &kv : by_kid) {
-    Group gr;
-    gr.kid = kv.first;
-    gr.item0 = (long long)items.size();
-    long long most = 1;                   // items of the widest level
-    for (auto &lv : kv.second) {
-      std::stable_sort(lv.begin(), lv.end(), [&](int x, int y) {
-        return b->passes[x].a.ntiles > b->passes[y].a.ntiles;
-      });
-      const long long before = (long long)items.size();
-      for (int pid : lv) {
-        const GroupArgs &a = b->passes[pid].a;
-        const Cell &c = b->cells[b->pass_cell[pid]];
-        gr.smem = std::max(gr.smem, b->passes[pid].smem);
-        if (gr.kid >= 0) {
-          bool single = true;
-          for (int p = c.first_pass; p < c.first_pass + c.npass; p++)
-            single = single && b->passes[p].a.ntiles == 1;
-          if (single) {
-            if (pid == c.first_pass)
-              items.push_back(make_int4(pid, 0, 1, c.npass));
-            continue;
+  auto add_items = [&](ByKid &kids, std::vector<Group> &out, bool gain) {
+    for (auto &kv : kids) {
+      Group gr;
+      gr.kid = kv.first;
+      gr.item0 = (long long)items.size();
+      long long most = 1;                 // items of the widest level
+      for (auto &lv : kv.second) {
+        std::stable_sort(lv.begin(), lv.end(), [&](int x, int y) {
+          return b->passes[x].a.ntiles > b->passes[y].a.ntiles;
+        });
+        const long long before = (long long)items.size();
+        for (int pid : lv) {
+          const GroupArgs &a = b->passes[pid].a;
+          const Cell &c = b->cells[b->pass_cell[pid]];
+          gr.smem = std::max(gr.smem, b->passes[pid].smem);
+          if (gr.kid >= 0) {
+            const int p0 = gain ? c.gain_pass : c.first_pass;
+            const int np = gain ? c.ngain : c.npass;
+            bool single = true;
+            for (int p = p0; p < p0 + np; p++)
+              single = single && b->passes[p].a.ntiles == 1;
+            if (single) {
+              if (pid == p0) items.push_back(make_int4(pid, 0, 1, np));
+              continue;
+            }
           }
+          const long long tw = (long long)a.Bo * a.mid * a.W;
+          const long long per = std::max<long long>(
+              1, item_words(gr.kid >= 0) / tw);
+          for (long long t = 0; t < a.ntiles; t += per)
+            items.push_back(make_int4(
+                pid, (int)t, (int)std::min<long long>(per, a.ntiles - t), 1));
         }
-        const long long tw = (long long)a.Bo * a.mid * a.W;
-        const long long per = std::max<long long>(
-            1, item_words(gr.kid >= 0) / tw);
-        for (long long t = 0; t < a.ntiles; t += per)
-          items.push_back(make_int4(
-              pid, (int)t, (int)std::min<long long>(per, a.ntiles - t), 1));
+        most = std::max(most, (long long)items.size() - before);
       }
-      most = std::max(most, (long long)items.size() - before);
+      gr.nitems = (long long)items.size() - gr.item0;
+      gr.grid = gr.kid < 0 ? batch_grid(gr.smem)
+                           : (int)std::min<long long>(
+                                 batch_groups_grid(gr.kid, gr.smem), most);
+      gr.next = (int)(b->groups.size() + b->gain_groups.size());
+      out.push_back(gr);
     }
-    gr.nitems = (long long)items.size() - gr.item0;
-    gr.grid = gr.kid < 0 ? batch_grid(gr.smem)
-                         : (int)std::min<long long>(
-                               batch_groups_grid(gr.kid, gr.smem), most);
-    b->groups.push_back(gr);
-  }
-  // the register kernels' launches onto the streams the big cells leave,
-  // most items first
-  {
+    // the register kernels' launches onto the streams the big cells leave,
+    // most items first
     std::vector<size_t> order;
-    for (size_t k = 0; k < b->groups.size(); k++)
-      if (b->groups[k].kid >= 0) order.push_back(k);
+    for (size_t k = 0; k < out.size(); k++)
+      if (out[k].kid >= 0) order.push_back(k);
     std::sort(order.begin(), order.end(), [&](size_t x, size_t y) {
-      return b->groups[x].nitems > b->groups[y].nitems;
+      return out[x].nitems > out[y].nitems;
     });
     const int first = b->nside < kSideStreams ? b->nside : 0;
     for (size_t k = 0; k < order.size(); k++)
-      b->groups[order[k]].side =
+      out[order[k]].side =
           first + (int)(k % (size_t)(kSideStreams - first));
-  }
+  };
+  add_items(by_kid, b->groups, false);
   b->nitems = (long long)items.size();
+  add_items(gain_by_kid, b->gain_groups, true);
   b->grid = 0;
   for (const Group &gr : b->groups) b->grid += gr.grid;
   auto F = [](void *p) { if (p) cudaFree(p); };
@@ -607,7 +664,8 @@ int make_schedule(Batch *b) {
   CC_CK(cudaMalloc(&b->d_need, npa * sizeof(unsigned)));
   CC_CK(cudaMalloc(&b->d_done, npa * sizeof(unsigned)));
   CC_CK(cudaMalloc(&b->d_pass_cell, npa * sizeof(int)));
-  CC_CK(cudaMalloc(&b->d_next, std::max<size_t>(1, b->groups.size()) * 8));
+  b->nnext = (int)(b->groups.size() + b->gain_groups.size());
+  CC_CK(cudaMalloc(&b->d_next, std::max<size_t>(1, b->nnext) * 8));
   CC_CK(cudaMalloc(&b->d_items, std::max<size_t>(1, items.size()) *
                                     sizeof(int4)));
   std::vector<GroupArgs> args;
@@ -662,16 +720,56 @@ int run_big_cell(Batch *b, size_t i, cudaStream_t s) {
   return 0;
 }
 
-// persistent launch k of the batch on its stream (nullptr active: every
+// one persistent launch of the batch on its stream (nullptr active: every
 // cell's items run)
-int launch_items(Batch *b, size_t k, const int *active) {
-  const Group &gr = b->groups[k];
+int launch_items(Batch *b, const Group &gr, const int *active) {
   if (!gr.nitems) return 0;
   BatchLaunch L{b->d_passes, b->d_dep, b->d_need, b->d_items + gr.item0,
-                gr.nitems, b->d_done, b->d_next + k, b->d_err, gr.smem,
+                gr.nitems, b->d_done, b->d_next + gr.next, b->d_err, gr.smem,
                 gr.grid, gr.kid, b->d_pass_cell, active};
   cudaStream_t s = gr.side < 0 ? b->stream : b->side[gr.side];
   return gr.kid < 0 ? launch_batch(L, s) : launch_batch_groups(L, s);
+}
+
+// the gain map of every cell with active[i] again (d_active: the same flags
+// on the device), on the streams the step uses
+int rebuild_gains(Batch *b, const std::vector<int> &active,
+                  const int *d_active) {
+  const size_t np = std::max<size_t>(1, b->passes.size());
+  CC_CK(cudaMemsetAsync(b->d_next, 0, std::max<size_t>(1, b->nnext) * 8,
+                        b->stream));
+  CC_CK(cudaMemsetAsync(b->d_done, 0, np * sizeof(unsigned), b->stream));
+  CC_CK(cudaEventRecord(b->fork, b->stream));
+  bool used[kSideStreams] = {false};
+  auto fork = [&](int k) -> int {
+    if (used[k]) return 0;
+    used[k] = true;
+    CC_CK(cudaStreamWaitEvent(b->side[k], b->fork, 0));
+    return 0;
+  };
+  int rc = 0;
+  for (size_t i = 0; i < b->cells.size() && !rc; i++) {
+    const Cell &c = b->cells[i];
+    if (!c.big || !active[i]) continue;
+    rc = fork(c.side);
+    for (size_t k = 0; k < c.fast[1].size() && !rc; k++)
+      rc = launch_group(c.fast[1][k], b->side[c.side]);
+  }
+  for (size_t k = 0; k < b->gain_groups.size() && !rc; k++) {
+    const Group &gr = b->gain_groups[k];
+    bool any = false;
+    for (size_t i = 0; i < b->cells.size(); i++)
+      any = any || (active[i] && !b->cells[i].big && b->cells[i].kid == gr.kid);
+    if (!any) continue;
+    if (gr.side >= 0) rc = fork(gr.side);
+    if (!rc) rc = launch_items(b, gr, d_active);
+  }
+  for (int k = 0; k < kSideStreams; k++) {
+    if (!used[k]) continue;
+    CC_CK(cudaEventRecord(b->join[k], b->side[k]));
+    CC_CK(cudaStreamWaitEvent(b->stream, b->join[k], 0));
+  }
+  return rc;
 }
 
 int capture_graph(Batch *b) {
@@ -687,7 +785,7 @@ int capture_graph(Batch *b) {
       rc = -(100 + (int)e);
     }
   };
-  ck(cudaMemsetAsync(b->d_next, 0, std::max<size_t>(1, b->groups.size()) * 8,
+  ck(cudaMemsetAsync(b->d_next, 0, std::max<size_t>(1, b->nnext) * 8,
                      b->stream), "memset next");
   ck(cudaMemsetAsync(b->d_err, 0, 4, b->stream), "memset err");
   ck(cudaMemsetAsync(b->d_done, 0, np * sizeof(unsigned), b->stream),
@@ -708,7 +806,7 @@ int capture_graph(Batch *b) {
   for (int k = 0; k < kSideStreams; k++)
     if (used[k]) ck(cudaStreamWaitEvent(b->side[k], b->fork, 0), "fork wait");
   for (size_t k = 0; k < b->groups.size() && !rc; k++)
-    rc = launch_items(b, k, nullptr);
+    rc = launch_items(b, b->groups[k], nullptr);
   for (size_t i = 0; i < b->cells.size() && !rc; i++)
     if (b->cells[i].big)
       rc = run_big_cell(b, i, b->side[b->cells[i].side]);
@@ -927,7 +1025,7 @@ int dct_batch_run(long long h, int mode) {
     // self-test of the bounded dependency wait: one launch in which the
     // first pass needs one more tile than it has, so its dependents time
     // out; the launch must end with an error status, not hang
-    if (b->passes.size() < 2) return -1;
+    if (b->nstep < 2) return -1;
     std::vector<unsigned> poisoned = b->need;
     poisoned[0] += 1;
     CC_CK(cudaMemcpyAsync(b->d_need, poisoned.data(),
@@ -975,7 +1073,7 @@ int dct_batch_info(long long h, long long *out, int cap) {
   Batch *b = get(h);
   if (!b || !out || cap < 6) return -1;
   out[0] = (long long)b->cells.size();
-  out[1] = (long long)b->passes.size();
+  out[1] = b->nstep;
   out[2] = b->nitems;
   out[3] = (long long)(b->tile_budget / 1024);
   out[4] = b->grid;
@@ -1061,11 +1159,25 @@ int dct_batch_set_table(long long h, int cell, const int32_t *tbl, int slots,
       }
       soa[(size_t)k * len + t] = v;
     }
-  if (c.dtbl) cudaFree(c.dtbl);
+  // one allocation and one copy: the entries, the table, its packed form
+  std::vector<uint32_t> pk;
+  std::vector<int4> ent;
+  if (!pack_walk(c.g, soa, slots, len, pk, ent)) { pk.clear(); ent.clear(); }
+  std::vector<int32_t> all(4 * ent.size() + soa.size() + pk.size());
+  memcpy(all.data(), ent.data(), ent.size() * sizeof(int4));
+  memcpy(all.data() + 4 * ent.size(), soa.data(), soa.size() * 4);
+  memcpy(all.data() + 4 * ent.size() + soa.size(), pk.data(), pk.size() * 4);
+  if (c.dtbl_base) cudaFree(c.dtbl_base);
+  c.dtbl_base = nullptr;
   c.dtbl = nullptr;
-  CC_CK(cudaMalloc(&c.dtbl, soa.size() * 4));
-  CC_CK(cudaMemcpy(c.dtbl, soa.data(), soa.size() * 4,
+  CC_CK(cudaMalloc(&c.dtbl_base, all.size() * 4));
+  CC_CK(cudaMemcpy(c.dtbl_base, all.data(), all.size() * 4,
                    cudaMemcpyHostToDevice));
+  c.dent = reinterpret_cast<int4 *>(c.dtbl_base);
+  c.dtbl = c.dtbl_base + 4 * ent.size();
+  c.dpk = pk.empty() ? nullptr
+                     : reinterpret_cast<uint32_t *>(c.dtbl + soa.size());
+  c.noff = (int)ent.size();
   c.slots = slots;
   c.tlen = len;
   return 0;
@@ -1096,6 +1208,9 @@ WalkArgs cell_walk(const Cell &c) {
   w.slots = c.slots;
   w.len = c.tlen;
   w.cnt = c.cnt;
+  w.pk = c.dpk;
+  w.ent = c.dent;
+  w.noff = c.noff;
   return w;
 }
 
@@ -1204,7 +1319,7 @@ int dct_batch_greedy(long long h, const int *cells, int n, const int *max_add,
   CC_CK(cudaMemcpyAsync(sc.data(), b->d_scal, sc.size() * 8,
                         cudaMemcpyDeviceToHost, b->stream));
   CC_CK(cudaStreamSynchronize(b->stream));
-  long long max_space = 0, steps = 0, fresh_words = 0;
+  long long steps = 0;
   for (int k = 0; k < n; k++) {
     if (cells[k] < 0 || cells[k] >= (int)b->cells.size() || max_add[k] < 0 ||
         max_add[k] > cap)
@@ -1221,104 +1336,211 @@ int dct_batch_greedy(long long h, const int *cells, int n, const int *max_add,
     if (std::min<long long>((long long)c.code.size() + max_add[k],
                             maxmult * ball_cardinality(c.g)) > 65535)
       return -1;
-    max_space = std::max(max_space, c.g.space);
     steps = std::max<long long>(steps, std::min<long long>(
         max_add[k], sc[3 * cells[k]]));
-    fresh_words += c.tlen;
   }
-  // device state: per cell a GreedyState, its placed list and fresh list
-  char *ws = nullptr;
+  // workspace: per cell its table entry, state, placed words, chunk keys and
+  // dirty flags; the rebuild flags of the listed cells and of the batch's
+  // cells; the jobs of the two launches of a step
+  auto pad = [](size_t x) { return (x + 63) / 64 * 64; };
   const size_t st_b = (size_t)n * kGreedyStateBytes;
   const size_t pl_b = (size_t)n * std::max(cap, 1) * 8;
-  const size_t fr_b = (size_t)fresh_words * 8;
-  const size_t tb_b = (size_t)n * sizeof(BatchGreedyCell);
-  CC_CK(cudaMalloc(&ws, st_b + pl_b + fr_b + tb_b));
+  std::vector<int2> jam, jpl;
+  std::vector<int> pats(n);
+  // blocks of a cell's ball: enough for all cells together to fill the GPU
+  const int ball_blocks = std::max(8, sm_count() * 16 / n);
+  size_t chunks = 0, fresh_words = 0;
+  for (int k = 0; k < n; k++) {
+    const Cell &c = b->cells[cells[k]];
+    chunks += (size_t)greedy_chunks(c.g.space);
+    fresh_words += (size_t)c.tlen;
+    for (int j = 0; j < greedy_argmax_blocks(c.g.space); j++)
+      jam.push_back(make_int2(k, j));
+    pats[k] = greedy_pats(c.tlen, ball_blocks);
+    for (long long j = 0; j * pats[k] < c.tlen; j++)
+      jpl.push_back(make_int2(k, (int)j));
+  }
+  size_t off = 0;
+  auto take = [&](size_t bytes) { const size_t o = off; off += pad(bytes);
+                                  return o; };
+  const size_t o_tab = take((size_t)n * sizeof(BatchGreedyCell));
+  const size_t o_st = take(st_b), o_pl = take(pl_b);
+  const size_t o_key = take(chunks * 8), o_dirty = take(chunks);
+  const size_t o_fresh = take(fresh_words * 8);
+  const size_t o_flag = take((size_t)n * 4);
+  const size_t o_act = take(b->cells.size() * 4);
+  const size_t o_jam = take(jam.size() * 8), o_jpl = take(jpl.size() * 8);
+  if (off > b->greedy_cap) {
+    if (b->d_greedy) CC_CK(cudaFree(b->d_greedy));
+    b->d_greedy = nullptr;
+    b->greedy_cap = 0;
+    CC_CK(cudaMalloc(&b->d_greedy, off));
+    b->greedy_cap = off;
+  }
+  if (2 * st_b > b->h_greedy_cap) {
+    if (b->h_greedy) CC_CK(cudaFreeHost(b->h_greedy));
+    b->h_greedy = nullptr;
+    b->h_greedy_cap = 0;
+    CC_CK(cudaHostAlloc((void **)&b->h_greedy, 2 * st_b,
+                        cudaHostAllocDefault));
+    b->h_greedy_cap = 2 * st_b;
+  }
+  for (auto &ev : b->ev_greedy)
+    if (!ev) CC_CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  char *ws = b->d_greedy;
   int rc = 0;
   std::vector<BatchGreedyCell> tab(n);
-  std::vector<unsigned char> st0(st_b, 0);
+  std::vector<GreedyHost> st0(n);
+  std::vector<int> flag(n, 0), act(b->cells.size(), 0);
   {
-    long long fo = 0;
+    size_t co = 0, fo = 0;
     for (int k = 0; k < n; k++) {
       Cell &c = b->cells[cells[k]];
       BatchGreedyCell &g = tab[k];
-      g.w = WalkArgs{};
-      g.w.g = c.g;
-      g.w.tbl = c.dtbl;
-      g.w.slots = c.slots;
-      g.w.len = c.tlen;
-      g.w.cnt = c.cnt;
+      g.w = cell_walk(c);
       g.map = c.gain;
-      g.st = ws + (size_t)k * kGreedyStateBytes;
-      g.placed = reinterpret_cast<long long *>(ws + st_b) +
+      g.st = ws + o_st + (size_t)k * kGreedyStateBytes;
+      g.placed = reinterpret_cast<long long *>(ws + o_pl) +
                  (size_t)k * std::max(cap, 1);
-      g.fresh = reinterpret_cast<long long *>(ws + st_b + pl_b) + fo;
+      g.ckey = reinterpret_cast<unsigned long long *>(ws + o_key) + co;
+      g.dirty = reinterpret_cast<uint8_t *>(ws + o_dirty) + co;
+      g.code = c.dcode;
+      g.ncode = (long long)c.code.size();
       g.max_add = max_add[k];
-      fo += c.tlen;
-      // state: best 0, deficit from the last launch, done when nothing to do
-      long long *words = reinterpret_cast<long long *>(&st0[(size_t)k *
-                                                          kGreedyStateBytes]);
-      words[1] = sc[3 * cells[k]];
-      int *flags = reinterpret_cast<int *>(words + 2);
-      flags[0] = (max_add[k] == 0 || sc[3 * cells[k]] == 0) ? 1 : 0;
+      g.pats = pats[k];
+      g.fresh = reinterpret_cast<long long *>(ws + o_fresh) + fo;
+      co += (size_t)greedy_chunks(c.g.space);
+      fo += (size_t)c.tlen;
+      // done from the start when there is nothing to do
+      st0[k] = GreedyHost{};
+      st0[k].deficit = sc[3 * cells[k]];
+      st0[k].done = (max_add[k] == 0 || sc[3 * cells[k]] == 0) ? 1 : 0;
       deficit_out[k] = sc[3 * cells[k]];
       nplaced_out[k] = 0;
     }
   }
-  BatchGreedyCell *dtab = reinterpret_cast<BatchGreedyCell *>(
-      ws + st_b + pl_b + fr_b);
+  const BatchGreedyCell *dtab =
+      reinterpret_cast<const BatchGreedyCell *>(ws + o_tab);
+  int *d_flag = reinterpret_cast<int *>(ws + o_flag);
+  int *d_act = reinterpret_cast<int *>(ws + o_act);
+  const int2 *d_jam = reinterpret_cast<const int2 *>(ws + o_jam);
+  const int2 *d_jpl = reinterpret_cast<const int2 *>(ws + o_jpl);
   constexpr int32_t kExcluded = INT_MIN / 2;
   auto ck = [&](cudaError_t e) {
     if (e != cudaSuccess && !rc) rc = -(100 + (int)e);
   };
-  ck(cudaMemcpyAsync(ws, st0.data(), st_b, cudaMemcpyHostToDevice,
-                     b->stream));
-  ck(cudaMemcpyAsync(dtab, tab.data(), tb_b, cudaMemcpyHostToDevice,
-                     b->stream));
+  auto up = [&](size_t o, const void *src, size_t bytes) {
+    if (bytes) ck(cudaMemcpyAsync(ws + o, src, bytes, cudaMemcpyHostToDevice,
+                                  b->stream));
+  };
+  up(o_tab, tab.data(), (size_t)n * sizeof(BatchGreedyCell));
+  up(o_st, st0.data(), st_b);
+  up(o_jam, jam.data(), jam.size() * 8);
+  up(o_jpl, jpl.data(), jpl.size() * 8);
+  up(o_flag, flag.data(), (size_t)n * 4);
   // incumbents never re-enter
-  for (int k = 0; k < n && !rc; k++) {
-    const Cell &c = b->cells[cells[k]];
-    if (!c.code.empty())
-      rc = launch_greedy_exclude(c.gain, c.dcode, (int)c.code.size(),
-                                 kExcluded, b->stream);
-  }
-  // steps in chunks, with one look at the states between chunks
-  long long issued = 0, chunk = 32;
-  std::vector<unsigned char> stv(st_b);
-  while (!rc && issued < steps) {
-    const long long m = std::min(chunk, steps - issued);
-    for (long long i = 0; i < m && !rc; i++)
-      rc = launch_batch_greedy_step(dtab, n, max_space, kExcluded,
-                                    b->stream);
-    issued += m;
-    ck(cudaMemcpyAsync(stv.data(), ws, st_b, cudaMemcpyDeviceToHost,
+  if (!rc) rc = launch_greedy_exclude(dtab, n, nullptr, kExcluded, b->stream);
+  GreedyHost *ring[2] = {
+      reinterpret_cast<GreedyHost *>(b->h_greedy),
+      reinterpret_cast<GreedyHost *>(b->h_greedy + st_b)};
+  auto read_states = [&](int slot) {
+    ck(cudaMemcpyAsync(ring[slot], ws + o_st, st_b, cudaMemcpyDeviceToHost,
                        b->stream));
-    ck(cudaStreamSynchronize(b->stream));
+    ck(cudaEventRecord(b->ev_greedy[slot], b->stream));
+  };
+  // While a placement of some cell may be worth a rebuild of its map, the
+  // host follows the gains one step behind (the first step knows them from
+  // the last launch) and the device stays busy; gains never grow, so after
+  // that the steps go out in chunks with one look between them.
+  long long issued = 0, chunk = 32;
+  bool follow = true;
+  while (!rc && issued < steps) {
+    const int par = (int)(issued & 1);
+    if (follow) {
+      rc = launch_greedy_argmax(dtab, d_jam, (int)jam.size(), par,
+                                issued == 0, d_flag, b->stream);
+      read_states(par);
+      const GreedyHost *h = ring[par ^ 1];
+      if (issued) ck(cudaEventSynchronize(b->ev_greedy[par ^ 1]));
+      if (rc) break;
+      bool live = issued == 0, any = false, changed = false;
+      for (int k = 0; k < n; k++) {
+        const Cell &c = b->cells[cells[k]];
+        const bool done = issued ? h[k].done != 0 : st0[k].done != 0;
+        const long long gain = issued ? h[k].gain(par ^ 1)
+                                      : sc[3 * cells[k] + 1];
+        const int want = !done && greedy_rebuild_pays(gain, c.tlen, c.gain_us);
+        live = live || !done;
+        any = any || want;
+        changed = changed || want != flag[k];
+        flag[k] = act[cells[k]] = want;
+      }
+      if (!live) break;
+      if (changed) {
+        up(o_flag, flag.data(), (size_t)n * 4);
+        up(o_act, act.data(), act.size() * 4);
+      }
+      if (!rc)
+        rc = launch_greedy_place(dtab, d_jpl, (int)jpl.size(), par, kExcluded,
+                                 b->stream);
+      if (!rc)
+        rc = launch_greedy_refresh(dtab, n, ball_blocks, d_flag, b->stream);
+      if (any && !rc) rc = rebuild_gains(b, act, d_act);
+      if (any && !rc)
+        rc = launch_greedy_exclude(dtab, n, d_flag, kExcluded, b->stream);
+      follow = any;
+      issued++;
+      continue;
+    }
+    const long long m = std::min(chunk, steps - issued);
+    for (long long i = 0; i < m && !rc; i++, issued++) {
+      const int p2 = (int)(issued & 1);
+      rc = launch_greedy_argmax(dtab, d_jam, (int)jam.size(), p2, 0, d_flag,
+                                b->stream);
+      if (!rc) rc = launch_greedy_place(dtab, d_jpl, (int)jpl.size(), p2,
+                                        kExcluded, b->stream);
+      if (!rc) rc = launch_greedy_refresh(dtab, n, ball_blocks, d_flag,
+                                          b->stream);
+    }
+    read_states(0);
+    ck(cudaEventSynchronize(b->ev_greedy[0]));
     bool all = true;
-    for (int k = 0; k < n; k++)
-      all &= reinterpret_cast<int *>(&stv[(size_t)k * kGreedyStateBytes +
-                                          16])[0] != 0;
+    for (int k = 0; k < n; k++) all = all && ring[0][k].done;
     if (all) break;
     chunk = std::min<long long>(chunk * 2, 512);
   }
   if (!rc) {
-    ck(cudaMemcpyAsync(stv.data(), ws, st_b, cudaMemcpyDeviceToHost,
-                       b->stream));
+    read_states(0);
     ck(cudaStreamSynchronize(b->stream));
+    int err = 0;
+    ck(cudaMemcpyAsync(&err, b->d_err, 4, cudaMemcpyDeviceToHost, b->stream));
+    // the placed words: one copy while that is small, else cell by cell
+    std::vector<long long> words;
+    const bool once = pl_b <= (8u << 20);
+    if (once && !rc) {
+      words.resize(pl_b / 8);
+      ck(cudaMemcpyAsync(words.data(), ws + o_pl, pl_b, cudaMemcpyDeviceToHost,
+                         b->stream));
+      ck(cudaStreamSynchronize(b->stream));
+    }
     for (int k = 0; k < n && !rc; k++) {
-      const long long *words = reinterpret_cast<const long long *>(
-          &stv[(size_t)k * kGreedyStateBytes]);
-      const int *flags = reinterpret_cast<const int *>(words + 2);
-      deficit_out[k] = words[1];
-      nplaced_out[k] = flags[1];
-      if (flags[1])
+      const GreedyHost &h = ring[0][k];
+      const int got = h.placed_now();
+      deficit_out[k] = h.deficit_now();
+      nplaced_out[k] = got;
+      if (!got) continue;
+      if (once)
+        memcpy(placed_out + (size_t)k * cap, words.data() + (size_t)k * cap,
+               (size_t)got * 8);
+      else
         ck(cudaMemcpyAsync(placed_out + (size_t)k * cap, tab[k].placed,
-                           (size_t)flags[1] * 8, cudaMemcpyDeviceToHost,
+                           (size_t)got * 8, cudaMemcpyDeviceToHost,
                            b->stream));
     }
     ck(cudaStreamSynchronize(b->stream));
+    if (!rc && err) rc = -7;
   }
   cudaStreamSynchronize(b->stream);
-  cudaFree(ws);
   return rc;
 }
 

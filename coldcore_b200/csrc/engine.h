@@ -272,7 +272,20 @@ struct WalkArgs {
   int slots;
   long long len;
   uint16_t *cnt;
+  // the packed form of the table (pack_walk), nullptr where it has none:
+  // pattern t is four 8-bit indices into the noff + 1 offsets that a word's
+  // (position, shift) entries give, entry noff the 0 of an unused slot
+  const uint32_t *pk = nullptr;
+  const int4 *ent = nullptr;            // (stride, axis size, shift, -)
+  int noff = 0;
 };
+constexpr int kMaxPackOff = 255;
+// Packs a validated SoA table; false when the cell does not qualify: the
+// open grid (it rejects patterns), 2^31 words or more, more than four slots
+// or more than 255 (position, shift) entries.
+bool pack_walk(const Geometry &g, const std::vector<int32_t> &soa, int slots,
+               long long len, std::vector<uint32_t> &pk,
+               std::vector<int4> &ent);
 constexpr int kParamWords = 1024;       // words passed by value per launch
 struct WordsParam { long long w[kParamWords]; };
 
@@ -295,27 +308,80 @@ int launch_list_pred(const Geometry &g, const uint16_t *cnt, int mode,
 int launch_gather_set(const Geometry &g, const long long *dcand, int nc,
                       const unsigned long long *Z, long long zn, int32_t *out,
                       bool zeroed, cudaStream_t s);
-// device-side exact greedy (walks.cu): state in device memory, one step =
-// argmax of the gain map, placement of that word, incremental gain update
-struct GreedyState;
-constexpr int kGreedyStateBytes = 32;
-int launch_greedy_exclude(int32_t *map, const long long *dwords, int n,
-                          int32_t exclude, cudaStream_t s);
-// the batched form: one cell's walk, gain map, state and buffers
+// device-side exact greedy (walks.cu) over one cell or many: a step is an
+// argmax over chunk keys and a placement that lowers the gains it changes
+constexpr int kGreedyStateBytes = 48;
+constexpr int kGreedyChunk = 1024;        // map words per kept key
+constexpr int kGreedyBlockChunks = 8;     // chunks per argmax block: a warp each
+constexpr int kGreedyMaxPat = 1024;       // ball patterns per place block
+// host view of one cell's state (GreedyState)
+struct GreedyHost {
+  unsigned long long best[2];
+  long long deficit;
+  unsigned long long served;
+  int done, placed, pend, nnew;
+  long long deficit_now() const { return deficit - (pend ? (long long)served : 0); }
+  int placed_now() const { return placed + (pend ? 1 : 0); }
+  int gain(int par) const {
+    return best[par] ? (int)((uint32_t)(best[par] >> 32) ^ 0x80000000u) : 0;
+  }
+};
+static_assert(sizeof(GreedyHost) == kGreedyStateBytes, "state layout");
+// one cell of a greedy: its walk, gain map, state and buffers
 struct BatchGreedyCell {
   WalkArgs w;
   int32_t *map;
   void *st;                 // GreedyState (kGreedyStateBytes)
   long long *placed;
-  long long *fresh;         // |B| words
+  long long *fresh;         // |B| words: those the last placement satisfied
+  unsigned long long *ckey; // best key of each chunk of kGreedyChunk words
+  uint8_t *dirty;           // its key is stale
+  const long long *code;    // words that are never placed (device)
+  long long ncode;
   int max_add;
+  int pats;                 // ball patterns per place block, <= kGreedyMaxPat
 };
-int launch_batch_greedy_step(const BatchGreedyCell *dcells, int ncells,
-                             long long max_space, int32_t exclude,
-                             cudaStream_t s);
-int launch_greedy_step(const WalkArgs &w, int32_t *map, long long N,
-                       GreedyState *st, long long *placed, int max_add,
-                       long long *fresh, int32_t exclude, cudaStream_t s);
+// the blocks of one cell in each launch, and its patterns per place block
+inline long long greedy_chunks(long long space) {
+  return (space + kGreedyChunk - 1) / kGreedyChunk;
+}
+inline int greedy_argmax_blocks(long long space) {
+  return (int)((greedy_chunks(space) + kGreedyBlockChunks - 1) /
+               kGreedyBlockChunks);
+}
+inline int greedy_pats(long long len, int blocks) {
+  long long p = (len + blocks - 1) / blocks;
+  if (p < 16) p = 16;
+  if (p > kGreedyMaxPat) p = kGreedyMaxPat;
+  return (int)p;
+}
+struct GreedyRun;         // barrier state of launch_greedy_run (device)
+// takes each cell's code and the words placed so far out of its map (cells
+// with rebuild[cell], or all)
+int launch_greedy_exclude(const BatchGreedyCell *dcells, int ncells,
+                          const int *rebuild, int32_t exclude,
+                          cudaStream_t s);
+// jobs: (cell, block of the cell) per block, or nullptr for one cell; par:
+// parity of the step; all / rebuilt[cell]: read every chunk; rebuild[cell]:
+// its gain map is left to a transform
+int launch_greedy_argmax(const BatchGreedyCell *dcells, const int2 *jobs,
+                         int njobs, int par, int all, const int *rebuilt,
+                         cudaStream_t s);
+int launch_greedy_place(const BatchGreedyCell *dcells, const int2 *jobs,
+                        int njobs, int par, int32_t exclude, cudaStream_t s);
+// the gains after a placement: `blocks` blocks per cell share its new words
+int launch_greedy_refresh(const BatchGreedyCell *dcells, int ncells,
+                          int blocks, const int *rebuild, cudaStream_t s);
+// `steps` whole steps of one cell in a cooperative launch; run:
+// kGreedyRunBytes of device state, zero before the first launch, whose second
+// word is set when a barrier timed out
+constexpr int kGreedyRunBytes = 16;
+int launch_greedy_run(const BatchGreedyCell &cell, int par, int steps,
+                      int32_t exclude, GreedyRun *run, cudaStream_t s);
+// Whether a placement of gain `gain` is followed by a transform of
+// `rebuild_us` microseconds rather than by gain * |B| gain updates
+// (CC_GREEDY_REBUILD = 0 / 1 pins it).
+bool greedy_rebuild_pays(long long gain, long long ball, double rebuild_us);
 // swap evaluation fast path: per drop its loss and the list of its ball
 // words at exactly mu (two walks and a segment scan), then per candidate
 // the listed words of its drop within distance R

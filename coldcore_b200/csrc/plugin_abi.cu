@@ -40,6 +40,7 @@ namespace {
 
 constexpr long long kCounterMax = 65535;    // uint16 cnt
 constexpr long long kStageCap = 1 << 16;    // words per staged chunk
+constexpr int kGreedyRing = 2;              // steps whose states are in flight
 
 struct Plan {
   std::vector<GroupPlan> groups;   // layered / small-axis path
@@ -68,6 +69,9 @@ struct State {
   long long h_layers_bytes = 0;
   // support tables, SoA slots
   int32_t *tbl = nullptr, *tbl2 = nullptr;
+  uint32_t *pk = nullptr, *pk2 = nullptr;    // packed forms (pack_walk)
+  int4 *ent = nullptr;
+  int noff = 0;
   int slots = 0, slots2 = 0;
   long long len = 0;
   int fmt = 0;
@@ -119,9 +123,14 @@ struct State {
   long long *d_list = nullptr;
   long long lcap = 0;
   // device greedy: state, placed words, words satisfied per placement
+  // [the cell's BatchGreedyCell][its state][chunk keys][fresh words][dirty]
   char *d_greedy = nullptr;
-  long long *d_placed = nullptr, *h_placed = nullptr, *d_fresh = nullptr;
+  GreedyHost *h_greedy = nullptr;  // pinned ring of kGreedyRing states
+  cudaEvent_t ev_greedy[kGreedyRing] = {nullptr};
+  long long *d_placed = nullptr, *h_placed = nullptr;
   long long placed_cap = 0;
+  long long *d_active = nullptr;   // active words (mu > 1: excluded again)
+  long long active_cap = 0;
   Plan plans[3][4];                // [init_mode][out_mode]
   bool plan_ok[3][4] = {{false}};
   bool tuned[3][4] = {{false}};
@@ -291,6 +300,9 @@ WalkArgs walk_args() {
   w.slots = ox ? S.slots2 : S.slots;
   w.len = S.len;
   w.cnt = S.cnt;
+  w.pk = ox ? S.pk2 : S.pk;
+  w.ent = S.ent;
+  w.noff = S.noff;
   return w;
 }
 
@@ -299,11 +311,14 @@ void free_all() {
   auto F = [](void *p) { if (p) cudaFree(p); };
   auto FH = [](void *p) { if (p) cudaFreeHost(p); };
   F(S.layers); F(S.cnt); F(S.owner); F(S.tbl); F(S.tbl2); F(S.d_code);
+  F(S.pk); F(S.pk2); F(S.ent);
   F(S.d_bounds);
   F(S.d_words); F(S.d_out); F(S.d_scalar); F(S.d_hist); F(S.d_ext32);
   F(S.d_ext64); F(S.d_extv); F(S.zbuf); F(S.d_found);
   F(S.d_swap); F(S.d_list); FH(S.h_swap);
-  F(S.d_greedy); F(S.d_placed); F(S.d_fresh); FH(S.h_placed);
+  F(S.d_greedy); F(S.d_placed); F(S.d_active); FH(S.h_placed);
+  FH(S.h_greedy);
+  for (cudaEvent_t e : S.ev_greedy) if (e) cudaEventDestroy(e);
   F(S.d_bits);
   FH(S.h_layers);
   FH(S.h_words); FH(S.h_out); FH(S.h_scalar);
@@ -836,13 +851,27 @@ int init_common(int problem, int n, const int *ax, int R, long long len,
 }
 
 int upload_table(const std::vector<int32_t> &soa, int slots, int32_t **dst,
-                 int *dslots) {
+                 int *dslots, uint32_t **dpk) {
   CC_CK(cudaMalloc(dst, soa.size() * 4));
   CC_CK(cudaMemcpyAsync(*dst, soa.data(), soa.size() * 4,
                         cudaMemcpyHostToDevice, g_stream));
-  CC_CK(cudaStreamSynchronize(g_stream));
   S.bytes_dev += (long long)soa.size() * 4;
   *dslots = slots;
+  std::vector<uint32_t> pk;
+  std::vector<int4> ent;
+  if (pack_walk(S.g, soa, slots, S.len, pk, ent)) {
+    CC_CK(cudaMalloc(dpk, pk.size() * 4));
+    CC_CK(cudaMemcpyAsync(*dpk, pk.data(), pk.size() * 4,
+                          cudaMemcpyHostToDevice, g_stream));
+    S.bytes_dev += (long long)pk.size() * 4;
+    if (!S.ent) {                        // the cell's, whatever the table
+      CC_CK(cudaMalloc(&S.ent, ent.size() * sizeof(int4)));
+      CC_CK(cudaMemcpyAsync(S.ent, ent.data(), ent.size() * sizeof(int4),
+                            cudaMemcpyHostToDevice, g_stream));
+      S.noff = (int)ent.size();
+    }
+  }
+  CC_CK(cudaStreamSynchronize(g_stream));
   return 0;
 }
 
@@ -1081,7 +1110,7 @@ int dct_init3(int problem, int n, const int *ax, int R,
   std::vector<int32_t> soa;
   int slots = 0;
   if (unpack_v1(ballpat, balllen, soa, &slots)) { free_all(); return -1; }
-  rc = upload_table(soa, slots, &S.tbl, &S.slots);
+  rc = upload_table(soa, slots, &S.tbl, &S.slots, &S.pk);
   if (rc) return rc;
   set_side_init(soa, slots);
   return finish_init(bytes);
@@ -1115,7 +1144,7 @@ int dct_b200_init3wm(int problem, int n, const int *ax, int R,
       }
       soa[(size_t)k * len + t] = c;
     }
-  rc = upload_table(soa, slots, &S.tbl, &S.slots);
+  rc = upload_table(soa, slots, &S.tbl, &S.slots, &S.pk);
   if (rc) return rc;
   set_side_init(soa, slots);
   return finish_init(bytes);
@@ -1160,7 +1189,8 @@ int dct_set_tbl2(const uint16_t *mask, const uint64_t *offs, long long len) {
     }
   }
   if (S.tbl2) { cudaFree(S.tbl2); S.tbl2 = nullptr; }
-  return upload_table(soa, w, &S.tbl2, &S.slots2);
+  if (S.pk2) { cudaFree(S.pk2); S.pk2 = nullptr; }
+  return upload_table(soa, w, &S.tbl2, &S.slots2, &S.pk2);
 }
 
 int dct_use_fmt(int fmt) {
@@ -1358,13 +1388,20 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
   // placed words are new (multiplicity 1): the counters stay within uint16
   if (!within_counter(S.active_size + max_add, std::max(S.act_max, 1)))
     return -1;
-  std::vector<long long> code;
-  code.reserve(S.active.size());
-  for (const auto &e : S.active) code.push_back(e.first);
-  const long long M = (long long)code.size();
+  const int mu = g_mu;
+  const long long nch = greedy_chunks(S.g.space);
+  const size_t o_st = (sizeof(BatchGreedyCell) + 63) / 64 * 64;
+  const size_t o_run = o_st + 64;
+  const size_t o_key = o_run + kGreedyRunBytes;
+  static_assert(kGreedyStateBytes <= 64, "greedy state");
+  const size_t o_fresh = o_key + (size_t)nch * 8;
+  const size_t o_dirty = o_fresh + (size_t)S.len * 8;
   if (!S.d_greedy) {
-    CC_CK(cudaMalloc(&S.d_greedy, kGreedyStateBytes));
-    CC_CK(cudaMalloc(&S.d_fresh, (size_t)S.len * 8));
+    CC_CK(cudaMalloc(&S.d_greedy, o_dirty + (size_t)nch));
+    CC_CK(cudaHostAlloc((void **)&S.h_greedy, kGreedyRing * kGreedyStateBytes,
+                        cudaHostAllocDefault));
+    for (auto &ev : S.ev_greedy)
+      CC_CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   }
   if (max_add > S.placed_cap) {
     if (S.d_placed) CC_CK(cudaFree(S.d_placed));
@@ -1379,7 +1416,7 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
   }
   // the deficit to start from, and the gain map of the current cnt
   CC_CK(cudaMemsetAsync(S.d_scalar, 0, 8, g_stream));
-  int rc = launch_cnt_reduce(S.cnt, S.g.space, kPredDef, 0, g_mu,
+  int rc = launch_cnt_reduce(S.cnt, S.g.space, kPredDef, 0, mu,
                              S.d_scalar, g_stream);
   if (rc) return rc;
   long long d0;
@@ -1389,46 +1426,127 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
   if (max_add == 0 || d0 == 0) return 0;
   rc = autotune(1, 1);
   if (rc) return rc;
-  rc = run_transform(1, 1);
-  if (rc) return rc;
-  S.layered_out = false;
   constexpr int32_t kExcluded = INT_MIN / 2;
-  for (long long off = 0; off < M; off += kStageCap) {
-    const int nb = (int)std::min<long long>(kStageCap, M - off);
-    rc = stage_words(code.data() + off, nb);
-    if (rc) return rc;
-    rc = launch_greedy_exclude(S.layers, S.d_words, nb, kExcluded, g_stream);
-    if (rc) return rc;
-    CC_CK(cudaStreamSynchronize(g_stream));     // staging buffer reused
+  // At mu = 1, with a table that is the metric ball, an active word's whole
+  // ball is covered: its gain is 0 and it is never placed.  Otherwise the
+  // active words are taken out of the map, after every transform of it.
+  const bool exclude = mu > 1 || !S.set_ok || S.fmt != 0;
+  std::vector<long long> code;
+  if (exclude) {
+    code.reserve(S.active.size());
+    for (const auto &e : S.active) code.push_back(e.first);
+    if ((long long)code.size() > S.active_cap) {
+      if (S.d_active) CC_CK(cudaFree(S.d_active));
+      S.d_active = nullptr;
+      S.active_cap = 0;
+      const long long cap = std::max<long long>(2 * code.size(), 1024);
+      CC_CK(cudaMalloc(&S.d_active, (size_t)cap * 8));
+      S.active_cap = cap;
+    }
+    if (!code.empty())
+      CC_CK(cudaMemcpyAsync(S.d_active, code.data(), code.size() * 8,
+                            cudaMemcpyHostToDevice, g_stream));
   }
-  struct { unsigned long long best; long long deficit; int done, placed,
-           nnew, pad; } st0 = {0, d0, 0, 0, 0, 0};
-  static_assert(sizeof(st0) == kGreedyStateBytes, "state layout");
-  CC_CK(cudaMemcpyAsync(S.d_greedy, &st0, sizeof(st0),
-                        cudaMemcpyHostToDevice, g_stream));
-  const WalkArgs w = walk_args();
-  GreedyState *st = reinterpret_cast<GreedyState *>(S.d_greedy);
-  // every placement serves at least one deficient word: at most d0 steps.
-  // Steps go out in chunks (32, 64, ... 512) with one look at the state
-  // between chunks; steps after the stop are no-ops on the device.
+  BatchGreedyCell gc{};
+  gc.w = walk_args();
+  gc.map = S.layers;
+  gc.st = S.d_greedy + o_st;
+  gc.placed = S.d_placed;
+  gc.fresh = reinterpret_cast<long long *>(S.d_greedy + o_fresh);
+  gc.ckey = reinterpret_cast<unsigned long long *>(S.d_greedy + o_key);
+  gc.dirty = reinterpret_cast<uint8_t *>(S.d_greedy + o_dirty);
+  gc.code = S.d_active;
+  gc.ncode = (long long)code.size();
+  gc.max_add = max_add;
+  gc.pats = greedy_pats(S.len, sm_count() * 4);
+  GreedyHost st{};
+  st.deficit = d0;
+  BatchGreedyCell *dcell = reinterpret_cast<BatchGreedyCell *>(S.d_greedy);
+  CC_CK(cudaMemcpyAsync(dcell, &gc, sizeof(gc), cudaMemcpyHostToDevice,
+                        g_stream));
+  CC_CK(cudaMemcpyAsync(gc.st, &st, sizeof(st), cudaMemcpyHostToDevice,
+                        g_stream));
+  GreedyRun *run = reinterpret_cast<GreedyRun *>(S.d_greedy + o_run);
+  CC_CK(cudaMemsetAsync(run, 0, kGreedyRunBytes, g_stream));
+  auto build_map = [&]() -> int {
+    const int r = run_transform(1, 1);
+    if (r || !exclude) return r;
+    return launch_greedy_exclude(dcell, 1, nullptr, kExcluded, g_stream);
+  };
+  if ((rc = build_map())) return rc;
+  S.layered_out = false;
+  const int nam = greedy_argmax_blocks(S.g.space);
+  const int npl = (int)((S.len + gc.pats - 1) / gc.pats);
+  const int nrf = sm_count() * 4;
+  // the time of a gain transform: measured by the autotuner, else launches
+  // and bytes at a small cell's rate; a streamed cell is never rebuilt
+  double rebuild_us = S.tune_ms[1][1] * 1e3;
+  if (rebuild_us <= 0) {
+    const Plan &P = plan_for(1, 1);
+    rebuild_us = 4.0 * (P.groups.size() + P.passes.size());
+    for (const auto &gp : P.groups) rebuild_us += group_bytes(gp.a) / 2.0e6;
+    for (size_t i = 0; i < P.passes.size(); i++)
+      rebuild_us += 6.0 * S.g.space / 1.0e6;
+  }
+  if (S.streamed) rebuild_us = 1e30;
+  auto read_state = [&](int slot) -> int {
+    CC_CK(cudaMemcpyAsync(S.h_greedy + slot, gc.st, sizeof(st),
+                          cudaMemcpyDeviceToHost, g_stream));
+    CC_CK(cudaEventRecord(S.ev_greedy[slot], g_stream));
+    return 0;
+  };
+  // Every placement serves at least one deficient word: at most d0 steps;
+  // those after the stop return at once.  While a placement may still be
+  // worth a rebuild the host follows the gains one step behind (the first
+  // step waits for its own), and the device stays busy; after that steps go
+  // out in chunks with one look at the state between them.
   const long long steps = std::min<long long>(max_add, d0);
   long long issued = 0, chunk = 32;
+  bool follow = true, rebuilt = true;
   while (issued < steps) {
-    const long long n = std::min(chunk, steps - issued);
-    for (long long i = 0; i < n; i++) {
-      rc = launch_greedy_step(w, S.layers, S.g.space, st, S.d_placed,
-                              max_add, S.d_fresh, kExcluded, g_stream);
+    if (follow) {
+      const int par = (int)(issued & 1);
+      rc = launch_greedy_argmax(dcell, nullptr, nam, par, rebuilt, nullptr,
+                                g_stream);
+      if (rc || (rc = read_state(par))) return rc;
+      const int look = issued ? par ^ 1 : par;
+      CC_CK(cudaEventSynchronize(S.ev_greedy[look]));
+      const GreedyHost &h = S.h_greedy[look];
+      if (h.done) break;
+      const bool rebuild = greedy_rebuild_pays(h.gain(look), S.len,
+                                               rebuild_us);
+      rc = launch_greedy_place(dcell, nullptr, npl, par, kExcluded, g_stream);
       if (rc) return rc;
+      rc = rebuild ? build_map()
+                   : launch_greedy_refresh(dcell, 1, nrf, nullptr, g_stream);
+      if (rc) return rc;
+      rebuilt = rebuild;
+      follow = rebuild;
+      issued++;
+      continue;
     }
+    const long long n = std::min(chunk, steps - issued);
+    rc = launch_greedy_run(gc, (int)(issued & 1), (int)n, kExcluded, run,
+                           g_stream);
+    if (rc) return rc;
     issued += n;
-    CC_CK(cudaMemcpyAsync(S.h_scalar + 16, S.d_greedy, sizeof(st0),
-                          cudaMemcpyDeviceToHost, g_stream));
-    CC_CK(cudaStreamSynchronize(g_stream));
-    memcpy(&st0, S.h_scalar + 16, sizeof(st0));
-    if (st0.done) break;
+    if ((rc = read_state(0))) return rc;
+    CC_CK(cudaEventSynchronize(S.ev_greedy[0]));
+    if (S.h_greedy[0].done) break;
     chunk = std::min<long long>(chunk * 2, 512);
   }
-  const int n = st0.placed;
+  if ((rc = read_state(0))) return rc;
+  int tail[kGreedyRunBytes / 4] = {0};
+  CC_CK(cudaMemcpyAsync(tail, run, kGreedyRunBytes, cudaMemcpyDeviceToHost,
+                        g_stream));
+  CC_CK(cudaStreamSynchronize(g_stream));
+  if (tail[1]) {
+    fprintf(stderr, "coldcore_b200: a greedy launch timed out at its grid "
+            "barrier\n");
+    return -8;
+  }
+  st = S.h_greedy[0];
+  const int n = st.placed_now();
   if (n) {
     CC_CK(cudaMemcpyAsync(S.h_placed, S.d_placed, (size_t)n * 8,
                           cudaMemcpyDeviceToHost, g_stream));
@@ -1439,7 +1557,7 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
     apply_active(batch, +1, n);
   }
   S.cnt_ver++;
-  *deficit = st0.deficit;
+  *deficit = st.deficit_now();
   return n;
 }
 

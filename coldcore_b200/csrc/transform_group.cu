@@ -407,7 +407,8 @@ constexpr long long kBatchSpinLimit = 1LL << 22;
 __global__ void __launch_bounds__(256)
 batch_kernel(const GroupArgs *passes, const int *pass_dep,
              const unsigned *pass_need, const int4 *items, long long nitems,
-             unsigned *done, unsigned long long *next, int *err) {
+             unsigned *done, unsigned long long *next, int *err,
+             const int *pass_cell, const int *active) {
   extern __shared__ int32_t sm[];
   __shared__ long long s_it;
   __shared__ int s_bad;
@@ -421,6 +422,10 @@ batch_kernel(const GroupArgs *passes, const int *pass_dep,
     const long long it = s_it;
     if (it >= nitems) break;
     const int4 item = items[it];           // pass, first tile, tiles
+    if (active && !active[pass_cell[item.x]]) {
+      __syncthreads();                     // s_it is read by every thread
+      continue;
+    }
     const int *src = reinterpret_cast<const int *>(passes + item.x);
     int *dst = reinterpret_cast<int *>(&sg);
     for (int i = threadIdx.x; i < (int)(sizeof(GroupArgs) / 4);
@@ -456,7 +461,8 @@ batch_kernel(const GroupArgs *passes, const int *pass_dep,
 
 int launch_batch(const BatchLaunch &b, cudaStream_t s) {
   batch_kernel<<<b.grid, 256, b.smem, s>>>(b.passes, b.dep, b.need, b.items,
-                                           b.nitems, b.done, b.next, b.err);
+                                           b.nitems, b.done, b.next, b.err,
+                                           b.pass_cell, b.active);
   CC_CK(cudaGetLastError());
   return 0;
 }

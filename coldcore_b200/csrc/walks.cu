@@ -15,32 +15,70 @@
 // block owns one word (or a slice of its ball when the ball is large): the
 // word's digits, axis sizes and strides sit in shared memory, and each
 // thread resolves one pattern at a time with a few integer ops per slot.
+#include <algorithm>
 #include <cstdlib>
 
 #include "engine.h"
 
 namespace cc {
 
+// Walk kinds: the table's slots resolved per pattern (kSlots; kGrid rejects
+// patterns that leave the board), or the packed table (kPack): a word's
+// (position, shift) offsets are computed once per block into shared memory,
+// and a pattern is one 32-bit table read, four shared reads and three adds
+// instead of up to four table reads with a digit, a wrap and a 64-bit
+// multiply each.
+enum Walk { kSlots = 0, kGridWalk = 1, kPack = 2 };
+
 struct WordSmem {
   int dig[kMaxAxes];
   int ax[kMaxAxes];
   long long pw[kMaxAxes];
 };
+union WalkSmem {
+  WordSmem s;
+  int32_t off[kMaxPackOff + 1];
+};
 
-__device__ __forceinline__ void word_setup(const Geometry &g, long long w,
-                                           WordSmem &s) {
-  for (int j = threadIdx.x; j < g.n; j += blockDim.x) {
-    s.dig[j] = (int)((w / g.pw[j]) % g.ax[j]);
-    s.ax[j] = g.ax[j];
-    s.pw[j] = g.pw[j];
+inline int walk_kind(const WalkArgs &w) {
+  return w.g.prob == kGrid ? kGridWalk : w.pk ? kPack : kSlots;
+}
+
+template <int WALK>
+__device__ __forceinline__ void word_setup(const WalkArgs &a, long long w,
+                                           WalkSmem &m) {
+  if (WALK == kPack) {
+    for (int e = threadIdx.x; e <= a.noff; e += blockDim.x) {
+      int v = 0;
+      if (e < a.noff) {
+        const int4 en = __ldg(a.ent + e);
+        const int dg = (int)((unsigned)w / (unsigned)en.x % (unsigned)en.y);
+        const int nd = dg + en.z >= en.y ? en.z - en.y : en.z;
+        v = nd * en.x;
+      }
+      m.off[e] = v;
+    }
+  } else {
+    for (int j = threadIdx.x; j < a.g.n; j += blockDim.x) {
+      m.s.dig[j] = (int)((w / a.g.pw[j]) % a.g.ax[j]);
+      m.s.ax[j] = a.g.ax[j];
+      m.s.pw[j] = a.g.pw[j];
+    }
   }
   __syncthreads();
 }
 
 // word index of pattern t around w; -1 when the open grid rejects it
-template <bool GRID>
+template <int WALK>
 __device__ __forceinline__ long long walk_word(const WalkArgs &a, long long w,
-                                               long long t, const WordSmem &s) {
+                                               long long t,
+                                               const WalkSmem &m) {
+  if (WALK == kPack) {
+    const uint32_t p = __ldg(a.pk + t);
+    return (int32_t)w + m.off[p & 255u] + m.off[(p >> 8) & 255u] +
+           m.off[(p >> 16) & 255u] + m.off[p >> 24];
+  }
+  const WordSmem &s = m.s;
   long long x = w;
 #pragma unroll 1
   for (int k = 0; k < a.slots; k++) {
@@ -51,10 +89,40 @@ __device__ __forceinline__ long long walk_word(const WalkArgs &a, long long w,
     int nd = dg + dl;
     if (nd >= s.ax[p]) nd -= s.ax[p];
     const int sh = nd - dg;
-    if (GRID && (sh > a.g.R || sh < -a.g.R)) return -1;
+    if (WALK == kGridWalk && (sh > a.g.R || sh < -a.g.R)) return -1;
     x += (long long)sh * s.pw[p];
   }
   return x;
+}
+
+bool pack_walk(const Geometry &g, const std::vector<int32_t> &soa, int slots,
+               long long len, std::vector<uint32_t> &pk,
+               std::vector<int4> &ent) {
+  if (g.prob == kGrid || g.space >= (1LL << 31) || slots > 4) return false;
+  std::vector<int> base(g.n + 1, 0);
+  for (int j = 0; j < g.n; j++) {
+    if (g.ax[j] > kMaxPackOff) return false;
+    base[j + 1] = base[j] + g.ax[j] - 1;
+  }
+  const int noff = base[g.n];
+  if (noff > kMaxPackOff) return false;
+  ent.clear();
+  for (int j = 0; j < g.n; j++)
+    for (int d = 1; d < g.ax[j]; d++)
+      ent.push_back(make_int4((int)g.pw[j], g.ax[j], d, 0));
+  pk.resize((size_t)len);
+  for (long long t = 0; t < len; t++) {
+    uint32_t v = 0;
+    bool open = true;                     // slots after an empty one: unused
+    for (int k = 0; k < 4; k++) {
+      const int32_t c = open && k < slots ? soa[(size_t)k * len + t] : 0;
+      open = open && c;
+      const int e = c ? base[c >> 24] + (c & 0xFFFFFF) - 1 : noff;
+      v |= (uint32_t)e << (8 * k);
+    }
+    pk[(size_t)t] = v;
+  }
+  return true;
 }
 
 __device__ __forceinline__ long long block_sum(long long v) {
@@ -73,19 +141,19 @@ __device__ __forceinline__ long long block_sum(long long v) {
 // cnt[x] += delta over each word's support set.  trans != nullptr also
 // counts the deficit transitions read off the atomics' old values (an
 // increment from c < mu, a decrement from c <= mu).
-template <bool GRID, bool PARAM>
+template <int WALK, bool PARAM>
 __global__ void __launch_bounds__(256)
 k_update(const WalkArgs a, const long long *words, const WordsParam pw,
          int split, int delta, unsigned long long *trans) {
-  __shared__ WordSmem s;
+  __shared__ WalkSmem s;
   const int wi = blockIdx.x / split, seg = blockIdx.x % split;
   const long long w = PARAM ? pw.w[wi] : words[wi];
-  word_setup(a.g, w, s);
+  word_setup<WALK>(a, w, s);
   long long acc = 0;
   const long long step = (long long)split * blockDim.x;
   for (long long t = (long long)seg * blockDim.x + threadIdx.x; t < a.len;
        t += step) {
-    const long long x = walk_word<GRID>(a, w, t, s);
+    const long long x = walk_word<WALK>(a, w, t, s);
     if (x < 0) continue;
     uint32_t *cell = reinterpret_cast<uint32_t *>(a.cnt + (x & ~1LL));
     const int sh = (x & 1) ? 16 : 0;
@@ -103,19 +171,19 @@ k_update(const WalkArgs a, const long long *words, const WordsParam pw,
 }
 
 // out[wi] = #{x in B(w_i) : pred(cnt[x])}; split blocks per word add up
-template <bool GRID>
+template <int WALK>
 __global__ void __launch_bounds__(256)
 k_gather(const WalkArgs a, const long long *words, int split, int mode,
          int target, int32_t *out) {
-  __shared__ WordSmem s;
+  __shared__ WalkSmem s;
   const int wi = blockIdx.x / split, seg = blockIdx.x % split;
   const long long w = words[wi];
-  word_setup(a.g, w, s);
+  word_setup<WALK>(a, w, s);
   long long acc = 0;
   const long long step = (long long)split * blockDim.x;
   for (long long t = (long long)seg * blockDim.x + threadIdx.x; t < a.len;
        t += step) {
-    const long long x = walk_word<GRID>(a, w, t, s);
+    const long long x = walk_word<WALK>(a, w, t, s);
     if (x >= 0) acc += cnt_pred(mode, (int)a.cnt[x], target, a.g.mu);
   }
   acc = block_sum(acc);
@@ -128,20 +196,20 @@ k_gather(const WalkArgs a, const long long *words, int split, int mode,
 // out[wi][b] = #{x in B(w_i) : bin(x) == b}.  src 0 bins the map in log2
 // steps (0 for v <= 0, 1 for v == 1, 2 for 2..3, 3 for 4..7, ...), src 1
 // bins cnt linearly (cnt == b); both clip to nbins - 1.
-template <bool GRID>
+template <int WALK>
 __global__ void __launch_bounds__(256)
 k_ball_hist(const WalkArgs a, const long long *words, int split,
             const int32_t *map, int src, int nbins, int32_t *out) {
-  __shared__ WordSmem s;
+  __shared__ WalkSmem s;
   __shared__ int32_t hist[32];
   const int wi = blockIdx.x / split, seg = blockIdx.x % split;
   const long long w = words[wi];
   for (int b = threadIdx.x; b < nbins; b += blockDim.x) hist[b] = 0;
-  word_setup(a.g, w, s);
+  word_setup<WALK>(a, w, s);
   const long long step = (long long)split * blockDim.x;
   for (long long t = (long long)seg * blockDim.x + threadIdx.x; t < a.len;
        t += step) {
-    const long long x = walk_word<GRID>(a, w, t, s);
+    const long long x = walk_word<WALK>(a, w, t, s);
     if (x < 0) continue;
     int b;
     if (src == 0) {
@@ -164,12 +232,13 @@ int launch_ball_hist(const WalkArgs &w, const long long *dwords, int nb,
   const int split = pick_split(w.len, nb);
   CC_CK(cudaMemsetAsync(out, 0, (size_t)nb * nbins * 4, s));
   const dim3 grid((unsigned)nb * split);
-  if (w.g.prob == kGrid)
-    k_ball_hist<true><<<grid, 256, 0, s>>>(w, dwords, split, map, src, nbins,
-                                           out);
-  else
-    k_ball_hist<false><<<grid, 256, 0, s>>>(w, dwords, split, map, src,
-                                            nbins, out);
+#define CC_BH(W)                                                            \
+  case W:                                                                   \
+    k_ball_hist<W><<<grid, 256, 0, s>>>(w, dwords, split, map, src, nbins,  \
+                                        out);                               \
+    break;
+  switch (walk_kind(w)) { CC_BH(kSlots) CC_BH(kGridWalk) CC_BH(kPack) }
+#undef CC_BH
   CC_CK(cudaGetLastError());
   return 0;
 }
@@ -195,19 +264,19 @@ int launch_layers_at(const int32_t *layers, long long plane, int R1,
 // swap evaluation, first walk: per drop word, its loss (critical ball words)
 // and nmu = its ball words at exactly mu, the words that become deficient
 // when one copy of the drop is removed
-template <bool GRID>
+template <int WALK>
 __global__ void __launch_bounds__(256)
 k_drop_count(const WalkArgs a, const long long *drops, int split,
              int32_t *loss, int32_t *nmu) {
-  __shared__ WordSmem s;
+  __shared__ WalkSmem s;
   const int wi = blockIdx.x / split, seg = blockIdx.x % split;
   const long long w = drops[wi];
-  word_setup(a.g, w, s);
+  word_setup<WALK>(a, w, s);
   long long lo = 0, at = 0;
   const long long step = (long long)split * blockDim.x;
   for (long long t = (long long)seg * blockDim.x + threadIdx.x; t < a.len;
        t += step) {
-    const long long x = walk_word<GRID>(a, w, t, s);
+    const long long x = walk_word<WALK>(a, w, t, s);
     if (x < 0) continue;
     const int c = (int)a.cnt[x];
     lo += c >= 1 && c <= a.g.mu;
@@ -222,18 +291,18 @@ k_drop_count(const WalkArgs a, const long long *drops, int split,
 // second walk: the words at exactly mu, into the drop's segment of `list`
 // (cursor[i] starts at the segment's offset); slots past cap are dropped and
 // the caller, seeing the total above cap, falls back
-template <bool GRID>
+template <int WALK>
 __global__ void __launch_bounds__(256)
 k_drop_list(const WalkArgs a, const long long *drops, int split,
             int32_t *cursor, long long cap, long long *list) {
-  __shared__ WordSmem s;
+  __shared__ WalkSmem s;
   const int wi = blockIdx.x / split, seg = blockIdx.x % split;
   const long long w = drops[wi];
-  word_setup(a.g, w, s);
+  word_setup<WALK>(a, w, s);
   const long long step = (long long)split * blockDim.x;
   for (long long t = (long long)seg * blockDim.x + threadIdx.x; t < a.len;
        t += step) {
-    const long long x = walk_word<GRID>(a, w, t, s);
+    const long long x = walk_word<WALK>(a, w, t, s);
     if (x < 0 || (int)a.cnt[x] != a.g.mu) continue;
     const int slot = atomicAdd(&cursor[wi], 1);
     if (slot < cap) list[slot] = x;
@@ -247,294 +316,542 @@ int launch_drop_walks(const WalkArgs &w, const long long *ddrops, int k,
   if (k <= 0) return 0;
   const int split = pick_split(w.len, k);
   const dim3 grid((unsigned)k * split);
-  const bool gp = w.g.prob == kGrid;
-  if (gp) k_drop_count<true><<<grid, 256, 0, s>>>(w, ddrops, split, loss, nmu);
-  else k_drop_count<false><<<grid, 256, 0, s>>>(w, ddrops, split, loss, nmu);
+  const int kind = walk_kind(w);
+#define CC_DC(W)                                                            \
+  case W:                                                                   \
+    k_drop_count<W><<<grid, 256, 0, s>>>(w, ddrops, split, loss, nmu);      \
+    break;
+  switch (kind) { CC_DC(kSlots) CC_DC(kGridWalk) CC_DC(kPack) }
+#undef CC_DC
   CC_CK(cudaGetLastError());
   int rc = launch_seg_scan(nmu, k, cap, offs, cursor, s);
   if (rc) return rc;
-  if (gp)
-    k_drop_list<true><<<grid, 256, 0, s>>>(w, ddrops, split, cursor, cap, list);
-  else
-    k_drop_list<false><<<grid, 256, 0, s>>>(w, ddrops, split, cursor, cap,
-                                            list);
+#define CC_DL(W)                                                            \
+  case W:                                                                   \
+    k_drop_list<W><<<grid, 256, 0, s>>>(w, ddrops, split, cursor, cap,      \
+                                        list);                              \
+    break;
+  switch (kind) { CC_DL(kSlots) CC_DL(kGridWalk) CC_DL(kPack) }
+#undef CC_DL
   CC_CK(cudaGetLastError());
   return 0;
 }
 
 // ------------------------------------------------------------ device greedy
-// State of one device-side greedy fill (all fields in device memory).
-// best: the packed argmax key of the current step, (gain ^ sign) << 32 |
-// ~index, so the largest gain wins and ties go to the smallest index.
+// The exact greedy over one cell (dct_b200_greedy_fill) or many at once (the
+// batched engine's campaign repair), three launches a step:
+//
+//   k_greedy_argmax   the word of largest gain (ties: the smallest index).
+//     The map is cut into chunks of kChunk words whose best keys are kept; a
+//     step reads only the chunks whose best word lost gain (dirty).
+//   k_greedy_place    the word's ball, split over many blocks: cnt += 1 with
+//     pair atomics; the words it satisfies (old count mu - 1) are listed.
+//   k_greedy_refresh  lowers the gain of every candidate whose ball holds a
+//     listed word, the list's balls shared out evenly in pieces.  (Blocks of
+//     the place launch that refresh their own words need no list and no
+//     third launch, but the words cluster: 46 us a step on K_3(14,3) near a
+//     cover, against 16 us for the three.)
+//
+// When a placement satisfies many words, |fresh| x |B| gain updates cost more
+// than a gain transform of the whole cell; the caller then leaves the map to
+// a transform (rebuild), and the next argmax reads every chunk.  Gains never
+// grow, so a cell leaves that regime for good.
+//
+// The state is committed by the NEXT argmax launch (block 0 of the cell), so
+// every block of one place launch decides the same stop from values that the
+// launch itself does not change.
 struct GreedyState {
-  unsigned long long best;
-  long long deficit;          // sum max(0, mu - cnt), maintained exactly
-  int done;                   // 1: no positive gain or nothing uncovered
-  int placed;                 // words placed so far
-  int nnew;                   // words satisfied by the last placement
-  int pad;
+  // packed argmax keys of even and odd steps: (gain ^ sign) << 32 | ~index,
+  // so the largest gain wins and ties go to the smallest index
+  unsigned long long best[2];
+  long long deficit;            // sum max(0, mu - cnt) before the last place
+  unsigned long long served;    // the last placement's part of it
+  int done;                     // no positive gain, or nothing uncovered
+  int placed;                   // words placed before the last place
+  int pend;                     // the last place launch placed a word
+  int nnew;                     // words it satisfied (old count mu - 1)
 };
 static_assert(sizeof(GreedyState) == kGreedyStateBytes, "state layout");
+
+constexpr int kChunk = kGreedyChunk;
+// updates a refresh makes in a microsecond: 36,000 (445 K of them in 12 us
+// on K_3(14,3)), against a transform of the cell
+constexpr double kGreedyUpdatesPerUs = 36000.0;
+constexpr int kBlockChunks = kGreedyBlockChunks;
 
 __device__ __forceinline__ unsigned long long greedy_key(int32_t v,
                                                          long long x) {
   return ((unsigned long long)((uint32_t)v ^ 0x80000000u) << 32) |
          (uint32_t)~(uint32_t)x;
 }
-
-// map[x] = exclude for every listed word (incumbents never re-enter)
-__global__ void k_greedy_exclude(int32_t *map, const long long *words, int n,
-                                 int32_t exclude) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) map[words[i]] = exclude;
+__device__ __forceinline__ int32_t key_gain(unsigned long long k) {
+  return (int32_t)((uint32_t)(k >> 32) ^ 0x80000000u);
 }
 
-// step 1: best = argmax map (largest value, then smallest index)
+// map[x] = exclude for a cell's code and placed words (they never re-enter);
+// runs after a place launch, whose own word counts (pend)
 __global__ void __launch_bounds__(256)
-k_greedy_argmax(const int32_t *map, long long N, GreedyState *st) {
-  if (st->done) return;
-  unsigned long long k = 0;
-  const long long gs = (long long)gridDim.x * blockDim.x;
-  const long long nv = N >> 2;
-  const int4 *v4 = reinterpret_cast<const int4 *>(map);
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-       i < nv; i += gs) {
-    const int4 q = __ldcg(v4 + i);
-    k = max(k, greedy_key(q.x, 4 * i));
-    k = max(k, greedy_key(q.y, 4 * i + 1));
-    k = max(k, greedy_key(q.z, 4 * i + 2));
-    k = max(k, greedy_key(q.w, 4 * i + 3));
-  }
-  if (blockIdx.x == 0 && threadIdx.x < (N & 3))
-    k = max(k, greedy_key(map[nv * 4 + threadIdx.x], nv * 4 + threadIdx.x));
-  for (int o = 16; o > 0; o >>= 1)
-    k = max(k, __shfl_down_sync(0xffffffffu, k, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(&st->best, k);
-}
-
-// step 2: place the argmax word (one block): cnt += 1 over its ball, the
-// words it satisfies (old count mu - 1) go to `fresh`, the deficit drops by
-// the words it serves (old count < mu)
-template <bool GRID>
-__global__ void __launch_bounds__(256)
-k_greedy_place(const WalkArgs a, int32_t *map, GreedyState *st,
-               long long *placed, int max_add, long long *fresh,
-               int32_t exclude) {
-  __shared__ WordSmem s;
-  __shared__ long long w_s;
-  __shared__ int stop;
-  __shared__ int nfresh;
-  __shared__ long long served;
-  if (threadIdx.x == 0) {
-    stop = st->done;
-    if (!stop) {
-      const unsigned long long k = st->best;
-      const int32_t v = (int32_t)((uint32_t)(k >> 32) ^ 0x80000000u);
-      const long long x = (long long)(uint32_t)~(uint32_t)k;
-      if (v <= 0 || st->deficit <= 0 || st->placed >= max_add) {
-        st->done = 1;
-        stop = 1;
-      } else {
-        w_s = x;
-        placed[st->placed] = x;
-        st->placed += 1;
-        map[x] = exclude;
-      }
-    }
-    st->best = 0;                     // fresh for the next step's argmax
-    st->nnew = 0;
-    nfresh = 0;
-    served = 0;
-  }
-  __syncthreads();
-  if (stop) return;
-  const long long w = w_s;
-  word_setup(a.g, w, s);
-  long long mine = 0;
-  for (long long t = threadIdx.x; t < a.len; t += blockDim.x) {
-    const long long x = walk_word<GRID>(a, w, t, s);
-    if (x < 0) continue;
-    uint32_t *cell = reinterpret_cast<uint32_t *>(a.cnt + (x & ~1LL));
-    const int sh = (x & 1) ? 16 : 0;
-    const uint32_t old = atomicAdd(cell, 1u << sh);
-    const int c = (int)((old >> sh) & 0xFFFFu);
-    if (c < a.g.mu) mine++;
-    if (c == a.g.mu - 1) fresh[atomicAdd(&nfresh, 1)] = x;
-  }
-  mine = block_sum(mine);
-  if (threadIdx.x == 0) {
-    st->deficit -= mine;
-    st->nnew = nfresh;
-  }
-}
-
-// step 3: every word satisfied by the placement stops counting towards the
-// gain of the candidates whose balls hold it: map[y] -= 1 for y in B(u)
-template <bool GRID>
-__global__ void __launch_bounds__(256)
-k_greedy_refresh(const WalkArgs a, int32_t *map, const GreedyState *st,
-                 const long long *fresh) {
-  __shared__ WordSmem s;
-  if (st->done) return;
-  const int n = st->nnew;
-  for (int u = blockIdx.x; u < n; u += gridDim.x) {
-    const long long x0 = fresh[u];
-    __syncthreads();                      // s is reused across words
-    word_setup(a.g, x0, s);
-    for (long long t = threadIdx.x; t < a.len; t += blockDim.x) {
-      const long long y = walk_word<GRID>(a, x0, t, s);
-      if (y >= 0) atomicSub(&map[y], 1);
-    }
-  }
-}
-
-// ------------------------------------------------------------ batched greedy
-// The same exact greedy over many cells at once (the batched engine's
-// campaign repair): one argmax, one place and one refresh launch per step
-// for every cell, each cell's state and buffers in its BatchGreedyCell.
-// Cells that are done return at once, so the launches of a step cost only
-// the cells still placing.
-constexpr int kArgmaxChunk = 8192;        // words per argmax block
-
-__global__ void __launch_bounds__(256)
-k_bgreedy_argmax(const BatchGreedyCell *cells) {
+k_greedy_exclude(const BatchGreedyCell *__restrict__ cells,
+                 const int *__restrict__ rebuild, int32_t exclude) {
+  if (rebuild && !rebuild[blockIdx.y]) return;
   const BatchGreedyCell &c = cells[blockIdx.y];
+  const GreedyState *st = reinterpret_cast<const GreedyState *>(c.st);
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long step = (long long)gridDim.x * blockDim.x;
+  for (long long i = t; i < c.ncode; i += step) c.map[c.code[i]] = exclude;
+  const long long n = st->placed + (st->pend ? 1 : 0);
+  for (long long i = t; i < n; i += step) c.map[c.placed[i]] = exclude;
+}
+
+// a warp: the key of chunk ch read from the map, and kept
+__device__ __forceinline__ unsigned long long read_chunk(
+    const BatchGreedyCell &c, long long ch) {
+  const long long N = c.w.g.space, x0 = ch * kChunk;
+  const int lane = threadIdx.x & 31;
+  unsigned long long m = 0;
+  if (x0 + kChunk <= N) {
+    const int4 *v4 = reinterpret_cast<const int4 *>(c.map + x0);
+    int4 q[kChunk / 128];
+#pragma unroll
+    for (int u = 0; u < kChunk / 128; u++) q[u] = __ldcg(v4 + lane + 32 * u);
+#pragma unroll
+    for (int u = 0; u < kChunk / 128; u++) {
+      const long long x = x0 + 4 * (lane + 32 * u);
+      m = max(m, greedy_key(q[u].x, x));
+      m = max(m, greedy_key(q[u].y, x + 1));
+      m = max(m, greedy_key(q[u].z, x + 2));
+      m = max(m, greedy_key(q[u].w, x + 3));
+    }
+  } else {
+    for (long long x = x0 + lane; x < N; x += 32)
+      m = max(m, greedy_key(__ldcg(c.map + x), x));
+  }
+  for (int o = 16; o > 0; o >>= 1)
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (lane == 0) {
+    c.ckey[ch] = m;
+    c.dirty[ch] = 0;
+  }
+  return m;
+}
+
+// jobs: (cell, block of the cell), or nullptr for cell 0 and blockIdx.x;
+// block 0 of a cell also commits its last placement
+__global__ void __launch_bounds__(32 * kBlockChunks)
+k_greedy_argmax(const BatchGreedyCell *__restrict__ cells,
+                const int2 *__restrict__ jobs, int par, int all,
+                const int *__restrict__ rebuilt) {
+  const int2 job = jobs ? jobs[blockIdx.x] : make_int2(0, (int)blockIdx.x);
+  const BatchGreedyCell &c = cells[job.x];
   GreedyState *st = reinterpret_cast<GreedyState *>(c.st);
   if (st->done) return;
-  const long long N = c.w.g.space;
-  const long long x0 = (long long)blockIdx.x * kArgmaxChunk;
-  if (x0 >= N) return;
-  const long long x1 = min(N, x0 + (long long)kArgmaxChunk);
-  unsigned long long k = 0;
-  for (long long x = x0 + threadIdx.x; x < x1; x += blockDim.x)
-    k = max(k, greedy_key(__ldcg(c.map + x), x));
-  for (int o = 16; o > 0; o >>= 1)
-    k = max(k, __shfl_down_sync(0xffffffffu, k, o));
-  if ((threadIdx.x & 31) == 0 && k) atomicMax(&st->best, k);
+  if (job.y == 0 && threadIdx.x == 0) {
+    if (st->pend) {
+      st->deficit -= (long long)st->served;
+      st->placed += 1;
+      st->pend = 0;
+    }
+    st->served = 0;
+    st->nnew = 0;
+    st->best[par ^ 1] = 0;
+  }
+  const long long ch = (long long)job.y * kBlockChunks + (threadIdx.x >> 5);
+  if (ch * kChunk >= c.w.g.space) return;           // a whole warp
+  const unsigned long long m =
+      all || (rebuilt && rebuilt[job.x]) || c.dirty[ch] ? read_chunk(c, ch)
+                                                        : c.ckey[ch];
+  // one atomic a warp; most warps see a larger key already there
+  if ((threadIdx.x & 31) == 0 && m > __ldcg(&st->best[par]))
+    atomicMax(&st->best[par], m);
 }
 
-template <bool GRID>
-__device__ __forceinline__ void bgreedy_place(const BatchGreedyCell &c,
-                                              int32_t exclude) {
-  __shared__ WordSmem s;
+template <int WALK>
+__device__ __forceinline__ void greedy_place(const BatchGreedyCell &c,
+                                             int seg, int par,
+                                             int32_t exclude) {
+  __shared__ WalkSmem s;
+  __shared__ long long fresh[kGreedyMaxPat];
   __shared__ long long w_s;
   __shared__ int stop;
-  __shared__ int nfresh;
+  __shared__ int nfresh, base;
   GreedyState *st = reinterpret_cast<GreedyState *>(c.st);
   const WalkArgs &a = c.w;
   if (threadIdx.x == 0) {
-    stop = st->done;
-    if (!stop) {
-      const unsigned long long k = st->best;
-      const int32_t v = (int32_t)((uint32_t)(k >> 32) ^ 0x80000000u);
-      const long long x = (long long)(uint32_t)~(uint32_t)k;
-      if (k == 0 || v <= 0 || st->deficit <= 0 || st->placed >= c.max_add) {
+    const unsigned long long k = __ldcg(&st->best[par]);
+    const long long x = (long long)(uint32_t)~(uint32_t)k;
+    const int done = __ldcg(&st->done), placed = __ldcg(&st->placed);
+    stop = done || k == 0 || key_gain(k) <= 0 || __ldcg(&st->deficit) <= 0 ||
+           placed >= c.max_add;
+    w_s = x;
+    nfresh = 0;
+    if (seg == 0) {
+      if (stop) {
         st->done = 1;
-        stop = 1;
       } else {
-        w_s = x;
-        c.placed[st->placed] = x;
-        st->placed += 1;
+        c.placed[placed] = x;
+        st->pend = 1;
         c.map[x] = exclude;
+        c.dirty[x / kChunk] = 1;
       }
     }
-    st->best = 0;
-    st->nnew = 0;
-    nfresh = 0;
   }
   __syncthreads();
   if (stop) return;
-  const long long w = w_s;
-  word_setup(a.g, w, s);
-  long long mine = 0;
-  for (long long t = threadIdx.x; t < a.len; t += blockDim.x) {
-    const long long x = walk_word<GRID>(a, w, t, s);
+  word_setup<WALK>(a, w_s, s);
+  int mine = 0;
+  const long long t1 = min(a.len, (long long)(seg + 1) * c.pats);
+  for (long long t = (long long)seg * c.pats + threadIdx.x; t < t1;
+       t += blockDim.x) {
+    const long long x = walk_word<WALK>(a, w_s, t, s);
     if (x < 0) continue;
     uint32_t *cell = reinterpret_cast<uint32_t *>(a.cnt + (x & ~1LL));
     const int sh = (x & 1) ? 16 : 0;
     const uint32_t old = atomicAdd(cell, 1u << sh);
     const int cv = (int)((old >> sh) & 0xFFFFu);
-    if (cv < a.g.mu) mine++;
-    if (cv == a.g.mu - 1) c.fresh[atomicAdd(&nfresh, 1)] = x;
+    mine += cv < a.g.mu;
+    if (cv == a.g.mu - 1) fresh[atomicAdd(&nfresh, 1)] = x;
   }
-  mine = block_sum(mine);
-  if (threadIdx.x == 0) {
-    st->deficit -= mine;
-    st->nnew = nfresh;
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  if ((threadIdx.x & 31) == 0 && mine)
+    atomicAdd(&st->served, (unsigned long long)mine);
+  __syncthreads();
+  if (threadIdx.x == 0 && nfresh) base = atomicAdd(&st->nnew, nfresh);
+  __syncthreads();
+  for (int i = threadIdx.x; i < nfresh; i += blockDim.x)
+    c.fresh[base + i] = fresh[i];
+}
+
+__global__ void __launch_bounds__(256)
+k_greedy_place(const BatchGreedyCell *__restrict__ cells,
+               const int2 *__restrict__ jobs, int par, int32_t exclude) {
+  const int2 job = jobs ? jobs[blockIdx.x] : make_int2(0, (int)blockIdx.x);
+  const BatchGreedyCell &c = cells[job.x];
+  if (c.w.g.prob == kGrid) greedy_place<kGridWalk>(c, job.y, par, exclude);
+  else if (c.w.pk) greedy_place<kPack>(c, job.y, par, exclude);
+  else greedy_place<kSlots>(c, job.y, par, exclude);
+}
+
+// every word satisfied by the placement stops counting towards the gain of
+// the candidates whose balls hold it: map[y] -= 1 for y in B(u), in pieces
+// of kRefreshPat patterns of one word shared out over the cell's blocks
+constexpr int kRefreshPat = 1024;          // four a thread of 256
+
+template <int WALK>
+__device__ __forceinline__ void greedy_refresh(const BatchGreedyCell &c) {
+  __shared__ WalkSmem s;
+  const WalkArgs &a = c.w;
+  const GreedyState *st = reinterpret_cast<const GreedyState *>(c.st);
+  const long long nseg = (a.len + kRefreshPat - 1) / kRefreshPat;
+  const long long n = st->nnew * nseg;
+  for (long long p = blockIdx.x; p < n; p += gridDim.x) {
+    const long long x0 = __ldcg(c.fresh + p / nseg);
+    const long long t0 = p % nseg * kRefreshPat;
+    const long long t1 = min(a.len, t0 + kRefreshPat);
+    __syncthreads();                      // s is reused across words
+    word_setup<WALK>(a, x0, s);
+    long long y[4];
+    int32_t old[4];
+    unsigned long long key[4];
+    const long long tt = t0 + threadIdx.x;
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      y[j] = tt + 256 * j < t1 ? walk_word<WALK>(a, x0, tt + 256 * j, s) : -1;
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (y[j] >= 0) old[j] = atomicSub(&c.map[y[j]], 1);
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (y[j] >= 0) key[j] = c.ckey[y[j] / kChunk];
+    // the chunk's best loses gain (or ties with it): its key is stale
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (y[j] >= 0 && old[j] == key_gain(key[j])) c.dirty[y[j] / kChunk] = 1;
   }
 }
 
 __global__ void __launch_bounds__(256)
-k_bgreedy_place(const BatchGreedyCell *cells, int32_t exclude) {
-  const BatchGreedyCell &c = cells[blockIdx.x];
-  if (c.w.g.prob == kGrid) bgreedy_place<true>(c, exclude);
-  else bgreedy_place<false>(c, exclude);
+k_greedy_refresh(const BatchGreedyCell *__restrict__ cells,
+                 const int *__restrict__ rebuild) {
+  if (rebuild && rebuild[blockIdx.y]) return;
+  const BatchGreedyCell &c = cells[blockIdx.y];
+  if (c.w.g.prob == kGrid) greedy_refresh<kGridWalk>(c);
+  else if (c.w.pk) greedy_refresh<kPack>(c);
+  else greedy_refresh<kSlots>(c);
 }
 
-template <bool GRID>
-__device__ __forceinline__ void bgreedy_refresh(const BatchGreedyCell &c) {
-  __shared__ WordSmem s;
-  const GreedyState *st = reinterpret_cast<const GreedyState *>(c.st);
-  if (st->done) return;
-  const int n = st->nnew;
-  for (int u = blockIdx.x; u < n; u += gridDim.x) {
-    const long long x0 = c.fresh[u];
-    __syncthreads();
-    word_setup(c.w.g, x0, s);
-    for (long long t = threadIdx.x; t < c.w.len; t += blockDim.x) {
-      const long long y = walk_word<GRID>(c.w, x0, t, s);
-      if (y >= 0) atomicSub(&c.map[y], 1);
+// ---------------------------------------------------- many steps, one launch
+// `steps` whole steps of ONE cell in a cooperative launch, a grid barrier
+// (1.2 us) between the phases.  Near a cover a phase is a few microseconds of
+// dependent L2 round trips, so what does not change is kept close: the cell
+// is a kernel parameter, the packed table and its entries sit in shared
+// memory.  On K_3(14,3) a step takes 11 us at gains of 5 and 17 us at 150;
+// the whole-map argmax, one-block place and refresh launches this replaces
+// took 49 us, the three launches above 25 us (9 of them gaps).  The grid is
+// resident as a whole (a cooperative launch) and every wait is bounded: a
+// block that has waited 2 s sets the run's error and returns, and so do the
+// others in their turn.
+struct GreedyRun {
+  unsigned arrived;             // blocks that reached a barrier so far
+  int err;
+  int pad[2];
+};
+static_assert(sizeof(GreedyRun) == kGreedyRunBytes, "run layout");
+
+// barrier number `bar` (1, 2, ...)
+__device__ __forceinline__ bool grid_barrier(GreedyRun *r, unsigned bar) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned target = bar * gridDim.x;
+    int good = 1;
+    unsigned seen;
+    unsigned long long t0 = 0;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&r->arrived)
+                 : "memory");
+    for (unsigned polls = 0;; polls++) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];"
+                   : "=r"(seen) : "l"(&r->arrived) : "memory");
+      if (seen >= target) break;
+      if ((polls & 1023u) != 1023u) continue;
+      unsigned long long now;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+      if (!t0) t0 = now;
+      if (now - t0 > 2000000000ULL) {
+        atomicExch(&r->err, 1);
+        good = 0;
+        break;
+      }
+    }
+    ok = good;
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+constexpr int kRunThreads = 256;
+constexpr int kRunWarps = kRunThreads / 32;
+constexpr int kRunPat = 128;            // patterns of one refresh piece
+constexpr int kRunTable = 8192;         // packed patterns kept in shared memory
+
+// one warp's form of word_setup
+template <int WALK>
+__device__ __forceinline__ void warp_setup(const WalkArgs &a, const int4 *ent,
+                                           long long w, WalkSmem &m) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();                         // the warp's last walk is over
+  if (WALK == kPack) {
+    for (int e = lane; e <= a.noff; e += 32) {
+      int v = 0;
+      if (e < a.noff) {
+        const int4 en = ent[e];
+        const int dg = (int)((unsigned)w / (unsigned)en.x % (unsigned)en.y);
+        v = (dg + en.z >= en.y ? en.z - en.y : en.z) * en.x;
+      }
+      m.off[e] = v;
+    }
+  } else {
+    for (int j = lane; j < a.g.n; j += 32) {
+      m.s.dig[j] = (int)((w / a.g.pw[j]) % a.g.ax[j]);
+      m.s.ax[j] = a.g.ax[j];
+      m.s.pw[j] = a.g.pw[j];
     }
   }
+  __syncwarp();
 }
 
-__global__ void __launch_bounds__(256)
-k_bgreedy_refresh(const BatchGreedyCell *cells) {
-  const BatchGreedyCell &c = cells[blockIdx.y];
-  if (c.w.g.prob == kGrid) bgreedy_refresh<true>(c);
-  else bgreedy_refresh<false>(c);
+// Each phase is shared out over the warps of the grid and needs no block
+// barrier: argmax by chunks, place by patterns (interleaved), refresh by
+// pieces of kRunPat patterns of one new word, whose updates are all in
+// flight together.  (A block refreshing its own new words saves a barrier,
+// 1.4 us, but a word's 2,969 updates by one block take 8 us.)
+template <int WALK>
+__global__ void __launch_bounds__(kRunThreads)
+k_greedy_run(const __grid_constant__ BatchGreedyCell c, int table_words,
+             int par, int steps, int32_t exclude, GreedyRun *run) {
+  extern __shared__ uint32_t table[];
+  __shared__ int4 ent[WALK == kPack ? kMaxPackOff : 1];
+  __shared__ WalkSmem smem[kRunWarps];
+  __shared__ unsigned long long wbest[kRunWarps];
+  GreedyState *st = reinterpret_cast<GreedyState *>(c.st);
+  const WalkArgs &a = c.w;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  WalkSmem &s = smem[warp];
+  // warps of the grid, the blocks' first warps first
+  const long long W = (long long)gridDim.x * kRunWarps;
+  const long long gw = (long long)warp * gridDim.x + blockIdx.x;
+  if (__ldcg(&st->done)) return;        // nobody sets it before barrier 1
+  if (WALK == kPack) {
+    if (tid < a.noff) ent[tid] = a.ent[tid];
+    for (int t = tid; t < table_words; t += kRunThreads) table[t] = a.pk[t];
+    __syncthreads();
+  }
+  auto walk = [&](long long w, long long t) -> long long {
+    if (WALK != kPack) return walk_word<WALK>(a, w, t, s);
+    const uint32_t p = table_words ? table[t] : __ldg(a.pk + t);
+    return (int32_t)w + s.off[p & 255u] + s.off[(p >> 8) & 255u] +
+           s.off[(p >> 16) & 255u] + s.off[p >> 24];
+  };
+  const long long nch = (a.g.space + kChunk - 1) / kChunk;
+  const long long nseg = (a.len + kRunPat - 1) / kRunPat;
+  unsigned bar = 0;
+  for (int i = 0; i < steps; i++, par ^= 1) {
+    // -------- argmax; block 0 commits the last placement
+    if (blockIdx.x == 0 && tid == 0) {
+      if (__ldcg(&st->pend)) {
+        st->deficit = __ldcg(&st->deficit) - (long long)__ldcg(&st->served);
+        st->placed = __ldcg(&st->placed) + 1;
+        st->pend = 0;
+      }
+      st->served = 0;
+      st->nnew = 0;
+      st->best[par ^ 1] = 0;
+    }
+    unsigned long long k = 0;
+    for (long long b = gw; b < nch; b += 32 * W) {
+      // 32 of the warp's chunks: a lane looks at each, the warp reads the
+      // stale ones
+      const long long ch = b + lane * W;
+      bool stale = false;
+      if (ch < nch) {
+        const unsigned long long key = __ldcg(c.ckey + ch);
+        stale = __ldcg(c.dirty + ch);
+        if (!stale) k = max(k, key);
+      }
+      for (unsigned m = __ballot_sync(0xffffffffu, stale); m; m &= m - 1)
+        k = max(k, read_chunk(c, b + (__ffs(m) - 1) * W));
+    }
+    for (int o = 16; o > 0; o >>= 1)
+      k = max(k, __shfl_xor_sync(0xffffffffu, k, o));
+    if (lane == 0) wbest[warp] = k;
+    __syncthreads();
+    if (tid == 0) {
+      for (int w = 1; w < kRunWarps; w++) k = max(k, wbest[w]);
+      if (k) atomicMax(&st->best[par], k);
+    }
+    if (!grid_barrier(run, ++bar)) return;
+    // -------- place: every thread of the grid reads the same verdict
+    const unsigned long long best = __ldcg(&st->best[par]);
+    const long long deficit = __ldcg(&st->deficit);
+    const int placed = __ldcg(&st->placed);
+    const long long x0 = (long long)(uint32_t)~(uint32_t)best;
+    if (best == 0 || key_gain(best) <= 0 || deficit <= 0 ||
+        placed >= c.max_add) {
+      if (blockIdx.x == 0 && tid == 0) st->done = 1;
+      return;
+    }
+    if (blockIdx.x == 0 && tid == 0) {
+      c.placed[placed] = x0;
+      st->pend = 1;
+      c.map[x0] = exclude;
+      c.dirty[x0 / kChunk] = 1;
+    }
+    if (gw < a.len) {
+      warp_setup<WALK>(a, ent, x0, s);
+      for (long long b = gw; b < a.len; b += 32 * W) {
+        const long long t = b + lane * W;
+        const long long x = t < a.len ? walk(x0, t) : -1;
+        int cv = 0x10000;
+        if (x >= 0) {
+          uint32_t *cell = reinterpret_cast<uint32_t *>(a.cnt + (x & ~1LL));
+          const int sh = (x & 1) ? 16 : 0;
+          cv = (int)((atomicAdd(cell, 1u << sh) >> sh) & 0xFFFFu);
+        }
+        const int mine = __popc(__ballot_sync(0xffffffffu, cv < a.g.mu));
+        const unsigned hit = __ballot_sync(0xffffffffu, cv == a.g.mu - 1);
+        int at = 0;
+        if (lane == 0 && mine) {
+          atomicAdd(&st->served, (unsigned long long)mine);
+          if (hit) at = atomicAdd(&st->nnew, __popc(hit));
+        }
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (cv == a.g.mu - 1)
+          c.fresh[at + __popc(hit & ((1u << lane) - 1u))] = x;
+      }
+    }
+    if (!grid_barrier(run, ++bar)) return;
+    // -------- refresh
+    const long long n = __ldcg(&st->nnew) * nseg;
+    for (long long p = gw; p < n; p += W) {
+      const long long u = __ldcg(c.fresh + p / nseg);
+      const long long t0 = p % nseg * kRunPat + lane;
+      warp_setup<WALK>(a, ent, u, s);
+      long long y[kRunPat / 32];
+      int32_t old[kRunPat / 32];
+      unsigned long long key[kRunPat / 32];
+#pragma unroll
+      for (int j = 0; j < kRunPat / 32; j++)
+        y[j] = t0 + 32 * j < a.len ? walk(u, t0 + 32 * j) : -1;
+#pragma unroll
+      for (int j = 0; j < kRunPat / 32; j++)
+        if (y[j] >= 0) old[j] = atomicSub(&c.map[y[j]], 1);
+#pragma unroll
+      for (int j = 0; j < kRunPat / 32; j++)
+        if (y[j] >= 0) key[j] = __ldcg(c.ckey + y[j] / kChunk);
+      // the chunk's best loses gain (or ties with it): its key is stale
+#pragma unroll
+      for (int j = 0; j < kRunPat / 32; j++)
+        if (y[j] >= 0 && old[j] == key_gain(key[j]))
+          c.dirty[y[j] / kChunk] = 1;
+    }
+    if (!grid_barrier(run, ++bar)) return;
+  }
 }
 
-// one step for every cell of the table
-int launch_batch_greedy_step(const BatchGreedyCell *dcells, int ncells,
-                             long long max_space, int32_t exclude,
-                             cudaStream_t s) {
-  if (ncells <= 0) return 0;
-  const dim3 ga((unsigned)((max_space + kArgmaxChunk - 1) / kArgmaxChunk),
-                (unsigned)ncells);
-  k_bgreedy_argmax<<<ga, 256, 0, s>>>(dcells);
-  k_bgreedy_place<<<(unsigned)ncells, 256, 0, s>>>(dcells, exclude);
-  k_bgreedy_refresh<<<dim3(16, (unsigned)ncells), 256, 0, s>>>(dcells);
+int launch_greedy_run(const BatchGreedyCell &cell, int par, int steps,
+                      int32_t exclude, GreedyRun *run, cudaStream_t s) {
+  const int kind = walk_kind(cell.w);
+  const void *fn = kind == kGridWalk ? (const void *)k_greedy_run<kGridWalk>
+                   : kind == kPack ? (const void *)k_greedy_run<kPack>
+                                   : (const void *)k_greedy_run<kSlots>;
+  // the packed table in shared memory where it is short
+  int table = kind == kPack && cell.w.len <= kRunTable ? (int)cell.w.len : 0;
+  // one block an SM: two or four measured slower (their barriers cost more
+  // than their warps give: 11 us a step against 14 and 18 near a cover)
+  const int grid = sm_count();
+  BatchGreedyCell c = cell;
+  // the barriers count from zero; err carries over
+  CC_CK(cudaMemsetAsync(&run->arrived, 0, sizeof(unsigned), s));
+  void *args[] = {&c, &table, &par, &steps, &exclude, &run};
+  CC_CK(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kRunThreads), args,
+                                    (size_t)table * 4, s));
+  return 0;
+}
+
+int launch_greedy_refresh(const BatchGreedyCell *dcells, int ncells,
+                          int blocks, const int *rebuild, cudaStream_t s) {
+  k_greedy_refresh<<<dim3((unsigned)blocks, (unsigned)ncells), 256, 0, s>>>(
+      dcells, rebuild);
   CC_CK(cudaGetLastError());
   return 0;
 }
 
-int launch_greedy_exclude(int32_t *map, const long long *dwords, int n,
-                          int32_t exclude, cudaStream_t s) {
-  if (n <= 0) return 0;
-  k_greedy_exclude<<<(n + 255) / 256, 256, 0, s>>>(map, dwords, n, exclude);
+int launch_greedy_argmax(const BatchGreedyCell *dcells, const int2 *jobs,
+                         int njobs, int par, int all, const int *rebuilt,
+                         cudaStream_t s) {
+  k_greedy_argmax<<<(unsigned)njobs, 32 * kBlockChunks, 0, s>>>(
+      dcells, jobs, par, all, rebuilt);
   CC_CK(cudaGetLastError());
   return 0;
 }
 
-int launch_greedy_step(const WalkArgs &w, int32_t *map, long long N,
-                       GreedyState *st, long long *placed, int max_add,
-                       long long *fresh, int32_t exclude, cudaStream_t s) {
-  long long blocks = ((N >> 2) + 255) / 256;
-  const long long cap = (long long)sm_count() * 4;
-  if (blocks > cap) blocks = cap;
-  if (blocks < 1) blocks = 1;
-  k_greedy_argmax<<<(unsigned)blocks, 256, 0, s>>>(map, N, st);
-  const bool gp = w.g.prob == kGrid;
-  if (gp)
-    k_greedy_place<true><<<1, 256, 0, s>>>(w, map, st, placed, max_add, fresh,
-                                           exclude);
-  else
-    k_greedy_place<false><<<1, 256, 0, s>>>(w, map, st, placed, max_add,
-                                            fresh, exclude);
-  const unsigned rb = (unsigned)(sm_count() * 4);
-  if (gp) k_greedy_refresh<true><<<rb, 256, 0, s>>>(w, map, st, fresh);
-  else k_greedy_refresh<false><<<rb, 256, 0, s>>>(w, map, st, fresh);
+int launch_greedy_place(const BatchGreedyCell *dcells, const int2 *jobs,
+                        int njobs, int par, int32_t exclude, cudaStream_t s) {
+  k_greedy_place<<<(unsigned)njobs, 256, 0, s>>>(dcells, jobs, par, exclude);
+  CC_CK(cudaGetLastError());
+  return 0;
+}
+
+bool greedy_rebuild_pays(long long gain, long long ball, double rebuild_us) {
+  const char *e = getenv("CC_GREEDY_REBUILD");
+  if (e) return atoi(e) != 0;
+  return (double)gain * (double)ball > kGreedyUpdatesPerUs * rebuild_us;
+}
+
+int launch_greedy_exclude(const BatchGreedyCell *dcells, int ncells,
+                          const int *rebuild, int32_t exclude,
+                          cudaStream_t s) {
+  k_greedy_exclude<<<dim3(8, (unsigned)ncells), 256, 0, s>>>(dcells, rebuild,
+                                                             exclude);
   CC_CK(cudaGetLastError());
   return 0;
 }
@@ -713,15 +1030,18 @@ int launch_update(const WalkArgs &w, const long long *dwords,
   if (nb <= 0) return 0;
   const int split = pick_split(w.len, nb);
   const dim3 grid((unsigned)nb * split);
-  const bool grid_prob = w.g.prob == kGrid;
   static WordsParam empty;
-  if (dwords) {
-    if (grid_prob) k_update<true, false><<<grid, 256, 0, s>>>(w, dwords, empty, split, delta, trans);
-    else k_update<false, false><<<grid, 256, 0, s>>>(w, dwords, empty, split, delta, trans);
-  } else {
-    if (grid_prob) k_update<true, true><<<grid, 256, 0, s>>>(w, nullptr, *pw, split, delta, trans);
-    else k_update<false, true><<<grid, 256, 0, s>>>(w, nullptr, *pw, split, delta, trans);
-  }
+#define CC_UP(W)                                                            \
+  case W:                                                                   \
+    if (dwords)                                                             \
+      k_update<W, false><<<grid, 256, 0, s>>>(w, dwords, empty, split,      \
+                                              delta, trans);                \
+    else                                                                    \
+      k_update<W, true><<<grid, 256, 0, s>>>(w, nullptr, *pw, split, delta, \
+                                             trans);                        \
+    break;
+  switch (walk_kind(w)) { CC_UP(kSlots) CC_UP(kGridWalk) CC_UP(kPack) }
+#undef CC_UP
   CC_CK(cudaGetLastError());
   return 0;
 }
@@ -755,10 +1075,12 @@ int launch_gather(const WalkArgs &w, const long long *dwords, int nb,
   if (split > 1 && !zeroed)
     CC_CK(cudaMemsetAsync(out, 0, (size_t)nb * 4, s));
   const dim3 grid((unsigned)nb * split);
-  if (w.g.prob == kGrid)
-    k_gather<true><<<grid, 256, 0, s>>>(w, dwords, split, mode, target, out);
-  else
-    k_gather<false><<<grid, 256, 0, s>>>(w, dwords, split, mode, target, out);
+#define CC_GA(W)                                                            \
+  case W:                                                                   \
+    k_gather<W><<<grid, 256, 0, s>>>(w, dwords, split, mode, target, out);  \
+    break;
+  switch (walk_kind(w)) { CC_GA(kSlots) CC_GA(kGridWalk) CC_GA(kPack) }
+#undef CC_GA
   CC_CK(cudaGetLastError());
   return 0;
 }

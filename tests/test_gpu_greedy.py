@@ -73,3 +73,65 @@ def test_searcher_device_repair_lns_is_exact():
         inc = s.uncov
         assert s.verify_full() == inc
         assert len(np.unique(s.code)) == len(s.code) <= M
+
+
+@pytest.mark.parametrize("rebuild", ["0", "1"])
+@pytest.mark.parametrize("cell", [("hamming", [2] * 10, 2, 1, 40),
+                                  ("hamming", [5, 5, 4, 10], 1, 2, 9),
+                                  ("hamming", [2] * 16, 1, 1, 3),
+                                  ("hamming", [3] * 11, 1, 2, 3),
+                                  ("torus_linf", [31, 33], 1, 1, 30),
+                                  ("grid_linf", [25, 41], 2, 1, 30),
+                                  ("lee", [4] * 5, 2, 1, 30)],
+                         ids=lambda c: f"{c[0]}-{c[1]}-mu{c[3]}")
+def test_device_greedy_by_updates_and_by_rebuilds(cell, rebuild, monkeypatch):
+    """Gains kept by updates alone and by a transform after every placement:
+    maps of just under, at and above a chunk and a block of chunks."""
+    prob, axes, R, mu, steps = cell
+    monkeypatch.setenv("CC_GREEDY_REBUILD", rebuild)
+    size = int(np.prod(axes))
+    code = np.random.default_rng(size).integers(0, size, max(1, size // 40))
+    ob = OracleBackend(axes, R, prob, mu=mu)
+    ob.recount(code)
+    want, wdef = exact_greedy(ob, code, steps)
+    with GpuBackend(axes, R, problem=prob, mu=mu) as b:
+        b.recount(code)
+        got, gdef = b.greedy_fill_device(steps)
+        assert got.tolist() == want.tolist()
+        assert gdef == wdef == b.uncovered()
+        assert np.array_equal(b.read_cnt(), ob.cnt.astype(np.uint16))
+
+
+@pytest.mark.parametrize("rebuild", ["0", "1", None])
+@pytest.mark.parametrize("steps", [1, 5, 70])
+def test_batched_greedy_by_updates_and_by_rebuilds(steps, rebuild,
+                                                   monkeypatch):
+    from coldcore_b200.batch import BatchEngine
+    from coldcore_b200.patterns import wide_table
+    if rebuild is not None:
+        monkeypatch.setenv("CC_GREEDY_REBUILD", rebuild)
+    cells = [("hamming", (3,) * 6, 2, 1), ("hamming", (4, 3, 5), 2, 2),
+             ("lee", (5,) * 5, 2, 1), ("torus_linf", (5, 7, 9), 1, 1),
+             ("grid_linf", (4, 5, 6), 2, 1), ("hamming", (2,) * 12, 1, 1),
+             ("hamming", (2,) * 16, 2, 1), ("hamming", (6,) * 2, 2, 1)]
+    with BatchEngine() as e:
+        codes = []
+        for p, a, R, mu in cells:
+            size = int(np.prod(a))
+            codes.append(np.random.default_rng(size).integers(
+                0, size, 1 + size // 200))
+            e.add(p, a, R, codes[-1], mu)
+        e.build(48)
+        for i, (p, a, R, mu) in enumerate(cells):
+            e.set_table(i, wide_table(a, R, p))
+        e.run()
+        adds = [min(steps, 5) if np.prod(c[1]) > 4096 else steps
+                for c in cells]
+        got = e.greedy(np.arange(len(cells)), adds)
+        for i, (p, a, R, mu) in enumerate(cells):
+            ob = OracleBackend(list(a), R, p, mu=mu)
+            ob.recount(codes[i])
+            want, wdef = exact_greedy(ob, codes[i], adds[i])
+            assert got[i][0].tolist() == want.tolist(), (i, p, a)
+            assert got[i][1] == wdef
+            assert np.array_equal(e.cnt(i), ob.cnt.astype(np.uint16))
