@@ -107,7 +107,8 @@ struct State {
   unsigned long long dd_last = 0;
   bool layered_out = false;        // last transform left N_0..N_R
   // set side (setside.cu): the listed predicate set Z, cached per cnt state
-  bool set_ok = false;             // support table proven == metric ball
+  bool ball_ok = false;            // support table proven == metric ball
+  bool set_ok = false;             // ... and the set side is on
   int set_policy = 1;              // DCT_SET_GATHER: 0 off, 1 auto, 2 force
   long long set_min = -1;          // DCT_SET_MIN: walk size that tries it
   long long set_ratio = 2;         // DCT_SET_RATIO: set side while |Z| <= r|B|
@@ -131,6 +132,8 @@ struct State {
   long long placed_cap = 0;
   long long *d_active = nullptr;   // active words (mu > 1: excluded again)
   long long active_cap = 0;
+  Plan gather_plan;                // a predicate's counts, untuned
+  bool gather_plan_ok = false;
   Plan plans[3][4];                // [init_mode][out_mode]
   bool plan_ok[3][4] = {{false}};
   bool tuned[3][4] = {{false}};
@@ -949,7 +952,8 @@ void set_side_init(const std::vector<int32_t> &soa, int slots) {
   S.set_policy = sp ? atoi(sp) : 1;
   S.set_min = sm ? atoll(sm) : -1;
   S.set_ratio = sr ? std::max(1LL, atoll(sr)) : 2;
-  S.set_ok = S.set_policy != 0 && table_is_ball(soa, slots, S.len);
+  S.ball_ok = table_is_ball(soa, slots, S.len);
+  S.set_ok = S.set_policy != 0 && S.ball_ok;
   S.zcap_max = std::min<long long>(S.g.space, 1LL << 27);
   S.z_mode = -1;
 }
@@ -1030,15 +1034,110 @@ int gather_launch(int mode, int target, int nb, const long long *dw,
                        bits);
 }
 
+// A transform of the predicate counts EVERY word's ball at once, so a call
+// that would walk enough of them (candidates x |B|) is a transform and a
+// read: 10^5 candidates of ternary n = 16, R = 4 walk 3.4e9 patterns in
+// 5.5 ms, the transform takes 0.48 ms.
+//
+// The counts go to the last layer plane and nothing else that a caller can
+// see changes: the launches pass 16-bit planes, which start at plane 1 and
+// leave plane 0, the map, alone, and by the last launch they end before the
+// last plane.  So: a layered cell in device memory with R >= 3, a table that
+// is the metric ball (the walk's answer), 16-bit exactness, and no exact
+// layers of an earlier call in the planes.  Returns the plan, or nullptr.
+// An untuned cell takes the streamed forms without tuning (a tuning run
+// costs hundreds of such calls, and would write the map).
+Plan *gather_transform_plan() {
+  if (S.streamed || S.layers_mode != 0 || S.cnt_mode != 0 || !S.ball_ok ||
+      S.layered_out || S.R1 < 4 || !half_planes_ok(kSrcCnt, kDstMap))
+    return nullptr;
+  Plan *P = nullptr;
+  if (S.tuned[1][1] && S.plan_ok[1][1]) {
+    P = &S.plans[1][1];
+  } else {
+    if (!S.gather_plan_ok) {
+      S.gather_plan_ok = true;
+      Knobs kn = default_knobs();
+      kn.pad = 1;
+      S.gather_plan = make_plan(1, 1, kn);
+      if (S.gather_plan.groups.empty()) {
+        S.gather_plan = make_plan(1, 1, default_knobs());
+        const char *te = getenv("CC_TMA");
+        if (!(te && atoi(te) == 0)) stream_groups(S.gather_plan.groups, S.R1);
+      }
+    }
+    P = &S.gather_plan;
+  }
+  if (P->window || P->groups.size() < 2) return nullptr;
+  for (size_t i = 0; i + 1 < P->groups.size(); i++)
+    if (!P->groups[i].a.out16 && !P->groups[i].a.out8) return nullptr;
+  const GroupArgs &last = P->groups.back().a;
+  // the last launch's source planes end before the last plane
+  if (!last.in16 || last.in8 ||
+      (long long)S.R1 * last.plane * 2 > (long long)(S.R1 - 2) * S.plane * 4)
+    return nullptr;
+  return P;
+}
+
+// Microseconds of a walk of nw candidates (k_gather_tiled over a bit plane:
+// 620,000 patterns a microsecond) against the transform: launches, and its
+// bytes at 3 TB/s.  CC_GATHER_TRANSFORM = 0 / 1 pins the choice.
+bool gather_transform_pays(const Plan &P, long long nw) {
+  const char *e = getenv("CC_GATHER_TRANSFORM");
+  if (e) return atoi(e) != 0;
+  double us = 20.0 + 5.0 * P.groups.size();
+  for (const auto &gp : P.groups) us += group_bytes(gp.a) / 3.0e6;
+  return (double)nw * (double)S.len / 6.2e5 > us;
+}
+
+int run_gather_transform(const Plan &P, int mode, int target) {
+  if (tma_fault_pending()) {
+    tma_fault_clear();
+    fprintf(stderr, "coldcore_b200: a streamed group launch timed out "
+            "waiting for its tensor loads\n");
+    return -8;
+  }
+  for (const auto &gp : P.groups) {
+    GroupPlan p = gp;
+    p.a.pmode = mode;
+    p.a.ptarget = target;
+    p.a.mu = g_mu;
+    p.a.map = S.layers + (long long)(S.R1 - 1) * S.plane;
+    const int rc = launch_group(p, g_stream);
+    if (rc) return rc;
+  }
+  return 0;
+}
+
 int gather_impl(const long long *words, int nwords, int mode, int target,
                 int32_t *out) {
   if (nwords <= 0) return 0;
   if (!out || !valid_words(words, nwords)) return -1;
+  // one route for the whole call: the set side where it serves, else the
+  // transform where that is cheaper than the walk
+  const int32_t *counts = nullptr;
+  Plan *P = (long long)nwords * S.len > (1 << 24) ? gather_transform_plan()
+                                                  : nullptr;
+  if (P && gather_transform_pays(*P, nwords)) {
+    const int nb = (int)std::min<long long>(kStageCap, nwords);
+    const int zs = want_set(mode, target, nb) ? ensure_zlist(mode, target) : 0;
+    if (zs < 0) return zs;
+    if (zs == 0) {
+      const int rc = run_gather_transform(*P, mode, target);
+      if (rc) return rc;
+      counts = S.layers + (long long)(S.R1 - 1) * S.plane;
+    }
+  }
   for (long long off = 0; off < nwords; off += kStageCap) {
     const int nb = (int)std::min<long long>(kStageCap, nwords - off);
     int rc = stage_words(words + off, nb);
     if (rc) return rc;
-    rc = gather_launch(mode, target, nb, S.d_words, S.d_out, false);
+    if (counts) {
+      S.stats[1]++;
+      rc = launch_read_at(counts, S.d_words, nb, S.d_out, g_stream);
+    } else {
+      rc = gather_launch(mode, target, nb, S.d_words, S.d_out, false);
+    }
     if (rc) return rc;
     CC_CK(cudaMemcpyAsync(S.h_out, S.d_out, (size_t)nb * 4,
                           cudaMemcpyDeviceToHost, g_stream));

@@ -909,17 +909,21 @@ k_pred_bits(const uint16_t *cnt, long long n, int mode, int target, int mu,
 template <int MAXS, bool BITS>
 __global__ void __launch_bounds__(256, 6)
 k_gather_tiled(const WalkArgs a, const long long *words, int nb, int mode,
-               int target, int32_t *out, int noff, const uint8_t *bits) {
-  constexpr int NQ = MAXS / 4;            // 64-bit words of indices a pattern
+               int target, int32_t *out, int noff, int group,
+               const uint8_t *bits) {
+  // MAXS 4: the packed table's own 8-bit indices, 32 bits a pattern; 8:
+  // 16-bit indices, two 64-bit words
+  constexpr int NQ = MAXS / 4;
   __shared__ int32_t off[kTileCand * kTileMaxOff];
-  __shared__ unsigned long long idx[kTilePat * NQ];
+  __shared__ unsigned long long idx[MAXS == 4 ? kTilePat / 2 : kTilePat * NQ];
   __shared__ int32_t base[kMaxAxes];
   __shared__ int32_t cand[kTileCand];
-  const int c0 = blockIdx.y * kTileCand;
-  const int nc = min(kTileCand, nb - c0);
+  uint32_t *idx4 = reinterpret_cast<uint32_t *>(idx);
+  const int c0 = blockIdx.y * group;
+  const int nc = min(group, nb - c0);
   const long long t0 = (long long)blockIdx.x * kTilePat;
   const int np = (int)min((long long)kTilePat, a.len - t0);
-  if (threadIdx.x == 0) {
+  if (MAXS != 4 && threadIdx.x == 0) {
     int b = 0;
     for (int j = 0; j < a.g.n; j++) { base[j] = b; b += a.g.ax[j] - 1; }
   }
@@ -933,10 +937,16 @@ k_gather_tiled(const WalkArgs a, const long long *words, int nb, int mode,
     const int c = i / (noff + 1), e = i % (noff + 1);
     int v = 0;
     if (e < noff) {
-      int j = 0;
-      while (j + 1 < a.g.n && base[j + 1] <= e) j++;
-      const int q = a.g.ax[j], dl = e - base[j] + 1;
-      const int pw = (int)a.g.pw[j];
+      int q, dl, pw;
+      if (MAXS == 4) {
+        const int4 en = __ldg(a.ent + e);
+        pw = en.x; q = en.y; dl = en.z;
+      } else {
+        int j = 0;
+        while (j + 1 < a.g.n && base[j + 1] <= e) j++;
+        q = a.g.ax[j]; dl = e - base[j] + 1;
+        pw = (int)a.g.pw[j];
+      }
       const int dg = (cand[c] / pw) % q;
       const int nd = dg + dl >= q ? dg + dl - q : dg + dl;
       v = (nd - dg) * pw;
@@ -945,6 +955,10 @@ k_gather_tiled(const WalkArgs a, const long long *words, int nb, int mode,
   }
   // the tile's patterns as offset indices
   for (int p = threadIdx.x; p < np; p += blockDim.x) {
+    if (MAXS == 4) {
+      idx4[p] = __ldg(a.pk + t0 + p);
+      continue;
+    }
 #pragma unroll
     for (int h = 0; h < NQ; h++) {
       unsigned long long wv = 0;
@@ -971,11 +985,17 @@ k_gather_tiled(const WalkArgs a, const long long *words, int nb, int mode,
 #pragma unroll 8
     for (int p = lane; p < np; p += 32) {
       int32_t x = w;
+      if (MAXS == 4) {
+        const uint32_t v = idx4[p];
+        x += oc[v & 255u] + oc[(v >> 8) & 255u] + oc[(v >> 16) & 255u] +
+             oc[v >> 24];
+      } else {
 #pragma unroll
-      for (int h = 0; h < NQ; h++) {
-        const unsigned long long wv = idx[p * NQ + h];
-        x += oc[wv & 0xFFFF] + oc[(wv >> 16) & 0xFFFF] +
-             oc[(wv >> 32) & 0xFFFF] + oc[wv >> 48];
+        for (int h = 0; h < NQ; h++) {
+          const unsigned long long wv = idx[p * NQ + h];
+          x += oc[wv & 0xFFFF] + oc[(wv >> 16) & 0xFFFF] +
+               oc[(wv >> 32) & 0xFFFF] + oc[wv >> 48];
+        }
       }
       if (BITS)
         hits += (__ldg(bits + (x >> 3)) >> (x & 7)) & 1;
@@ -1061,11 +1081,16 @@ int launch_gather(const WalkArgs &w, const long long *dwords, int nb,
                                                 target, w.g.mu, bits);
       CC_CK(cudaGetLastError());
     }
-    const dim3 tg((unsigned)((w.len + kTilePat - 1) / kTilePat),
-                  (unsigned)((nb + kTileCand - 1) / kTileCand));
+    // candidates a block shares its table tile with: 32, or a warp each when
+    // that leaves too few blocks (64 candidates x 34,113 patterns: 134 blocks
+    // of 32 candidates, 536 of 8)
+    const long long tiles = (w.len + kTilePat - 1) / kTilePat;
+    const int group = tiles * ((nb + kTileCand - 1) / kTileCand) <
+                              (long long)sm_count() * 4 ? 8 : kTileCand;
+    const dim3 tg((unsigned)tiles, (unsigned)((nb + group - 1) / group));
 #define TG(M, B) k_gather_tiled<M, B><<<tg, 256, 0, s>>>(                  \
-        w, dwords, nb, mode, target, out, noff, bits)
-    if (w.slots <= 4) { if (bits) TG(4, true); else TG(4, false); }
+        w, dwords, nb, mode, target, out, noff, group, bits)
+    if (w.pk) { if (bits) TG(4, true); else TG(4, false); }
     else { if (bits) TG(8, true); else TG(8, false); }
 #undef TG
     CC_CK(cudaGetLastError());
