@@ -69,7 +69,9 @@ def build_sparse(verbose=False, extra=()):
     the reference: ``csrc/sparse/*.cu`` -> ``libcoldcore_sparse.so``."""
     os.makedirs(OBJ, exist_ok=True)
     srcs = sorted(glob.glob(os.path.join(CSRC, "sparse", "*.cu")))
-    headers = [os.path.join(ROOT, "include", "coldcore_b200", "sparse.h")]
+    headers = [os.path.join(ROOT, "include", "coldcore_b200", "sparse.h"),
+               os.path.join(CSRC, "map_queries.cuh"),
+               os.path.join(CSRC, "query_out.h")]
     res = [_compile(s, headers, list(extra)) for s in srcs]
     objs = [o for o, _ in res]
     if verbose:

@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <vector>
 
+#include "query_out.h"
+
 namespace cc {
 
 constexpr int kMaxAxes = 40;      // |X| <= 2^40 with every axis >= 2
@@ -404,13 +406,15 @@ int launch_layers_at(const int32_t *layers, long long plane, int R1,
 
 // ------------------------------------------------------------ reductions
 int launch_cnt_reduce(const uint16_t *cnt, long long N, int mode, int target,
-                      int mu, long long *out, cudaStream_t s);
-int launch_max(const int32_t *A, long long N, long long *out, cudaStream_t s);
+                      int mu, long long *out, cudaStream_t s,
+                      RedOut r = RedOut());
+int launch_max(const int32_t *A, long long N, long long *out, cudaStream_t s,
+               RedOut r = RedOut());
 int launch_hist(const int32_t *A, long long N, int nbins, int32_t vmax,
-                int32_t *hist, cudaStream_t s);
+                int32_t *hist, cudaStream_t s, RedOut r = RedOut());
 int launch_extract(const int32_t *A, long long N, int32_t thr, void *oidx,
                    bool wide, int32_t *oval, long long cap, long long *ocount,
-                   cudaStream_t s);
+                   cudaStream_t s, RedOut r = RedOut());
 int launch_read_at(const int32_t *A, const long long *idx, int k,
                    int32_t *out, cudaStream_t s);
 int launch_scatter(int32_t *A, const long long *idx, long long M,

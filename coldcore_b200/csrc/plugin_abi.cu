@@ -287,6 +287,20 @@ int fetch_scalar(long long *r, int slot = 0) {
   return 0;
 }
 
+// a query's accumulator (d_scalar), and its result's way to the host
+constexpr int kQuerySlot = 40, kTicketSlot = 44;
+RedOut red_out(void *host = nullptr) {
+  RedOut r;
+  r.ticket = reinterpret_cast<unsigned *>(S.d_scalar + kTicketSlot);
+  r.host = host ? static_cast<long long *>(host) : S.h_scalar + kQuerySlot;
+  return r;
+}
+int query_result(long long *r) {
+  CC_CK(cudaStreamSynchronize(g_stream));
+  *r = *(volatile long long *)(S.h_scalar + kQuerySlot);
+  return 0;
+}
+
 int stage_words(const long long *words, long long nb) {
   memcpy(S.h_words, words, (size_t)nb * 8);
   CC_CK(cudaMemcpyAsync(S.d_words, S.h_words, (size_t)nb * 8,
@@ -842,6 +856,7 @@ int init_common(int problem, int n, const int *ax, int R, long long len,
                       cudaHostAllocDefault));
   CC_CK(cudaHostAlloc((void **)&S.h_scalar, 64 * 8, cudaHostAllocDefault));
   CC_CK(cudaMemsetAsync(S.d_scalar, 0, 64 * 8, g_stream));
+  CC_CK(cudaMemsetAsync(S.d_hist, 0, 4096 * 4, g_stream));
   S.bytes_dev += kStageCap * 12 + 64 * 8 + 4096 * 4;
   S.extract_cap = extract_cap;
   CC_CK(cudaMalloc(&S.d_ext32, (size_t)extract_cap * 4));
@@ -1514,12 +1529,11 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
     S.placed_cap = cap;
   }
   // the deficit to start from, and the gain map of the current cnt
-  CC_CK(cudaMemsetAsync(S.d_scalar, 0, 8, g_stream));
   int rc = launch_cnt_reduce(S.cnt, S.g.space, kPredDef, 0, mu,
-                             S.d_scalar, g_stream);
+                             S.d_scalar + kQuerySlot, g_stream, red_out());
   if (rc) return rc;
   long long d0;
-  rc = fetch_scalar(&d0);
+  rc = query_result(&d0);
   if (rc) return rc;
   *deficit = d0;
   if (max_add == 0 || d0 == 0) return 0;
@@ -1733,33 +1747,31 @@ long long dct_count_eq(int target) {
     S.stats[6]++;
     return S.z_n;
   }
-  CC_CK(cudaMemsetAsync(S.d_scalar, 0, 8, g_stream));
   int rc = launch_cnt_reduce(S.cnt, S.g.space, kPredEq, target, g_mu,
-                             S.d_scalar, g_stream);
+                             S.d_scalar + kQuerySlot, g_stream, red_out());
   if (rc) return rc;
   long long r;
-  rc = fetch_scalar(&r);
+  rc = query_result(&r);
   return rc ? rc : r;
 }
 
 long long dct_count_deficit(void) {
   if (!S.live) return -1;
-  CC_CK(cudaMemsetAsync(S.d_scalar, 0, 8, g_stream));
-  int rc = launch_cnt_reduce(S.cnt, S.g.space, kPredDef, 0, g_mu, S.d_scalar,
-                             g_stream);
+  int rc = launch_cnt_reduce(S.cnt, S.g.space, kPredDef, 0, g_mu,
+                             S.d_scalar + kQuerySlot, g_stream, red_out());
   if (rc) return rc;
   long long r;
-  rc = fetch_scalar(&r);
+  rc = query_result(&r);
   return rc ? rc : r;
 }
 
 int dct_map_max(int32_t *out) {
   if (!S.live || !out) return -1;
-  CC_CK(cudaMemsetAsync(S.d_scalar, 0, 8, g_stream));
-  int rc = launch_max(S.layers, S.g.space, S.d_scalar, g_stream);
+  int rc = launch_max(S.layers, S.g.space, S.d_scalar + kQuerySlot, g_stream,
+                      red_out());
   if (rc) return rc;
   long long r;
-  rc = fetch_scalar(&r);
+  rc = query_result(&r);
   if (rc) return rc;
   *out = (int32_t)r;
   return 0;
@@ -1767,11 +1779,9 @@ int dct_map_max(int32_t *out) {
 
 int dct_map_hist(int nbins, int32_t vmax, int32_t *out) {
   if (!S.live || nbins < 1 || nbins > 4096 || vmax < 1 || !out) return -1;
-  CC_CK(cudaMemsetAsync(S.d_hist, 0, (size_t)nbins * 4, g_stream));
-  int rc = launch_hist(S.layers, S.g.space, nbins, vmax, S.d_hist, g_stream);
+  const int rc = launch_hist(S.layers, S.g.space, nbins, vmax, S.d_hist,
+                             g_stream, red_out(S.h_out));
   if (rc) return rc;
-  CC_CK(cudaMemcpyAsync(S.h_out, S.d_hist, (size_t)nbins * 4,
-                        cudaMemcpyDeviceToHost, g_stream));
   CC_CK(cudaStreamSynchronize(g_stream));
   memcpy(out, S.h_out, (size_t)nbins * 4);
   return 0;
@@ -1782,13 +1792,12 @@ static long long extract_impl(int32_t thr, void *out_idx, bool wide,
   if (!S.live) return -1;
   if (cap > S.extract_cap) cap = (int)S.extract_cap;
   if (cap < 0) cap = 0;
-  CC_CK(cudaMemsetAsync(S.d_scalar, 0, 8, g_stream));
   void *didx = wide ? (void *)S.d_ext64 : (void *)S.d_ext32;
   int rc = launch_extract(S.layers, S.g.space, thr, didx, wide, S.d_extv, cap,
-                          S.d_scalar, g_stream);
+                          S.d_scalar + kQuerySlot, g_stream, red_out());
   if (rc) return rc;
   long long found;
-  rc = fetch_scalar(&found);
+  rc = query_result(&found);
   if (rc) return rc;
   const long long m = found < cap ? found : cap;
   if (m > 0) {

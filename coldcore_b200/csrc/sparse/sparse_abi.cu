@@ -32,6 +32,7 @@
 
 #include <cuda_runtime.h>
 
+#include "../map_queries.cuh"
 #include "coldcore_b200/sparse.h"
 
 #define SK(x)                                                               \
@@ -60,7 +61,8 @@ struct Cell {
   int32_t *w = nullptr;            // CSR incidence weights
   int32_t *uw = nullptr;           // CSR universe weights (HBM)
   int32_t *cnt = nullptr, *map = nullptr;
-  unsigned long long *acc = nullptr;   // reduction / extraction counters
+  unsigned long long *acc = nullptr;   // a query's accumulator and ticket
+  long long *h_res = nullptr;      // its result, pinned host memory
   int32_t *hist = nullptr;
   int64_t *xidx = nullptr;
   int32_t *xval = nullptr;
@@ -288,7 +290,7 @@ __device__ __forceinline__ long long warp_sum64(long long v) {
 __global__ void k_cnt_reduce(const int32_t *__restrict__ cnt,
                              const int32_t *__restrict__ uw, long long n,
                              int kind, int target, int mu,
-                             unsigned long long *acc) {
+                             unsigned long long *acc, cc::RedOut r) {
   long long s = 0;
   const long long gs = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -299,57 +301,8 @@ __global__ void k_cnt_reduce(const int32_t *__restrict__ cnt,
   }
   s = warp_sum64(s);
   if ((threadIdx.x & 31) == 0 && s) atomicAdd(acc, (unsigned long long)s);
-}
-
-__global__ void k_map_max(const int32_t *__restrict__ map, long long n,
-                          int *out) {
-  int v = 0;
-  const long long gs = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += gs)
-    v = max(v, map[i]);
-  for (int o = 16; o > 0; o >>= 1)
-    v = max(v, __shfl_down_sync(0xffffffffu, v, o));
-  if ((threadIdx.x & 31) == 0 && v > 0) atomicMax(out, v);
-}
-
-// positive v in bin (v - 1) * nbins / vmax, clipped to the last bin
-__global__ void k_hist(const int32_t *__restrict__ map, long long n,
-                       int nbins, int vmax, int32_t *hist) {
-  extern __shared__ int32_t bins[];
-  for (int b = threadIdx.x; b < nbins; b += blockDim.x) bins[b] = 0;
-  __syncthreads();
-  const long long gs = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += gs) {
-    const int v = map[i];
-    if (v > 0) {
-      long long b = (long long)(v - 1) * nbins / vmax;
-      if (b >= nbins) b = nbins - 1;
-      atomicAdd(&bins[b], 1);
-    }
-  }
-  __syncthreads();
-  for (int b = threadIdx.x; b < nbins; b += blockDim.x)
-    if (bins[b]) atomicAdd(&hist[b], bins[b]);
-}
-
-// map >= thr: slot by an atomic counter that keeps counting past cap
-__global__ void k_extract(const int32_t *__restrict__ map, long long n,
-                          int thr, int cap, int64_t *oidx, int32_t *oval,
-                          unsigned long long *count) {
-  const long long gs = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += gs) {
-    const int v = map[i];
-    if (v >= thr) {
-      const unsigned long long slot = atomicAdd(count, 1ULL);
-      if (slot < (unsigned long long)cap) {
-        oidx[slot] = i;
-        oval[slot] = v;
-      }
-    }
-  }
+  if (cc::last_block(r) && threadIdx.x == 0)
+    *r.host = (long long)atomicExch(acc, 0ULL);
 }
 
 __global__ void k_read_at(const int32_t *__restrict__ map,
@@ -404,10 +357,14 @@ int alloc_fields(int extract_cap) {
   if ((rc = alloc_dev((void **)&C.cnt, (size_t)C.nuniv * 4))) return rc;
   if ((rc = alloc_dev((void **)&C.map, (size_t)C.ncand * 4))) return rc;
   if ((rc = alloc_dev((void **)&C.acc, 16))) return rc;
+  SK(cudaHostAlloc((void **)&C.h_res, (size_t)kHistMax * 4,
+                   cudaHostAllocDefault));
+  SK(cudaMemsetAsync(C.acc, 0, 16, g_s));
   if ((rc = alloc_dev((void **)&C.hist, (size_t)kHistMax * 4))) return rc;
   C.xcap = extract_cap;
   if ((rc = alloc_dev((void **)&C.xidx, (size_t)extract_cap * 8))) return rc;
   if ((rc = alloc_dev((void **)&C.xval, (size_t)extract_cap * 4))) return rc;
+  SK(cudaMemsetAsync(C.hist, 0, (size_t)kHistMax * 4, g_s));
   SK(cudaMemsetAsync(C.cnt, 0, (size_t)C.nuniv * 4, g_s));
   SK(cudaMemsetAsync(C.map, 0, (size_t)C.ncand * 4, g_s));
   SK(cudaStreamSynchronize(g_s));
@@ -419,6 +376,7 @@ void free_all() {
   F(C.inc); F(C.indptr); F(C.w); F(C.uw); F(C.cnt); F(C.map); F(C.acc);
   F(C.hist); F(C.xidx); F(C.xval); F(C.words); F(C.out); F(C.bits);
   F(C.binom32); F(C.lev[0]); F(C.lev[1]);
+  if (C.h_res) cudaFreeHost(C.h_res);
   C = Cell();
 }
 
@@ -548,12 +506,19 @@ int update_impl(const long long *idx, long long m, int delta) {
   return 0;
 }
 
-long long read_acc() {
-  unsigned long long v = 0;
-  SK(cudaMemcpyAsync(&v, C.acc, 8, cudaMemcpyDeviceToHost, g_s));
-  SK(cudaStreamSynchronize(g_s));
-  return (long long)v;
+cc::RedOut red_out() {
+  cc::RedOut r;
+  r.ticket = reinterpret_cast<unsigned *>(C.acc + 1);
+  r.host = C.h_res;
+  return r;
 }
+
+long long query_result() {
+  SK(cudaStreamSynchronize(g_s));
+  return C.h_res[0];
+}
+
+int map_grid() { return cc::query_blocks(C.ncand / 4, C.sms); }
 
 // ------------------------------------------------- covering designs
 // C(v,k,t) rows built on the device, in the reference's layout
@@ -1071,46 +1036,39 @@ int sparse_ball_gather(const long long *idx, long long m, int target,
 
 long long sparse_count_eq(int target) {
   if (!C.live) return -1;
-  SK(cudaMemsetAsync(C.acc, 0, 8, g_s));
   k_cnt_reduce<<<grid_for(C.nuniv), kThreads, 0, g_s>>>(
-      C.cnt, nullptr, C.nuniv, 0, target, g_mu, C.acc);
+      C.cnt, nullptr, C.nuniv, 0, target, g_mu, C.acc, red_out());
   SK(cudaGetLastError());
-  return read_acc();
+  return query_result();
 }
 
 long long sparse_count_deficit(void) {
   if (!C.live) return -1;
-  SK(cudaMemsetAsync(C.acc, 0, 8, g_s));
   k_cnt_reduce<<<grid_for(C.nuniv), kThreads, 0, g_s>>>(
-      C.cnt, C.csr ? C.uw : nullptr, C.nuniv, 1, 0, g_mu, C.acc);
+      C.cnt, C.csr ? C.uw : nullptr, C.nuniv, 1, 0, g_mu, C.acc, red_out());
   SK(cudaGetLastError());
-  return read_acc();
+  return query_result();
 }
 
 int sparse_map_max(int32_t *out) {
   if (!C.live) return -1;
   if (!out) return -2;
-  SK(cudaMemsetAsync(C.acc, 0, 8, g_s));
-  k_map_max<<<grid_for(C.ncand), kThreads, 0, g_s>>>(
-      C.map, C.ncand, reinterpret_cast<int *>(C.acc));
+  cc::k_max<<<map_grid(), cc::kQueryThreads, 0, g_s>>>(
+      C.map, C.ncand, reinterpret_cast<long long *>(C.acc), red_out());
   SK(cudaGetLastError());
-  int v = 0;
-  SK(cudaMemcpyAsync(&v, C.acc, 4, cudaMemcpyDeviceToHost, g_s));
   SK(cudaStreamSynchronize(g_s));
-  *out = v;
+  *out = (int32_t)C.h_res[0];
   return 0;
 }
 
 int sparse_map_hist(int nbins, int32_t vmax, int32_t *out) {
   if (!C.live) return -1;
   if (nbins < 1 || nbins > kHistMax || vmax < 1 || !out) return -2;
-  SK(cudaMemsetAsync(C.hist, 0, (size_t)nbins * 4, g_s));
-  k_hist<<<grid_for(C.ncand), kThreads, (size_t)nbins * 4, g_s>>>(
-      C.map, C.ncand, nbins, vmax, C.hist);
+  cc::k_hist<<<map_grid(), cc::kQueryThreads, (size_t)nbins * 4, g_s>>>(
+      C.map, C.ncand, cc::bin_args(nbins, vmax), C.hist, red_out());
   SK(cudaGetLastError());
-  SK(cudaMemcpyAsync(out, C.hist, (size_t)nbins * 4, cudaMemcpyDeviceToHost,
-                     g_s));
   SK(cudaStreamSynchronize(g_s));
+  memcpy(out, C.h_res, (size_t)nbins * 4);
   return 0;
 }
 
@@ -1119,12 +1077,11 @@ long long sparse_map_extract(int32_t thr, int64_t *idx, int32_t *val,
   if (!C.live) return -1;
   if (cap > C.xcap) cap = C.xcap;
   if (cap < 0) return -2;
-  SK(cudaMemsetAsync(C.acc, 0, 8, g_s));
-  k_extract<<<grid_for(C.ncand), kThreads, 0, g_s>>>(
-      C.map, C.ncand, thr, cap, C.xidx, C.xval, C.acc);
+  cc::k_extract<int64_t><<<map_grid(), cc::kQueryThreads, 0, g_s>>>(
+      C.map, C.ncand, thr, C.xidx, C.xval, cap, C.acc, red_out());
   SK(cudaGetLastError());
-  const long long found = read_acc();
-  if (found < 0) return found;
+  SK(cudaStreamSynchronize(g_s));
+  const long long found = C.h_res[0];
   const long long m = found < cap ? found : cap;
   if (m > 0) {
     if (!idx || !val) return -2;
