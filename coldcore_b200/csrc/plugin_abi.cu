@@ -11,6 +11,7 @@
 #include <climits>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <unordered_map>
 #include <vector>
 
@@ -40,6 +41,7 @@ namespace {
 
 constexpr long long kCounterMax = 65535;    // uint16 cnt
 constexpr long long kStageCap = 1 << 16;    // words per staged chunk
+constexpr long long kExtFirst = 1 << 15;    // extracted entries in one go
 constexpr int kGreedyRing = 2;              // steps whose states are in flight
 
 struct Plan {
@@ -48,6 +50,31 @@ struct Plan {
   bool window = false;
   int scatter_plane = -1;          // window recount: plane of the code counts
 };
+
+// sorted words in pinned host memory
+struct WordBuf {
+  long long *p = nullptr;
+  long long cap = 0, n = 0;
+  int reserve(long long m) {
+    if (m <= cap) return 0;
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    const long long want = std::max<long long>(m + m / 2, 1024);
+    cap = n = 0;
+    CC_CK(cudaHostAlloc((void **)&p, (size_t)want * 8, cudaHostAllocDefault));
+    cap = want;
+    return 0;
+  }
+  long long count(long long w) const {
+    const auto r = std::equal_range(p, p + n, w);
+    return r.second - r.first;
+  }
+};
+// multiplicity -> distinct words that have it
+typedef std::map<int, long long> MultHist;
+inline int max_mult(const MultHist &h) {
+  return h.empty() ? 0 : h.rbegin()->first;
+}
 
 struct State {
   bool live = false;
@@ -83,25 +110,26 @@ struct State {
   // staging
   long long *h_words = nullptr, *d_words = nullptr;
   int32_t *h_out = nullptr, *d_out = nullptr;
+  cudaEvent_t ev_stage[2] = {nullptr};
   long long *h_scalar = nullptr, *d_scalar = nullptr;
   // one bit per word, the predicate of a large gather call (walks.cu)
   uint8_t *d_bits = nullptr;
   int32_t *d_hist = nullptr;
+  char *h_ext = nullptr;           // pinned: the first extracted entries
   uint32_t *d_ext32 = nullptr;
   int64_t *d_ext64 = nullptr;
   int32_t *d_extv = nullptr;
   long long extract_cap = 0;
-  // multisets (coldcore dct_hc.cu:46-56) + max multiplicity of `active`
-  // uploaded: the staged code, sorted; active: the represented multiset.
-  // A recount makes active = uploaded; the hash map is then built lazily,
-  // on the first call that needs per-word counts (ensure_active).
-  std::vector<long long> up_sorted;
-  std::unordered_map<long long, int> active;
-  bool active_pending = false;
+  // multisets (coldcore dct_hc.cu:46-56).  uploaded: the staged code, sorted
+  // in pinned memory (buffer `up`).  active: the represented multiset, the
+  // code of the last recount (buffer `act`) plus `delta`, what updates
+  // added and removed since.  A recount is act = up: nothing is built.
+  WordBuf code_buf[2];
+  int up = 0, act = 0;
+  bool code_in_flight = false;     // a copy from code_buf[up] may be running
+  std::unordered_map<long long, int> delta;
   long long active_size = 0;
-  int up_max = 0;
-  std::vector<int> mult_hist;      // distinct active words per multiplicity
-  int act_max = 0;
+  MultHist up_hist, act_hist;      // distinct words per multiplicity
   long long stats[8] = {0};
   long long bytes_dev = 0, bytes_host = 0;
   unsigned long long dd_last = 0;
@@ -202,78 +230,72 @@ bool within_counter(long long total, long long maxmult) {
   return b <= kCounterMax;
 }
 
-void hist_move(int from, int to) {
-  if (from > 0) S.mult_hist[from]--;
-  if (to > 0) S.mult_hist[to]++;
-  if (to > S.act_max) S.act_max = to;
-  while (S.act_max > 0 && S.mult_hist[S.act_max] == 0) S.act_max--;
-}
-
-void set_active(const std::unordered_map<long long, int> &m, long long sz) {
-  S.active_pending = false;
-  S.active = m;
-  S.active_size = sz;
-  std::fill(S.mult_hist.begin(), S.mult_hist.end(), 0);
-  S.act_max = 0;
-  for (const auto &e : m) {
-    S.mult_hist[e.second]++;
-    if (e.second > S.act_max) S.act_max = e.second;
+void hist_move(MultHist &h, int from, int to) {
+  if (from > 0) {
+    auto it = h.find(from);
+    if (--it->second == 0) h.erase(it);
   }
+  if (to > 0) ++h[to];
 }
 
-// the multiset of the last recount, as a hash map with its histogram
-void ensure_active() {
-  if (!S.active_pending) return;
-  S.active_pending = false;
-  S.active.clear();
-  S.active.reserve(S.up_sorted.size() * 2 + 1);
-  std::fill(S.mult_hist.begin(), S.mult_hist.end(), 0);
-  S.act_max = 0;
-  const auto &v = S.up_sorted;
+// the multiplicity of w in the active multiset
+int active_count(long long w) {
+  const auto it = S.delta.find(w);
+  return (int)S.code_buf[S.act].count(w) +
+         (it == S.delta.end() ? 0 : it->second);
+}
+
+// f(word, multiplicity) for every active word
+template <typename F>
+void each_active(F f) {
+  const WordBuf &b = S.code_buf[S.act];
+  for (long long i = 0; i < b.n;) {
+    long long j = i + 1;
+    while (j < b.n && b.p[j] == b.p[i]) j++;
+    const auto it = S.delta.empty() ? S.delta.end() : S.delta.find(b.p[i]);
+    const int c = (int)(j - i) + (it == S.delta.end() ? 0 : it->second);
+    if (c > 0) f(b.p[i], c);
+    i = j;
+  }
+  for (const auto &e : S.delta)
+    if (e.second > 0 && !b.count(e.first)) f(e.first, e.second);
+}
+
+// an update's distinct words and their occurrences
+typedef std::vector<std::pair<long long, int>> Batch1;
+void count_words(const long long *words, int nw, Batch1 &batch) {
+  std::vector<long long> v(words, words + nw);
+  if (!std::is_sorted(v.begin(), v.end())) std::sort(v.begin(), v.end());
   for (size_t i = 0; i < v.size();) {
     size_t j = i + 1;
     while (j < v.size() && v[j] == v[i]) j++;
-    const int c = (int)(j - i);
-    S.active.emplace(v[i], c);
-    S.mult_hist[c]++;
-    if (c > S.act_max) S.act_max = c;
+    batch.push_back({v[i], (int)(j - i)});
     i = j;
   }
-  S.active_size = (long long)v.size();
 }
 
-void apply_active(const std::unordered_map<long long, int> &batch,
-                  int delta, long long nw) {
-  ensure_active();
+void apply_active(const Batch1 &batch, int delta, long long nw) {
   for (const auto &e : batch) {
-    int &c = S.active[e.first];
-    const int before = c;
-    c += delta * e.second;
-    hist_move(before, c);
-    if (c == 0) S.active.erase(e.first);
+    const int before = active_count(e.first), d = delta * e.second;
+    int &c = S.delta[e.first];
+    c += d;
+    if (c == 0) S.delta.erase(e.first);
+    hist_move(S.act_hist, before, before + d);
   }
   S.active_size += delta * nw;
 }
 
 // validate an update batch against `active`; fills `batch`
-int check_update(const long long *words, int nw, int delta,
-                 std::unordered_map<long long, int> &batch) {
-  ensure_active();
+int check_update(const long long *words, int nw, int delta, Batch1 &batch) {
   if (!valid_words(words, nw) || (delta != 1 && delta != -1)) return -1;
-  batch.reserve((size_t)nw * 2 + 1);
-  for (int i = 0; i < nw; i++) ++batch[words[i]];
+  count_words(words, nw, batch);
   if (delta == -1) {
-    for (const auto &e : batch) {
-      auto it = S.active.find(e.first);
-      if (it == S.active.end() || it->second < e.second) return -1;
-    }
+    for (const auto &e : batch)
+      if (active_count(e.first) < e.second) return -1;
   } else {
-    long long mx = S.act_max;
-    for (const auto &e : batch) {
-      auto it = S.active.find(e.first);
-      long long m = (it == S.active.end() ? 0 : it->second) + e.second;
-      if (m > mx) mx = m;
-    }
+    long long mx = max_mult(S.act_hist);
+    for (const auto &e : batch)
+      mx = std::max(mx, (long long)active_count(e.first) + e.second);
     if (!within_counter(S.active_size + nw, mx)) return -1;
   }
   return 0;
@@ -308,6 +330,42 @@ int stage_words(const long long *words, long long nb) {
   return 0;
 }
 
+// out[i] = f(words[i]) for many words: half the staging buffers at a time,
+// so the host stages one half while the device works on the other.
+// launch(dwords, nb, dout) queues one half's work.
+template <typename F>
+int staged_words(const long long *words, long long n, int32_t *out,
+                 F launch) {
+  const long long half = kStageCap / 2;
+  const long long steps = (n + half - 1) / half;
+  auto take = [&](long long i) -> int {      // step i's answers
+    const int k = (int)(i & 1);
+    CC_CK(cudaEventSynchronize(S.ev_stage[k]));
+    memcpy(out + i * half, S.h_out + k * half,
+           (size_t)std::min(half, n - i * half) * 4);
+    return 0;
+  };
+  for (auto &ev : S.ev_stage)
+    if (!ev) CC_CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  int rc = 0;
+  for (long long i = 0; i < steps; i++) {
+    const int k = (int)(i & 1);
+    const long long nb = std::min(half, n - i * half);
+    if (i >= 2 && (rc = take(i - 2))) return rc;
+    memcpy(S.h_words + k * half, words + i * half, (size_t)nb * 8);
+    CC_CK(cudaMemcpyAsync(S.d_words + k * half, S.h_words + k * half,
+                          (size_t)nb * 8, cudaMemcpyHostToDevice, g_stream));
+    if ((rc = launch(S.d_words + k * half, (int)nb, S.d_out + k * half)))
+      return rc;
+    CC_CK(cudaMemcpyAsync(S.h_out + k * half, S.d_out + k * half,
+                          (size_t)nb * 4, cudaMemcpyDeviceToHost, g_stream));
+    CC_CK(cudaEventRecord(S.ev_stage[k], g_stream));
+  }
+  for (long long i = std::max(0LL, steps - 2); i < steps; i++)
+    if ((rc = take(i))) return rc;
+  return 0;
+}
+
 WalkArgs walk_args() {
   WalkArgs w;
   w.g = S.g;
@@ -333,12 +391,14 @@ void free_all() {
   F(S.d_words); F(S.d_out); F(S.d_scalar); F(S.d_hist); F(S.d_ext32);
   F(S.d_ext64); F(S.d_extv); F(S.zbuf); F(S.d_found);
   F(S.d_swap); F(S.d_list); FH(S.h_swap);
+  for (WordBuf &b : S.code_buf) FH(b.p);
   F(S.d_greedy); F(S.d_placed); F(S.d_active); FH(S.h_placed);
   FH(S.h_greedy);
   for (cudaEvent_t e : S.ev_greedy) if (e) cudaEventDestroy(e);
+  for (cudaEvent_t e : S.ev_stage) if (e) cudaEventDestroy(e);
   F(S.d_bits);
   FH(S.h_layers);
-  FH(S.h_words); FH(S.h_out); FH(S.h_scalar);
+  FH(S.h_words); FH(S.h_out); FH(S.h_scalar); FH(S.h_ext);
   S.~State();
   new (&S) State();
 }
@@ -511,7 +571,7 @@ int run_streamed(int init_mode, int out_mode) {
   const long long M = init_mode == 0 ? S.codeM : 0;
   const int rc = dct_b200_ooc_transform(
       S.g.prob, S.g.n, S.g.ax, S.g.R, init_mode, out_mode, g_mu,
-      M ? S.up_sorted.data() : nullptr, M, S.cnt, out, S.h_layers,
+      M ? S.code_buf[S.up].p : nullptr, M, S.cnt, out, S.h_layers,
       S.h_layers_bytes, ooc_budget(), 0, ms);
   if (rc) return rc;
   g_last_n = 0;
@@ -863,7 +923,6 @@ int init_common(int problem, int n, const int *ax, int R, long long len,
   CC_CK(cudaMalloc(&S.d_ext64, (size_t)extract_cap * 8));
   CC_CK(cudaMalloc(&S.d_extv, (size_t)extract_cap * 4));
   S.bytes_dev += (long long)extract_cap * 16;
-  S.mult_hist.assign(kCounterMax + 2, 0);
   S.live = true;
   return 0;
 }
@@ -1143,16 +1202,18 @@ int gather_impl(const long long *words, int nwords, int mode, int target,
       counts = S.layers + (long long)(S.R1 - 1) * S.plane;
     }
   }
+  if (counts) {
+    S.stats[1] += (nwords + kStageCap - 1) / kStageCap;
+    return staged_words(words, nwords, out,
+                        [&](const long long *w, int nb, int32_t *o) {
+                          return launch_read_at(counts, w, nb, o, g_stream);
+                        });
+  }
   for (long long off = 0; off < nwords; off += kStageCap) {
     const int nb = (int)std::min<long long>(kStageCap, nwords - off);
     int rc = stage_words(words + off, nb);
     if (rc) return rc;
-    if (counts) {
-      S.stats[1]++;
-      rc = launch_read_at(counts, S.d_words, nb, S.d_out, g_stream);
-    } else {
-      rc = gather_launch(mode, target, nb, S.d_words, S.d_out, false);
-    }
+    rc = gather_launch(mode, target, nb, S.d_words, S.d_out, false);
     if (rc) return rc;
     CC_CK(cudaMemcpyAsync(S.h_out, S.d_out, (size_t)nb * 4,
                           cudaMemcpyDeviceToHost, g_stream));
@@ -1316,18 +1377,35 @@ int dct_use_fmt(int fmt) {
 }
 
 int dct_set_code(const long long *idx, int M) {
-  if (!S.live || !valid_words(idx, M)) return -1;
-  std::vector<long long> sorted(idx, idx + M);
-  if (!std::is_sorted(sorted.begin(), sorted.end()))
-    std::sort(sorted.begin(), sorted.end());
-  int mx = 0;                                  // largest multiplicity
-  for (int i = 0; i < M;) {
-    int j = i + 1;
-    while (j < M && sorted[j] == sorted[i]) j++;
-    mx = std::max(mx, j - i);
-    i = j;
+  if (!S.live || M < 0 || (M && !idx)) return -1;
+  // one pass: in range, ascending, free of repeats
+  unsigned outside = 0, down = 0, same = 0;
+  const unsigned long long space = (unsigned long long)S.g.space;
+  for (int i = 0; i < M; i++) {
+    outside |= (unsigned long long)idx[i] >= space;
+    if (i) {
+      down |= idx[i] < idx[i - 1];
+      same |= idx[i] == idx[i - 1];
+    }
   }
-  if (!within_counter(M, mx)) return -1;
+  if (outside) return -1;
+  MultHist hist;
+  std::vector<long long> sorted;
+  const long long *src = idx;
+  if (down || same) {
+    sorted.assign(idx, idx + M);
+    if (down) std::sort(sorted.begin(), sorted.end());
+    for (int i = 0; i < M;) {
+      int j = i + 1;
+      while (j < M && sorted[j] == sorted[i]) j++;
+      ++hist[j - i];
+      i = j;
+    }
+    src = sorted.data();
+  } else if (M) {
+    hist[1] = M;
+  }
+  if (!within_counter(M, max_mult(hist))) return -1;
   if (M > S.code_cap) {
     if (S.d_code) cudaFree(S.d_code);
     S.d_code = nullptr;
@@ -1335,14 +1413,25 @@ int dct_set_code(const long long *idx, int M) {
     CC_CK(cudaMalloc(&S.d_code, (size_t)cap * 8));
     S.code_cap = cap;
   }
+  // the buffer that does not hold the active multiset; a copy out of it may
+  // still be on its way when the last call staged a code that no transform
+  // has used since
+  if (S.code_in_flight) CC_CK(cudaStreamSynchronize(g_stream));
+  S.code_in_flight = false;
+  const int to = S.act == S.up ? 1 - S.up : S.up;
+  WordBuf &b = S.code_buf[to];
+  int rc = b.reserve(M);
+  if (rc) return rc;
   if (M) {
-    CC_CK(cudaMemcpyAsync(S.d_code, sorted.data(), (size_t)M * 8,
+    memcpy(b.p, src, (size_t)M * 8);
+    CC_CK(cudaMemcpyAsync(S.d_code, b.p, (size_t)M * 8,
                           cudaMemcpyHostToDevice, g_stream));
-    CC_CK(cudaStreamSynchronize(g_stream));
+    S.code_in_flight = true;
   }
+  b.n = M;
+  S.up = to;
   S.codeM = M;
-  S.up_sorted.swap(sorted);
-  S.up_max = mx;
+  S.up_hist.swap(hist);
   return 0;
 }
 
@@ -1357,13 +1446,14 @@ int dct_transform(int init_mode, int out_mode) {
   rc = run_transform(init_mode, out_mode);
   if (rc) return rc;
   CC_CK(cudaStreamSynchronize(g_stream));
+  S.code_in_flight = false;
   S.layered_out = out_mode == 3;
   if (out_mode == 2) {
-    // active = uploaded; its size and largest multiplicity now, the
-    // per-word counts when a call needs them
-    S.active_pending = true;
+    // active = uploaded
+    S.act = S.up;
+    S.delta.clear();
     S.active_size = S.codeM;
-    S.act_max = S.up_max;
+    S.act_hist = S.up_hist;
     S.cnt_ver++;
   }
   return 0;
@@ -1371,7 +1461,7 @@ int dct_transform(int init_mode, int out_mode) {
 
 int dct_ball_update(const long long *words, int nwords, int delta) {
   if (!S.live) return -1;
-  std::unordered_map<long long, int> batch;
+  Batch1 batch;
   if (check_update(words, nwords, delta, batch)) return -1;
   if (nwords == 0) return 0;
   int rc = update_impl(words, nwords, delta, nullptr);
@@ -1385,7 +1475,7 @@ int dct_ball_update_delta(const long long *words, int nwords, int delta,
   if (!dd) return -1;
   *dd = 0;
   if (!S.live) return -1;
-  std::unordered_map<long long, int> batch;
+  Batch1 batch;
   if (check_update(words, nwords, delta, batch)) return -1;
   if (nwords == 0) return 0;
   auto *trans = reinterpret_cast<unsigned long long *>(S.d_scalar + 2);
@@ -1424,17 +1514,19 @@ int dct_ball_gather_mu(const long long *words, int nwords, int role,
 // error code.
 int swap_eval_fast(const long long *drops, int k, const long long *cand,
                    const long long *off, int32_t *gain, int32_t *loss) {
-  constexpr long long kMaxN = 65536;
-  // staging: [cand kMaxN x 8][drops kMaxN x 8][coff (kMaxN + 1) x 4]
-  // results: [gain kMaxN x 4][loss kMaxN x 4][nmu x 4][offs (+1) x 4]
-  //          [cursor x 4]
-  const size_t in_drop = kMaxN * 8, in_coff = 2 * kMaxN * 8;
-  const size_t in_bytes = in_coff + (kMaxN + 1) * 4;
-  const size_t r0 = in_bytes + 64;           // results start, 16-aligned
-  const size_t r_loss = r0 + kMaxN * 4, r_nmu = r_loss + kMaxN * 4;
-  const size_t r_offs = r_nmu + kMaxN * 4, r_cur = r_offs + (kMaxN + 1) * 4;
-  const size_t total_bytes = r_cur + kMaxN * 4 + 64;
+  // one staging block of what this call needs, inputs then results:
+  // [cand nc x 8][drops k x 8][coff (k + 1) x 4]
+  // [gain nc x 4][loss k x 4][nmu k x 4][offs (k + 1) x 4][cursor k x 4]
+  const long long nc = off[k];
+  const size_t in_drop = (size_t)nc * 8, in_coff = in_drop + (size_t)k * 8;
+  const size_t in_bytes = in_coff + (size_t)(k + 1) * 4;
+  const size_t r0 = (in_bytes + 15) / 16 * 16;
+  const size_t r_loss = r0 + (size_t)nc * 4, r_nmu = r_loss + (size_t)k * 4;
+  const size_t r_offs = r_nmu + (size_t)k * 4;
+  const size_t r_cur = r_offs + (size_t)(k + 1) * 4;
   if (!S.d_swap) {
+    constexpr size_t kMaxN = 65536;
+    const size_t total_bytes = kMaxN * 40 + 256;
     CC_CK(cudaMalloc(&S.d_swap, total_bytes));
     CC_CK(cudaHostAlloc((void **)&S.h_swap, total_bytes,
                         cudaHostAllocDefault));
@@ -1442,7 +1534,6 @@ int swap_eval_fast(const long long *drops, int k, const long long *cand,
                                  1LL << 22);
     CC_CK(cudaMalloc(&S.d_list, (size_t)S.lcap * 8));
   }
-  const long long nc = off[k];
   char *h = S.h_swap, *d = S.d_swap;
   if (nc) memcpy(h, cand, (size_t)nc * 8);
   memcpy(h + in_drop, drops, (size_t)k * 8);
@@ -1498,9 +1589,8 @@ int swap_eval_fast(const long long *drops, int k, const long long *cand,
 int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
   if (!S.live || max_add < 0 || (max_add && !placed) || !deficit) return -1;
   if (S.g.space >= (1LL << 32)) return -1;    // 32-bit index in the key
-  ensure_active();
   // placed words are new (multiplicity 1): the counters stay within uint16
-  if (!within_counter(S.active_size + max_add, std::max(S.act_max, 1)))
+  if (!within_counter(S.active_size + max_add, std::max(max_mult(S.act_hist), 1)))
     return -1;
   const int mu = g_mu;
   const long long nch = greedy_chunks(S.g.space);
@@ -1546,8 +1636,7 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
   const bool exclude = mu > 1 || !S.set_ok || S.fmt != 0;
   std::vector<long long> code;
   if (exclude) {
-    code.reserve(S.active.size());
-    for (const auto &e : S.active) code.push_back(e.first);
+    each_active([&](long long w, int) { code.push_back(w); });
     if ((long long)code.size() > S.active_cap) {
       if (S.d_active) CC_CK(cudaFree(S.d_active));
       S.d_active = nullptr;
@@ -1665,8 +1754,8 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
                           cudaMemcpyDeviceToHost, g_stream));
     CC_CK(cudaStreamSynchronize(g_stream));
     memcpy(placed, S.h_placed, (size_t)n * 8);
-    std::unordered_map<long long, int> batch;
-    for (int i = 0; i < n; i++) ++batch[placed[i]];
+    Batch1 batch;
+    count_words(placed, n, batch);
     apply_active(batch, +1, n);
   }
   S.cnt_ver++;
@@ -1688,9 +1777,8 @@ int dct_swap_eval(const long long *drops, int k, const long long *cand,
   const long long nc = off[k];
   if (nc > 65535 || (nc && (!cand || !gain))) return -1;
   if (!valid_words(drops, k) || !valid_words(cand, nc)) return -1;
-  ensure_active();
   for (int i = 0; i < k; i++)
-    if (S.active.find(drops[i]) == S.active.end()) return -1;
+    if (active_count(drops[i]) <= 0) return -1;
   if (S.set_ok) {
     const int rc = swap_eval_fast(drops, k, cand, off, gain, loss);
     if (rc <= 0) return rc;                  // done (0) or an error
@@ -1718,14 +1806,26 @@ int dct_swap_eval(const long long *drops, int k, const long long *cand,
 int dct_loss_owner(const long long *words, int M, int32_t *out) {
   if (!S.live || !S.owner) return -1;
   if (!valid_words(words, M) || (M && !out)) return -2;
-  std::unordered_map<long long, int> ms;
-  int mx = 0;
-  for (int i = 0; i < M; i++) mx = std::max(mx, ++ms[words[i]]);
-  if (!within_counter(M, mx)) return -2;
+  Batch1 batch;
+  count_words(words, M, batch);
+  MultHist hist;
+  for (const auto &e : batch) ++hist[e.second];
+  if (!within_counter(M, max_mult(hist))) return -2;
+  // the words become the active multiset: into the buffer that does not
+  // hold the staged code
+  const int to = S.act == S.up ? 1 - S.up : S.act;
+  if (S.code_buf[to].reserve(M)) return -2;
   CC_CK(cudaMemsetAsync(S.cnt, 0, (size_t)S.cnt_len * 2, g_stream));
   int rc = update_impl(words, M, +1, nullptr);
   if (rc) return rc;
-  set_active(ms, M);
+  long long *p = S.code_buf[to].p;
+  for (const auto &e : batch)
+    for (int i = 0; i < e.second; i++) *p++ = e.first;
+  S.code_buf[to].n = M;
+  S.act = to;
+  S.delta.clear();
+  S.active_size = M;
+  S.act_hist.swap(hist);
   if (M == 0) return 0;
   int lm, lt;
   mode_role(1, &lm, &lt);
@@ -1796,14 +1896,35 @@ static long long extract_impl(int32_t thr, void *out_idx, bool wide,
   int rc = launch_extract(S.layers, S.g.space, thr, didx, wide, S.d_extv, cap,
                           S.d_scalar + kQuerySlot, g_stream, red_out());
   if (rc) return rc;
+  // the first entries come back with the count, through pinned memory; a
+  // larger answer's rest is copied once the count is known
+  const size_t isz = wide ? 8 : 4;
+  const long long first = std::min<long long>(cap, kExtFirst);
+  if (first && !S.h_ext)
+    CC_CK(cudaHostAlloc((void **)&S.h_ext, (size_t)kExtFirst * 12,
+                        cudaHostAllocDefault));
+  char *hv = S.h_ext + (size_t)kExtFirst * 8;
+  if (first) {
+    CC_CK(cudaMemcpyAsync(S.h_ext, didx, (size_t)first * isz,
+                          cudaMemcpyDeviceToHost, g_stream));
+    CC_CK(cudaMemcpyAsync(hv, S.d_extv, (size_t)first * 4,
+                          cudaMemcpyDeviceToHost, g_stream));
+  }
   long long found;
   rc = query_result(&found);
   if (rc) return rc;
   const long long m = found < cap ? found : cap;
-  if (m > 0) {
-    CC_CK(cudaMemcpyAsync(out_idx, didx, (size_t)m * (wide ? 8 : 4),
-                          cudaMemcpyDeviceToHost, g_stream));
-    CC_CK(cudaMemcpyAsync(out_val, S.d_extv, (size_t)m * 4,
+  const long long m0 = std::min(m, first);
+  if (m0 > 0) {
+    memcpy(out_idx, S.h_ext, (size_t)m0 * isz);
+    memcpy(out_val, hv, (size_t)m0 * 4);
+  }
+  if (m > m0) {
+    CC_CK(cudaMemcpyAsync(static_cast<char *>(out_idx) + m0 * isz,
+                          static_cast<char *>(didx) + m0 * isz,
+                          (size_t)(m - m0) * isz, cudaMemcpyDeviceToHost,
+                          g_stream));
+    CC_CK(cudaMemcpyAsync(out_val + m0, S.d_extv + m0, (size_t)(m - m0) * 4,
                           cudaMemcpyDeviceToHost, g_stream));
     CC_CK(cudaStreamSynchronize(g_stream));
   }
@@ -1823,18 +1944,10 @@ int dct_map_read_at(const long long *idx, int k, int32_t *out) {
   if (!S.live) return -1;
   if (k <= 0) return 0;
   if (!out || !valid_words(idx, k)) return -1;
-  for (long long off = 0; off < k; off += kStageCap) {
-    const int nb = (int)std::min<long long>(kStageCap, k - off);
-    int rc = stage_words(idx + off, nb);
-    if (rc) return rc;
-    rc = launch_read_at(S.layers, S.d_words, nb, S.d_out, g_stream);
-    if (rc) return rc;
-    CC_CK(cudaMemcpyAsync(S.h_out, S.d_out, (size_t)nb * 4,
-                          cudaMemcpyDeviceToHost, g_stream));
-    CC_CK(cudaStreamSynchronize(g_stream));
-    memcpy(out + off, S.h_out, (size_t)nb * 4);
-  }
-  return 0;
+  return staged_words(idx, k, out,
+                      [](const long long *w, int nb, int32_t *o) {
+                        return launch_read_at(S.layers, w, nb, o, g_stream);
+                      });
 }
 
 int dct_read_cnt(long long off, long long len, uint16_t *out) {
