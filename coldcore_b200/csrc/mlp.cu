@@ -5,8 +5,8 @@
 // mma.sync m16n8k16 (bf16 x bf16 -> f32); the 128-wide output layer, the
 // loss and the Adam step are FP32 SIMT.
 //
-// One CTA owns 64 samples and every weight (the whole net is 20,865
-// parameters: W1 and W2 sit in shared memory as bf16).  Forward:
+// A CTA takes blocks of 64 samples and holds every weight (the whole net is
+// 20,865 parameters: W1 and W2 sit in shared memory as bf16).  Forward:
 //   h1 = bf16(relu(bf16(x) W1b + b1)), h2 = bf16(relu(h1 W2b + b2)),
 //   y = h2 . w3 + b3;
 // training loss: binary cross-entropy with logits against t in {0,1},
@@ -20,6 +20,7 @@
 // gradient check.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <unordered_map>
@@ -36,193 +37,228 @@ constexpr int kW1 = 0, kB1 = kW1 + kIn * kHid, kW2 = kB1 + kHid,
               kB2 = kW2 + kHid * kHid, kW3 = kB2 + kHid, kB3 = kW3 + kHid,
               kParams = kB3 + 1;
 
+// Rows of the shared tiles are padded by 8 bf16 (272 and 80 bytes): the eight
+// rows of an 8 x 8 matrix start in different banks, so every ldmatrix is free
+// of conflicts.  h2 becomes dz2 and h1 becomes dz1 in place, each after its
+// last reader.
+constexpr int kThreads = 512, kWarps = kThreads / 32;
+constexpr int kLdH = kHid + 8, kLdX = kIn + 8;
 struct MlpSmem {
-  __nv_bfloat16 w1[kIn * kHid];      // [in][hid]
-  __nv_bfloat16 w2[kHid * kHid];     // [in][out]
-  __nv_bfloat16 x[kRows * kIn];
-  __nv_bfloat16 h1[kRows * kHid];
-  __nv_bfloat16 h2[kRows * kHid];
-  __nv_bfloat16 dz2[kRows * kHid];
-  __nv_bfloat16 dz1[kRows * kHid];
+  __nv_bfloat16 w1[kIn * kLdH];      // [in][hid]
+  __nv_bfloat16 w2[kHid * kLdH];     // [in][out]
+  __nv_bfloat16 x[kRows * kLdX];
+  __nv_bfloat16 h1[kRows * kLdH];    // then dz1
+  __nv_bfloat16 h2[kRows * kLdH];    // then dz2
   float b1[kHid], b2[kHid], w3[kHid];
   float y[kRows], dy[kRows];
   float b3;
 };
 
-__device__ __forceinline__ uint32_t pack2(__nv_bfloat16 lo,
-                                          __nv_bfloat16 hi) {
-  return (uint32_t)__bfloat16_as_ushort(lo) |
-         ((uint32_t)__bfloat16_as_ushort(hi) << 16);
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t *>(&v);
 }
 
-// C[16x8] += A[16xK] B[Kx8] with A(i, k), B(k, n) read through accessors,
-// K a multiple of 16; one warp, fragments as the m16n8k16 .bf16 layout
-// defines them (g = lane / 4, t = lane % 4).
-template <typename FA, typename FB>
-__device__ __forceinline__ void warp_mma(FA A, FB B, int K, float c[4]) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  for (int k0 = 0; k0 < K; k0 += 16) {
-    const uint32_t a0 = pack2(A(g, k0 + 2 * t), A(g, k0 + 2 * t + 1));
-    const uint32_t a1 = pack2(A(g + 8, k0 + 2 * t), A(g + 8, k0 + 2 * t + 1));
-    const uint32_t a2 = pack2(A(g, k0 + 2 * t + 8), A(g, k0 + 2 * t + 9));
-    const uint32_t a3 = pack2(A(g + 8, k0 + 2 * t + 8),
-                              A(g + 8, k0 + 2 * t + 9));
-    const uint32_t b0 = pack2(B(k0 + 2 * t, g), B(k0 + 2 * t + 1, g));
-    const uint32_t b1 = pack2(B(k0 + 2 * t + 8, g), B(k0 + 2 * t + 9, g));
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 "
-        "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+// four 8 x 8 matrices; lane l gives the address of row l % 8 of matrix l / 8
+__device__ __forceinline__ void ldm4(uint32_t (&r)[4], const void *p) {
+  asm volatile(
+      "ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+      : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldm4t(uint32_t (&r)[4], const void *p) {
+  asm volatile(
+      "ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+      : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4],
+                                    uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 "
+      "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// One warp: C[16 x 8 NT] += A[16 x K] B[K x 8 NT], from shared memory.
+// TA: A(i, k) is stored [k][i], else [i][k]; TB: B(k, j) is stored [j][k],
+// else [k][j].  A and B point at the warp's first row and column.
+template <int K, int NT, bool TA, bool TB>
+__device__ __forceinline__ void warp_gemm(const __nv_bfloat16 *A, int lda,
+                                          const __nv_bfloat16 *B, int ldb,
+                                          float (&c)[NT][4]) {
+  static_assert(NT % 2 == 0, "B comes two column tiles at a time");
+  const int lane = threadIdx.x & 31, r = lane & 7, q = lane >> 3;
+#pragma unroll
+  for (int k = 0; k < K; k += 16) {
+    uint32_t a[4];
+    // matrices: (i 0-7, k 0-7), (i 8-15, k 0-7), (i 0-7, k 8-15), (8-15, 8-15)
+    if (TA) ldm4t(a, A + (k + (q >> 1) * 8 + r) * lda + (q & 1) * 8);
+    else ldm4(a, A + ((q & 1) * 8 + r) * lda + k + (q >> 1) * 8);
+#pragma unroll
+    for (int n = 0; n < NT; n += 2) {
+      uint32_t b[4];
+      // matrices: (k 0-7, n 0-7), (k 8-15, n 0-7), and both for n 8-15
+      if (TB) ldm4(b, B + (8 * n + (q >> 1) * 8 + r) * ldb + k + (q & 1) * 8);
+      else ldm4t(b, B + (k + (q & 1) * 8 + r) * ldb + 8 * n + (q >> 1) * 8);
+      mma(c[n], a, b[0], b[1]);
+      mma(c[n + 1], a, b[2], b[3]);
+    }
   }
 }
 
-// element (row, col) of the warp's C fragment register r
-__device__ __forceinline__ void frag_pos(int r, int *row, int *col) {
+// c[n][2 h + v] is row g + 8 h, column 8 n + 2 t + v of the warp's block
+template <int NT, typename F>
+__device__ __forceinline__ void each_pair(const float (&c)[NT][4], F f) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  *row = g + (r >= 2 ? 8 : 0);
-  *col = 2 * t + (r & 1);
+#pragma unroll
+  for (int n = 0; n < NT; n++)
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+      f(g + 8 * h, 8 * n + 2 * t, c[n][2 * h], c[n][2 * h + 1]);
 }
 
+// h[rows m0.., cols n0..] = bf16(relu(A W + b)), 16 x 32 of it per warp
+template <int K>
+__device__ __forceinline__ void hidden_layer(const __nv_bfloat16 *A, int lda,
+                                             const __nv_bfloat16 *W,
+                                             const float *bias,
+                                             __nv_bfloat16 *h) {
+  const int warp = threadIdx.x >> 5;
+  const int m0 = (warp & 3) * 16, n0 = (warp >> 2) * 32;
+  float c[4][4] = {};
+  warp_gemm<K, 4, false, false>(A + m0 * lda, lda, W + n0, kLdH, c);
+  each_pair(c, [&](int i, int j, float u, float v) {
+    u += bias[n0 + j];
+    v += bias[n0 + j + 1];
+    *reinterpret_cast<uint32_t *>(h + (m0 + i) * kLdH + n0 + j) =
+        pack2(u > 0.f ? u : 0.f, v > 0.f ? v : 0.f);
+  });
+}
+
+__device__ __forceinline__ void add2(float *p, float u, float v) {
+  asm volatile("red.global.add.v2.f32 [%0], {%1, %2};\n" ::"l"(p), "f"(u),
+               "f"(v)
+               : "memory");
+}
+
+// One CTA of 16 warps takes blocks of 64 samples, one an SM at most, with the
+// weights in shared memory throughout; the weight gradients stay in registers
+// (40 a thread) until its last block, so a gradient vector is added to memory
+// once per CTA.  Fragments are loaded with ldmatrix: built from two-byte
+// shared loads, as they were, the gradient over 20,000 samples took 172 us
+// (two CTAs an SM, 313 of them, 6.5 M atomics); it takes 28 us.
 template <bool TRAIN>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kThreads, 1)
 k_mlp(const float *P, const __nv_bfloat16 *w1b, const __nv_bfloat16 *w2b,
       const float *X, const float *T, int n, float scale, float *out_y,
       float *G) {
   extern __shared__ __align__(16) unsigned char smraw[];
   MlpSmem &s = *reinterpret_cast<MlpSmem *>(smraw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int r0 = blockIdx.x * kRows;
-  for (int i = tid; i < kIn * kHid; i += blockDim.x) s.w1[i] = w1b[i];
-  for (int i = tid; i < kHid * kHid; i += blockDim.x) s.w2[i] = w2b[i];
-  for (int i = tid; i < kHid; i += blockDim.x) {
+  for (int i = tid; i < kIn * kHid / 8; i += kThreads)
+    *reinterpret_cast<uint4 *>(s.w1 + (i / 16) * kLdH + (i % 16) * 8) =
+        reinterpret_cast<const uint4 *>(w1b)[i];
+  for (int i = tid; i < kHid * kHid / 8; i += kThreads)
+    *reinterpret_cast<uint4 *>(s.w2 + (i / 16) * kLdH + (i % 16) * 8) =
+        reinterpret_cast<const uint4 *>(w2b)[i];
+  for (int i = tid; i < kHid; i += kThreads) {
     s.b1[i] = P[kB1 + i];
     s.b2[i] = P[kB2 + i];
     s.w3[i] = P[kW3 + i];
   }
   if (tid == 0) s.b3 = P[kB3];
-  for (int i = tid; i < kRows * kIn; i += blockDim.x) {
-    const int r = i / kIn;
-    s.x[i] = __float2bfloat16(r0 + r < n ? X[(long long)r0 * kIn + i] : 0.f);
-  }
-  __syncthreads();
-  // ---- layer 1: 64 x 128 outputs = 4 x 16 tiles, 8 per warp, K = 32
-  for (int tile = warp; tile < 64; tile += 8) {
-    const int m0 = (tile >> 4) * 16, n0 = (tile & 15) * 8;
-    float c[4] = {0, 0, 0, 0};
-    warp_mma([&](int i, int k) { return s.x[(m0 + i) * kIn + k]; },
-             [&](int k, int j) { return s.w1[k * kHid + n0 + j]; }, kIn, c);
-    for (int r = 0; r < 4; r++) {
-      int row, col;
-      frag_pos(r, &row, &col);
-      const float z = c[r] + s.b1[n0 + col];
-      s.h1[(m0 + row) * kHid + n0 + col] = __float2bfloat16(z > 0.f ? z : 0.f);
+  // gradients of this CTA's blocks: dW2 rows 16 (warp % 8), columns
+  // 64 (warp / 8); dW1 rows 16 (warp % 2), columns 16 (warp / 2); a column
+  // and a quarter of the rows a thread for the vectors
+  float gw2[8][4] = {}, gw1[2][4] = {};
+  float gw3 = 0.f, gb2 = 0.f, gb1 = 0.f, gb3 = 0.f;
+  const int m2 = (warp & 7) * 16, n2 = (warp >> 3) * 64;
+  const int m1 = (warp & 1) * 16, n1 = (warp >> 1) * 16;
+  const int col = tid & (kHid - 1), rq = tid / kHid * (kRows / 4);
+  const int blocks = (n + kRows - 1) / kRows;
+  for (int blk = blockIdx.x; blk < blocks; blk += gridDim.x) {
+    const int r0 = blk * kRows;
+    {
+      const int r = tid >> 3, c = (tid & 7) * 4;       // 64 rows x 8 float4
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r0 + r < n)
+        v = *reinterpret_cast<const float4 *>(X + (long long)(r0 + r) * kIn +
+                                              c);
+      *reinterpret_cast<uint2 *>(s.x + r * kLdX + c) =
+          make_uint2(pack2(v.x, v.y), pack2(v.z, v.w));
     }
-  }
-  __syncthreads();
-  // ---- layer 2: 64 x 128, K = 128
-  for (int tile = warp; tile < 64; tile += 8) {
-    const int m0 = (tile >> 4) * 16, n0 = (tile & 15) * 8;
-    float c[4] = {0, 0, 0, 0};
-    warp_mma([&](int i, int k) { return s.h1[(m0 + i) * kHid + k]; },
-             [&](int k, int j) { return s.w2[k * kHid + n0 + j]; }, kHid, c);
-    for (int r = 0; r < 4; r++) {
-      int row, col;
-      frag_pos(r, &row, &col);
-      const float z = c[r] + s.b2[n0 + col];
-      s.h2[(m0 + row) * kHid + n0 + col] = __float2bfloat16(z > 0.f ? z : 0.f);
+    __syncthreads();
+    hidden_layer<kIn>(s.x, kLdX, s.w1, s.b1, s.h1);
+    __syncthreads();
+    hidden_layer<kHid>(s.h1, kLdH, s.w2, s.b2, s.h2);
+    __syncthreads();
+    // output layer and the loss gradient: a warp per row
+    for (int r = warp; r < kRows; r += kWarps) {
+      float acc = 0.f;
+#pragma unroll
+      for (int c = 0; c < kHid; c += 64) {
+        const int j = c + 2 * lane;
+        const float2 h = __bfloat1622float2(
+            *reinterpret_cast<const __nv_bfloat162 *>(s.h2 + r * kLdH + j));
+        acc += h.x * s.w3[j] + h.y * s.w3[j + 1];
+      }
+      for (int o = 16; o > 0; o >>= 1)
+        acc += __shfl_down_sync(0xffffffffu, acc, o);
+      if (lane == 0) {
+        const float y = acc + s.b3;
+        const bool in = r0 + r < n;
+        if (in && out_y) out_y[r0 + r] = y;
+        if (TRAIN)
+          s.dy[r] = in ? (1.f / (1.f + expf(-y)) - T[r0 + r]) * scale : 0.f;
+      }
     }
-  }
-  __syncthreads();
-  // ---- output layer: one warp per row
-  for (int r = warp; r < kRows; r += 8) {
-    float acc = 0.f;
-    for (int c = lane; c < kHid; c += 32)
-      acc += __bfloat162float(s.h2[r * kHid + c]) * s.w3[c];
-    for (int o = 16; o > 0; o >>= 1)
-      acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if (lane == 0) {
-      s.y[r] = acc + s.b3;
-      if (r0 + r < n && out_y) out_y[r0 + r] = s.y[r];
+    __syncthreads();
+    if (!TRAIN) continue;
+    // dw3, db2, db3; dz2 in place of h2
+    for (int r = rq; r < rq + kRows / 4; r++) {
+      __nv_bfloat16 *p = s.h2 + r * kLdH + col;
+      const float h = __bfloat162float(*p), d = s.dy[r];
+      gw3 += d * h;
+      const __nv_bfloat16 dz = __float2bfloat16(h > 0.f ? d * s.w3[col] : 0.f);
+      *p = dz;
+      gb2 += __bfloat162float(dz);
+      if (col == 0) gb3 += d;
     }
+    __syncthreads();
+    // dW2 += h1^T dz2, and dz1 = dz2 W2^T where h1 > 0
+    warp_gemm<kRows, 8, true, false>(s.h1 + m2, kLdH, s.h2 + n2, kLdH, gw2);
+    const int m0 = (warp & 3) * 16, n0 = (warp >> 2) * 32;
+    float c[4][4] = {};
+    warp_gemm<kHid, 4, false, true>(s.h2 + m0 * kLdH, kLdH, s.w2 + n0 * kLdH,
+                                    kLdH, c);
+    __syncthreads();                     // h1's last readers are through
+    each_pair(c, [&](int i, int j, float u, float v) {
+      __nv_bfloat162 *p = reinterpret_cast<__nv_bfloat162 *>(
+          s.h1 + (m0 + i) * kLdH + n0 + j);
+      const float2 h = __bfloat1622float2(*p);
+      *reinterpret_cast<uint32_t *>(p) =
+          pack2(h.x > 0.f ? u : 0.f, h.y > 0.f ? v : 0.f);
+    });
+    __syncthreads();
+    // db1, dW1 += x^T dz1
+    for (int r = rq; r < rq + kRows / 4; r++)
+      gb1 += __bfloat162float(s.h1[r * kLdH + col]);
+    warp_gemm<kRows, 2, true, false>(s.x + m1, kLdX, s.h1 + n1, kLdH, gw1);
+    __syncthreads();                     // the next block's x, h1, h2
   }
   if (!TRAIN) return;
-  __syncthreads();
-  // ---- loss gradient
-  for (int r = tid; r < kRows; r += blockDim.x) {
-    float d = 0.f;
-    if (r0 + r < n) {
-      const float p = 1.f / (1.f + expf(-s.y[r]));
-      d = (p - T[r0 + r]) * scale;
-    }
-    s.dy[r] = d;
-  }
-  __syncthreads();
-  // dw3, db3, dz2, db2
-  for (int c = tid; c < kHid; c += blockDim.x) {
-    float gw = 0.f, gb = 0.f;
-    for (int r = 0; r < kRows; r++) {
-      const float h = __bfloat162float(s.h2[r * kHid + c]);
-      gw += s.dy[r] * h;
-      const __nv_bfloat16 dz =
-          __float2bfloat16(h > 0.f ? s.dy[r] * s.w3[c] : 0.f);
-      s.dz2[r * kHid + c] = dz;
-      gb += __bfloat162float(dz);
-    }
-    atomicAdd(G + kW3 + c, gw);
-    atomicAdd(G + kB2 + c, gb);
-  }
-  if (tid == 0) {
-    float gb3 = 0.f;
-    for (int r = 0; r < kRows; r++) gb3 += s.dy[r];
-    atomicAdd(G + kB3, gb3);
-  }
-  __syncthreads();
-  // ---- dW2 = h1^T dz2: 128 x 128 = 8 x 16 tiles, 16 per warp, K = 64
-  for (int tile = warp; tile < 128; tile += 8) {
-    const int m0 = (tile >> 4) * 16, n0 = (tile & 15) * 8;
-    float c[4] = {0, 0, 0, 0};
-    warp_mma([&](int i, int k) { return s.h1[k * kHid + m0 + i]; },
-             [&](int k, int j) { return s.dz2[k * kHid + n0 + j]; }, kRows, c);
-    for (int r = 0; r < 4; r++) {
-      int row, col;
-      frag_pos(r, &row, &col);
-      atomicAdd(G + kW2 + (m0 + row) * kHid + n0 + col, c[r]);
-    }
-  }
-  // ---- dz1 = (dz2 W2^T) masked: 64 x 128, K = 128
-  for (int tile = warp; tile < 64; tile += 8) {
-    const int m0 = (tile >> 4) * 16, n0 = (tile & 15) * 8;
-    float c[4] = {0, 0, 0, 0};
-    warp_mma([&](int i, int k) { return s.dz2[(m0 + i) * kHid + k]; },
-             [&](int k, int j) { return s.w2[(n0 + j) * kHid + k]; }, kHid, c);
-    for (int r = 0; r < 4; r++) {
-      int row, col;
-      frag_pos(r, &row, &col);
-      const int at = (m0 + row) * kHid + n0 + col;
-      s.dz1[at] = __float2bfloat16(
-          __bfloat162float(s.h1[at]) > 0.f ? c[r] : 0.f);
-    }
-  }
-  __syncthreads();
-  // db1
-  for (int c = tid; c < kHid; c += blockDim.x) {
-    float gb = 0.f;
-    for (int r = 0; r < kRows; r++) gb += __bfloat162float(s.dz1[r * kHid + c]);
-    atomicAdd(G + kB1 + c, gb);
-  }
-  // ---- dW1 = x^T dz1: 32 x 128 = 2 x 16 tiles, 4 per warp, K = 64
-  for (int tile = warp; tile < 32; tile += 8) {
-    const int m0 = (tile >> 4) * 16, n0 = (tile & 15) * 8;
-    float c[4] = {0, 0, 0, 0};
-    warp_mma([&](int i, int k) { return s.x[k * kIn + m0 + i]; },
-             [&](int k, int j) { return s.dz1[k * kHid + n0 + j]; }, kRows, c);
-    for (int r = 0; r < 4; r++) {
-      int row, col;
-      frag_pos(r, &row, &col);
-      atomicAdd(G + kW1 + (m0 + row) * kHid + n0 + col, c[r]);
-    }
-  }
+  each_pair(gw2, [&](int i, int j, float u, float v) {
+    add2(G + kW2 + (m2 + i) * kHid + n2 + j, u, v);
+  });
+  each_pair(gw1, [&](int i, int j, float u, float v) {
+    add2(G + kW1 + (m1 + i) * kHid + n1 + j, u, v);
+  });
+  atomicAdd(G + kW3 + col, gw3);
+  atomicAdd(G + kB2 + col, gb2);
+  atomicAdd(G + kB1 + col, gb1);
+  if (col == 0) atomicAdd(G + kB3, gb3);
 }
 
 // Adam on the fp32 master copy; refreshes the bf16 copies of W1 / W2 and
@@ -294,12 +330,12 @@ int launch_mlp(Mlp *m, bool train, const float *X, const float *T, int n,
                                (int)smem));
     attr = true;
   }
-  const int grid = (n + kRows - 1) / kRows;
+  const int grid = std::min((n + kRows - 1) / kRows, cc::sm_count());
   if (train)
-    k_mlp<true><<<grid, 256, smem, m->s>>>(m->P, m->w1b, m->w2b, X, T, n,
+    k_mlp<true><<<grid, kThreads, smem, m->s>>>(m->P, m->w1b, m->w2b, X, T, n,
                                            scale, Y, m->G);
   else
-    k_mlp<false><<<grid, 256, smem, m->s>>>(m->P, m->w1b, m->w2b, X, T, n,
+    k_mlp<false><<<grid, kThreads, smem, m->s>>>(m->P, m->w1b, m->w2b, X, T, n,
                                             scale, Y, m->G);
   CC_CK(cudaGetLastError());
   return 0;
