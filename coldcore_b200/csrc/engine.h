@@ -256,11 +256,15 @@ int launch_batch_groups(const BatchLaunch &b, cudaStream_t s);
 // resident CTAs of that kernel over the whole GPU, opted in to `smem` bytes
 int batch_groups_grid(int kernel, size_t smem);
 
-// window pass (torus / grid) over one axis, any width, out of place
+// window pass (torus / grid) over one axis, or (q2) that axis and the next,
+// any width, out of place
+constexpr int kWindowPairMaxR = 3;
+bool window_pair_ok(long long stride, int q, int R);
 struct WindowArgs {
   const int32_t *src32; const uint16_t *src16; int pmode, ptarget, mu;
   int32_t *dst32; uint16_t *dst16;
   long long space, stride; int q, R, grid;
+  int q2;                   // size of the next axis (0: one axis)
 };
 int launch_window(const WindowArgs &w, cudaStream_t s);
 

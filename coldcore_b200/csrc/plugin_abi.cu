@@ -483,7 +483,14 @@ Plan build_window_plan(int init_mode, int out_mode) {
   Plan P;
   P.window = true;
   const Geometry &g = S.g;
-  const int n = g.n;
+  // passes: two axes at a time where the pair form applies
+  std::vector<std::pair<int, int>> axes;        // (first, how many)
+  for (int j = 0; j < g.n;) {
+    const int k = j + 1 < g.n && window_pair_ok(g.pw[j], g.ax[j], g.R) ? 2 : 1;
+    axes.push_back({j, k});
+    j += k;
+  }
+  const int n = (int)axes.size();
   std::vector<int> buf(n + 1);
   buf[0] = init_mode == 0 ? 2 : -1;
   P.scatter_plane = init_mode == 0 ? 2 : -1;
@@ -502,10 +509,11 @@ Plan build_window_plan(int init_mode, int out_mode) {
     w.pmode = kPredEq;
     w.mu = g_mu;
     w.space = g.space;
-    w.stride = g.pw[j];
-    w.q = g.ax[j];
+    w.stride = g.pw[axes[j].first];
+    w.q = g.ax[axes[j].first];
     w.R = g.R;
     w.grid = g.prob == kGrid;
+    w.q2 = axes[j].second == 2 ? g.ax[axes[j].first + 1] : 0;
     P.passes.push_back(w);
   }
   return P;
@@ -1975,11 +1983,14 @@ int dct_b200_plan(int init_mode, int out_mode, long long *info, int cap) {
   const long long X = S.g.space;
   int n = 0;
   if (P.window) {
+    int axis = 0;
     for (size_t i = 0; i < P.passes.size(); i++, n++) {
       const WindowArgs &w = P.passes[i];
       const long long by = X * ((w.src16 ? 2 : 4) + (w.dst16 ? 2 : 4));
+      const int first = axis, many = w.q2 ? 2 : 1;
+      axis += many;
       if (info && 4 * n + 3 < cap) {
-        info[4 * n] = (long long)i; info[4 * n + 1] = 1;
+        info[4 * n] = first; info[4 * n + 1] = many;
         info[4 * n + 2] = by; info[4 * n + 3] = -2;
       }
     }
