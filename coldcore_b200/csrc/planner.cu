@@ -320,25 +320,36 @@ std::vector<GroupPlan> group_variants(const GroupPlan &p, int R1,
   return out;
 }
 
-// The padded plan of a cell whose first group has an odd word count T0
-// (ternary): the first group writes its 16-bit layers at a pitch of P0 =
+// axes of the widest streamed group of a padded plan (its middle extent at
+// most 256, the tensor map's box limit); 0: none
+int pad_max_axes(int prob, int q) {
+  if (prob == kHamming && q == 3) return 5;
+  if (q == 4) return 4;
+  if (q == 5 || q == 6) return 3;
+  if (prob == kLee && q == 7) return 2;
+  return 0;
+}
+
+// The padded plan of a cell whose first group has a word count T0 that is no
+// multiple of 64 (or is one, of an axis size without another streamed form):
+// the first group writes its 16-bit layers at a pitch of P0 =
 // round_up(T0, 64) words a row, so every later group's rows start on 128-
 // byte boundaries and run as streamed launches over packed pairs; the last
 // writes the map or cnt back at the canonical index.  The axes after the
-// first group are split evenly into groups of at most kPadMaxAxes (the
-// widest streamed ternary group), and the first group takes the packed
-// row-pair form where it applies.  false when the cell does not qualify or
+// first group are split evenly into groups of at most pad_max_axes, and a
+// ternary first group takes the packed row-pair form where it applies.  false when the cell does not qualify or
 // the padded planes do not fit the room16 u16 words of the allocation.
-constexpr int kPadMaxAxes = 5;
-
 bool pad_plan(std::vector<GroupPlan> &groups, const Geometry &g,
               const PlanPtrs &ptr, int dst, int R1, long long room16) {
-  if (groups.size() < 2 || g.prob != kHamming) return false;
+  if (groups.size() < 2 || (g.prob != kHamming && g.prob != kLee))
+    return false;
   GroupPlan &f = groups[0];
   const GroupArgs &a0 = f.a;
   if (f.kernel < 0 || a0.inner != 1 || a0.W != 1 || !a0.out16 || a0.pack ||
-      a0.pair_axis || (a0.mid & 1) == 0)
+      a0.pair_axis)
     return false;
+  const int most = pad_max_axes(g.prob, g.ax[a0.k < g.n ? a0.k : 0]);
+  if (!most) return false;
   const int k0 = a0.k;
   const int rem = g.n - k0;
   if (rem < 1) return false;
@@ -352,7 +363,7 @@ bool pad_plan(std::vector<GroupPlan> &groups, const Geometry &g,
   // room16: the u16 words from the start of the 16-bit planes on
   if ((long long)R1 * plane16 > room16) return false;
   std::vector<GroupPlan> later;
-  const int nch = (rem + kPadMaxAxes - 1) / kPadMaxAxes;
+  const int nch = (rem + most - 1) / most;
   // one group per range: the budget only has to admit its K axes
   const Knobs kn{(size_t)1 << 30, 0, 1, 0, 0};
   long long reach = 0;

@@ -35,372 +35,10 @@
 #include <unordered_map>
 
 #include "engine.h"
+#include "tma_group.cuh"
 
 namespace cc {
 namespace {
-
-constexpr size_t kTmaSmemMax = 227 * 1024;
-constexpr unsigned long long kTmaWaitNs = 2000000000ULL;   // 2 s
-constexpr unsigned long long kTmaDrainNs = 200000000ULL;   // 0.2 s
-
-template <int Q, int E>
-struct P { static constexpr int v = Q * P<Q, E - 1>::v; };
-template <int Q>
-struct P<Q, 0> { static constexpr int v = 1; };
-
-// ------------------------------------------------------------ PTX helpers
-__device__ __forceinline__ uint32_t saddr(const void *p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint64_t *bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(saddr(bar))
-               : "memory");
-}
-__device__ __forceinline__ void mbar_expect(uint64_t *bar, uint32_t bytes) {
-  asm volatile(
-      "mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(
-          saddr(bar)),
-      "r"(bytes)
-      : "memory");
-}
-__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n"
-      " mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(saddr(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ unsigned long long now_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-// true once the phase of `parity` has completed; false after `limit` ns
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity,
-                                          unsigned long long limit) {
-  if (mbar_test(bar, parity)) return true;
-  const unsigned long long t0 = now_ns();
-  for (unsigned it = 1;; it++) {
-    if (mbar_test(bar, parity)) return true;
-    if ((it & 255) == 0 && now_ns() - t0 > limit) return false;
-  }
-}
-__device__ __forceinline__ void tma_load4(void *dst, const CUtensorMap *map,
-                                          uint64_t *bar, int c0, int c1,
-                                          int c2, int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::"
-      "complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(
-          saddr(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2),
-      "r"(c3), "r"(saddr(bar))
-      : "memory");
-}
-
-// ------------------------------------------------------------ axis math
-// One Hamming axis over a register block: the fibres are the Q entries at
-// element stride ST; layers descend so layer d-1 is read before it changes.
-template <int Q, int R1, int QB, int ST>
-__device__ __forceinline__ void ham_axis(uint32_t (&v)[R1][QB]) {
-#pragma unroll
-  for (int e = 0; e < QB; e++) {
-    if ((e / ST) % Q != 0) continue;
-#pragma unroll
-    for (int d = R1 - 1; d >= 1; d--) {
-      if (Q == 2) {
-        const uint32_t a0 = v[d - 1][e], a1 = v[d - 1][e + ST];
-        v[d][e] += a1;
-        v[d][e + ST] += a0;
-      } else {
-        const uint32_t a0 = v[d - 1][e], a1 = v[d - 1][e + ST],
-                       a2 = v[d - 1][e + 2 * ST];
-        v[d][e] += a1 + a2;
-        v[d][e + ST] += a0 + a2;
-        v[d][e + 2 * ST] += a0 + a1;
-      }
-    }
-  }
-}
-
-template <int Q, int R1, int B, int T>
-struct Axes {
-  static __device__ __forceinline__ void run(uint32_t (&v)[R1][P<Q, B>::v]) {
-    ham_axis<Q, R1, P<Q, B>::v, P<Q, T>::v>(v);
-    Axes<Q, R1, B, T + 1>::run(v);
-  }
-};
-template <int Q, int R1, int B>
-struct Axes<Q, R1, B, B> {
-  static __device__ __forceinline__ void run(uint32_t (&)[R1][P<Q, B>::v]) {}
-};
-
-// axes per register round: Q^b x R1 registers at most 64
-template <int Q, int R1>
-struct RoundAxes {
-  static constexpr int v = (P<Q, 4>::v * R1 <= 64) ? 4
-                           : (P<Q, 3>::v * R1 <= 64) ? 3
-                           : (P<Q, 2>::v * R1 <= 64) ? 2 : 1;
-};
-
-// Epilogue reductions of a streamed launch's output (TmaArgs::red_mode): 2
-// the map maximum, 1 the deficit sum max(0, mu - c) of the cnt written; a
-// packed lane's two words, each only where it is a word of the cell.
-__device__ __forceinline__ void tma_red(long long *acc, const TmaArgs &a,
-                                        int w0, int w1, bool ok0, bool ok1) {
-  if (a.red_mode == 2) {
-    if (ok0 && w0 > *acc) *acc = w0;
-    if (ok1 && w1 > *acc) *acc = w1;
-  } else {
-    if (ok0 && w0 < a.mu) *acc += a.mu - w0;
-    if (ok1 && w1 < a.mu) *acc += a.mu - w1;
-  }
-}
-
-// ------------------------------------------------------------ one round
-// Round over axes [A, A + B) of the group on a stage of L lanes x MID mid
-// positions x R1 layers (32-bit packed lanes, layer-major as the tensor
-// load lays it down).  FIRST: layers >= lin start at zero.  LAST: the
-// block goes to HBM (OUT 0 layers, 1 map, 2 cnt) instead of the stage.
-template <int Q, int K, int R1, int L, int OUT, int A, int B, bool FIRST,
-          bool LAST, bool IN8 = false>
-__device__ __forceinline__ void tma_round(uint32_t *st, const TmaArgs &a,
-                                          long long o, long long i0,
-                                          const uint16_t *s8 = nullptr,
-                                          long long *racc = nullptr) {
-  constexpr int MID = P<Q, K>::v;
-  constexpr int QB = P<Q, B>::v;
-  constexpr int QA = P<Q, A>::v;
-  constexpr int NB = L * MID / QB;            // register blocks in the tile
-  for (int blk = threadIdx.x; blk < NB; blk += blockDim.x) {
-    const int l = blk % L;
-    const int rest = blk / L;                 // mid digits outside [A, A+B)
-    const int mb = rest % QA + (rest / QA) * (QA * QB);
-    uint32_t *p = st + mb * L + l;
-    uint32_t v[R1][QB];
-    if (IN8 && FIRST) {
-      // the staged 8-bit planes: one 16-bit read gives the lane's two
-      // words, widened to the two 16-bit halves of the packed lane
-      const uint16_t *p8 = s8 + mb * L + l;
-#pragma unroll
-      for (int d = 0; d < R1; d++) {
-        const bool live = d < a.lin;
-#pragma unroll
-        for (int e = 0; e < QB; e++)
-          v[d][e] = live ? __byte_perm((uint32_t)p8[(d * MID + e * QA) * L],
-                                       0u, 0x4140)
-                         : 0u;
-      }
-    } else {
-#pragma unroll
-      for (int d = 0; d < R1; d++) {
-        const bool live = !FIRST || d < a.lin;
-#pragma unroll
-        for (int e = 0; e < QB; e++)
-          v[d][e] = live ? p[(d * MID + e * QA) * L] : 0u;
-      }
-    }
-    Axes<Q, R1, B, 0>::run(v);
-    if (!LAST) {
-#pragma unroll
-      for (int d = 0; d < R1; d++)
-#pragma unroll
-        for (int e = 0; e < QB; e++) p[(d * MID + e * QA) * L] = v[d][e];
-      continue;
-    }
-    // HBM word of element e: o*(MID*inner) + (mb + e*QA)*inner + i0 + 2l
-    const long long x0 = (o * MID + mb) * a.inner + i0 + 2 * l;
-    const long long step = (long long)QA * a.inner;
-    if (OUT == 0) {
-#pragma unroll
-      for (int d = 0; d < R1; d++) {
-        if (d >= a.lout) break;
-        uint16_t *q = a.layers16 + d * a.plane + x0;
-#pragma unroll
-        for (int e = 0; e < QB; e++)
-          __stcs(reinterpret_cast<unsigned *>(q + e * step), v[d][e]);
-      }
-    } else if (OUT == 1 || OUT == 2) {
-#pragma unroll
-      for (int e = 0; e < QB; e++) {
-        uint32_t s = 0;
-#pragma unroll
-        for (int d = 0; d < R1; d++) s += v[d][e];
-        if (OUT == 1)
-          __stcs(reinterpret_cast<int2 *>(a.map + x0 + e * step),
-                 make_int2((int)(s & 0xFFFFu), (int)(s >> 16)));
-        else
-          *reinterpret_cast<unsigned *>(a.cnt + x0 + e * step) = s;
-        if (racc)
-          tma_red(racc, a, (int)(s & 0xFFFFu), (int)(s >> 16), true, true);
-      }
-    } else {
-      // OUT 3 (map) / 4 (cnt) of a padded plan: the pair's words j', j'+1
-      // of the padded inner go back to the canonical index, padding dropped
-      const long long jp = i0 + 2 * l;
-      const long long r = jp / a.pitch, i = jp - r * a.pitch;
-      const bool ok0 = i < a.t0, ok1 = i + 1 < a.t0;
-      const long long xc = (o * MID + mb) * a.inner_c + r * a.t0 + i;
-      const long long stepc = (long long)QA * a.inner_c;
-#pragma unroll
-      for (int e = 0; e < QB; e++) {
-        uint32_t s = 0;
-#pragma unroll
-        for (int d = 0; d < R1; d++) s += v[d][e];
-        const long long x = xc + e * stepc;
-        if (OUT == 3) {
-          if (ok0) __stcs(a.map + x, (int)(s & 0xFFFFu));
-          if (ok1) __stcs(a.map + x + 1, (int)(s >> 16));
-        } else {
-          if (ok0) a.cnt[x] = (uint16_t)(s & 0xFFFFu);
-          if (ok1) a.cnt[x + 1] = (uint16_t)(s >> 16);
-        }
-        if (racc) tma_red(racc, a, (int)(s & 0xFFFFu), (int)(s >> 16), ok0, ok1);
-      }
-    }
-  }
-}
-
-// The rounds of a K-axis group: RoundAxes-sized rounds from axis 0 up (or
-// BMX axes a round: smaller register blocks, twice the blocks a round, for
-// twice the threads), the remainder last.
-template <int Q, int K, int R1, int L, int OUT, int A, bool IN8 = false,
-          int BMX = 0>
-struct Rounds {
-  static constexpr int BM = BMX ? BMX : RoundAxes<Q, R1>::v;
-  static constexpr int B = (K - A) < BM ? (K - A) : BM;
-  static __device__ __forceinline__ void run(uint32_t *st, const TmaArgs &a,
-                                             long long o, long long i0,
-                                             const uint16_t *s8 = nullptr,
-                                             long long *racc = nullptr) {
-    tma_round<Q, K, R1, L, OUT, A, B, A == 0, A + B == K, IN8>(st, a, o, i0,
-                                                              s8, racc);
-    if (A + B < K) __syncthreads();
-    Rounds<Q, K, R1, L, OUT, (A + B < K ? A + B : K), IN8, BMX>::run(
-        st, a, o, i0, s8, racc);
-  }
-};
-template <int Q, int K, int R1, int L, int OUT, bool IN8, int BMX>
-struct Rounds<Q, K, R1, L, OUT, K, IN8, BMX> {
-  static __device__ __forceinline__ void run(uint32_t *, const TmaArgs &,
-                                             long long, long long,
-                                             const uint16_t *,
-                                             long long * = nullptr) {}
-};
-
-// stage stride: the tile's words rounded up to 1 KB (tensor loads land on
-// 128-byte-aligned shared addresses)
-template <int Q, int K, int R1, int L>
-struct Stage {
-  static constexpr int words = (R1 * P<Q, K>::v * L + 255) / 256 * 256;
-};
-// 8-bit staged planes: a stage is R1 x mid x 2L bytes (1 KB multiples),
-// and the rounds run on one 32-bit work buffer of the Stage size
-template <int Q, int K, int R1, int L>
-struct Stage8 {
-  static constexpr int bytes = (R1 * P<Q, K>::v * 2 * L + 1023) / 1024 * 1024;
-};
-
-template <int Q, int K, int R1, int L, int OUT, bool IN8 = false,
-          int BMX = 0>
-__global__ void __launch_bounds__(512)
-tma_group(const __grid_constant__ CUtensorMap map, const TmaArgs a) {
-  extern __shared__ __align__(128) uint8_t dyn[];
-  constexpr int MID = P<Q, K>::v;
-  constexpr int SW = Stage<Q, K, R1, L>::words;
-  // bytes a stage: the 16-bit planes' tile, or the 8-bit planes' tile
-  constexpr int SB = IN8 ? Stage8<Q, K, R1, L>::bytes : SW * 4;
-  const int S = a.stages;
-  // stages on a 1 KB boundary, then (8-bit planes) the work buffer, then
-  // the barriers and the stop flag
-  uint8_t *base = dyn + ((1024u - (saddr(dyn) & 1023u)) & 1023u);
-  uint8_t *stage = base;
-  uint32_t *work = IN8 ? reinterpret_cast<uint32_t *>(base + (size_t)S * SB)
-                       : nullptr;
-  uint64_t *bar = reinterpret_cast<uint64_t *>(
-      base + (size_t)S * SB + (IN8 ? (size_t)SW * 4 : 0));
-  volatile int *stop = reinterpret_cast<volatile int *>(bar + kTmaMaxStages);
-  const uint32_t bytes = (uint32_t)(2 * L * (IN8 ? 1 : 2)) * MID * a.lin;
-  long long acc = 0;                    // epilogue reduction (red_mode)
-  long long *racc = (OUT != 0 && a.red_mode) ? &acc : nullptr;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < S; s++) mbar_init(&bar[s]);
-    *stop = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
-  __syncthreads();
-  const long long grid = gridDim.x;
-  auto issue = [&](long long t, int s) {
-    const int i0 = (int)((t % a.nchunk) * (2 * L));
-    const int o = (int)(t / a.nchunk);
-    mbar_expect(&bar[s], bytes);
-    tma_load4(stage + (size_t)s * SB, &map, &bar[s], i0, 0, o, 0);
-  };
-  if (threadIdx.x == 0) {
-    asm volatile("prefetch.tensormap [%0];\n" ::"l"(
-                     reinterpret_cast<uint64_t>(&map))
-                 : "memory");
-    for (int s = 0; s < S; s++) {
-      const long long t = blockIdx.x + s * grid;
-      if (t < a.ntiles) issue(t, s);
-    }
-  }
-  long long it = 0;
-  long long t = blockIdx.x;
-  for (; t < a.ntiles; it++, t += grid) {
-    const int s = (int)(it % S);
-    const uint32_t parity = (uint32_t)((it / S) & 1);
-    if (!mbar_wait(&bar[s], parity, kTmaWaitNs)) *stop = 1;
-    __syncthreads();
-    if (*stop) break;
-    const long long o = t / a.nchunk;
-    const long long i0 = (t % a.nchunk) * (2 * L);
-    if (IN8)
-      Rounds<Q, K, R1, L, OUT, 0, IN8, BMX>::run(
-          work, a, o, i0,
-          reinterpret_cast<const uint16_t *>(stage + (size_t)s * SB), racc);
-    else
-      Rounds<Q, K, R1, L, OUT, 0, false, BMX>::run(
-          reinterpret_cast<uint32_t *>(stage + (size_t)s * SB), a, o, i0,
-          nullptr, racc);
-    __syncthreads();                          // stage s is free again
-    if (threadIdx.x == 0) {
-      const long long nt = t + S * grid;
-      if (nt < a.ntiles) {
-        // the rounds wrote the stage through the generic proxy; order those
-        // writes before the tensor load overwrites it
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        issue(nt, s);
-      }
-    }
-  }
-  if (t < a.ntiles && threadIdx.x == 0) {
-    // a load never completed: report, then wait (bounded) for every load
-    // this CTA still has outstanding before the CTA's memory goes away
-    *a.fault = 1;
-    __threadfence_system();
-    for (long long k = it; k < it + S; k++) {
-      const long long tk = blockIdx.x + k * grid;
-      if (tk >= a.ntiles) break;
-      mbar_wait(&bar[k % S], (uint32_t)((k / S) & 1), kTmaDrainNs);
-    }
-  }
-  if (racc) {
-    for (int o2 = 16; o2 > 0; o2 >>= 1) {
-      const long long other = __shfl_down_sync(0xffffffffu, acc, o2);
-      acc = a.red_mode == 2 ? (other > acc ? other : acc) : acc + other;
-    }
-    if ((threadIdx.x & 31) == 0 && acc) {
-      if (a.red_mode == 2)
-        atomicMax((unsigned long long *)a.red, (unsigned long long)acc);
-      else
-        atomicAdd((unsigned long long *)a.red, (unsigned long long)acc);
-    }
-  }
-}
 
 // ------------------------------------------------------------ first group
 // The first group of a binary Hamming cell read from cnt: a tile is the
@@ -837,11 +475,6 @@ tern_first(const TmaArgs a) {
 }
 
 // ------------------------------------------------------------ dispatch
-typedef void (*TmaFn)(const CUtensorMap, const TmaArgs);
-
-struct TmaEntry { int q, k, r1, lanes, out; TmaFn fn; int in8 = 0;
-                  int bm = 0; };
-
 #define TE(Q, K, R1, L)                                                     \
   {Q, K, R1, L, 0, tma_group<Q, K, R1, L, 0>},                              \
   {Q, K, R1, L, 1, tma_group<Q, K, R1, L, 1>},                              \
@@ -919,13 +552,29 @@ int out_code(const GroupArgs &a) {
   return (a.pitch && out) ? out + 2 : out;
 }
 
-const TmaEntry *find_tma(int q, int k, int r1, int lanes, int out,
-                         int in8 = 0, int bm = 0) {
-  for (const auto &e : kTma)
-    if (e.q == q && e.k == k && e.r1 == r1 && e.lanes == lanes &&
+// every instance, this file's first
+constexpr int kTmaHere = sizeof(kTma) / sizeof(kTma[0]);
+const TmaEntry &tma_entry(int i) {
+  return i < kTmaHere ? kTma[i] : tma_table_q(nullptr)[i - kTmaHere];
+}
+int tma_entries() {
+  int n = 0;
+  tma_table_q(&n);
+  return kTmaHere + n;
+}
+int axis_kind(int prob, int q) { return prob == kLee ? 32 + q : q; }
+
+// index of an instance, -1 when there is none
+int find_tma(int kind, int k, int r1, int lanes, int out, int in8 = 0,
+             int bm = 0) {
+  static const int n = tma_entries();
+  for (int i = 0; i < n; i++) {
+    const TmaEntry &e = tma_entry(i);
+    if (e.kind == kind && e.k == k && e.r1 == r1 && e.lanes == lanes &&
         e.out == out && e.in8 == (in8 ? 1 : 0) && e.bm == bm)
-      return &e;
-  return nullptr;
+      return i;
+  }
+  return -1;
 }
 
 // the first group's OUT: 0 16-bit layers, 5 8-bit layers, 1 map, 2 cnt
@@ -991,17 +640,18 @@ size_t tma_smem_bytes(int q, int k, int r1, int lanes, int stages,
   return (size_t)stages * words * 4 + 1024 + kTmaMaxStages * 8 + 16;
 }
 
-// The groups the streamed form serves: binary Hamming groups over 16-bit
-// planes in packed pairs (an even inner stride) (16-bit planes, the map or cnt out),
-// one tile per W inner words x the whole group, an instantiated (q, k,
+// The groups the streamed form serves: Hamming (q <= 6) and Lee (q <= 7) groups
+// over 16-bit planes in packed pairs (an even inner stride), 16-bit planes, the
+// map or cnt out, one tile per W inner words x the whole group, an instantiated (q, k,
 // layers, lanes) and its stages within 227 KB of shared memory.
 bool tma_group_ok(const GroupArgs &a, int q, int r1, int lanes, int stages) {
   // one stage: a CTA small enough for two a SM, whose loads then overlap
   // the other CTA's rounds
   if (stages < 1 || stages > kTmaMaxStages || !encode_fn()) return false;
   const int out = out_code(a);
-  if (!find_tma(q, a.k, r1, lanes, out, a.in8, a.tbm)) return false;
-  if (a.prob != kHamming || !a.pack || !a.in16 || a.pair_axis ||
+  if (find_tma(axis_kind(a.prob, q), a.k, r1, lanes, out, a.in8, a.tbm) < 0)
+    return false;
+  if ((a.prob != kHamming && a.prob != kLee) || !a.pack || !a.in16 || a.pair_axis ||
       a.src != kSrcLayers || a.R + 1 != r1)
     return false;
   if (out == 0 && !a.out16) return false;
@@ -1156,21 +806,21 @@ int tern_opt_in(const TernEntry *e) {
   return 0;
 }
 
-const TmaEntry *entry_of(const GroupPlan &p) {
+int entry_of(const GroupPlan &p) {
   const GroupArgs &a = p.a;
   const int out = out_code(a);
-  return find_tma(a.rq[0] ? a.rq[0] : a.qax[0], a.k, a.R + 1, a.W / 2, out,
-                  a.in8, a.tbm);
+  return find_tma(axis_kind(a.prob, a.rq[0] ? a.rq[0] : a.qax[0]), a.k,
+                  a.R + 1, a.W / 2, out, a.in8, a.tbm);
 }
 
 // opt every streamed kernel in to the largest dynamic shared memory once
-int opt_in(const TmaEntry *e) {
+int opt_in(int idx) {
   static std::mutex mu;
-  static bool done[sizeof(kTma) / sizeof(kTma[0])];
+  static std::vector<bool> done;
   std::lock_guard<std::mutex> g(mu);
-  const size_t idx = (size_t)(e - kTma);
+  if (done.empty()) done.resize(tma_entries(), false);
   if (!done[idx]) {
-    CC_CK(cudaFuncSetAttribute((const void *)e->fn,
+    CC_CK(cudaFuncSetAttribute((const void *)tma_entry(idx).fn,
                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kTmaSmemMax));
     done[idx] = true;
@@ -1192,9 +842,8 @@ int tma_prepare(const GroupPlan &p) {
     const FirstEntry *f = first_of(p);
     return f ? first_opt_in(f) : -9;
   }
-  const TmaEntry *e = entry_of(p);
-  if (!e) return -9;
-  return opt_in(e);
+  const int e = entry_of(p);
+  return e < 0 ? -9 : opt_in(e);
 }
 
 int tma_blocks_per_sm(const GroupPlan &p) {
@@ -1208,9 +857,9 @@ int tma_blocks_per_sm(const GroupPlan &p) {
     if (!f || first_opt_in(f)) return 0;
     fn = (const void *)f->fn;
   } else {
-    const TmaEntry *e = entry_of(p);
-    if (!e || opt_in(e)) return 0;
-    fn = (const void *)e->fn;
+    const int e = entry_of(p);
+    if (e < 0 || opt_in(e)) return 0;
+    fn = (const void *)tma_entry(e).fn;
   }
   int n = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
@@ -1353,9 +1002,9 @@ int launch_tma_group(const GroupPlan &p, cudaStream_t s) {
   const GroupArgs &a = p.a;
   const int q = a.rq[0] ? a.rq[0] : a.qax[0];
   const int lanes = a.W / 2;
-  const TmaEntry *e = entry_of(p);
+  const int e = entry_of(p);
   PFN_cuTensorMapEncodeTiled_v12000 enc = encode_fn();
-  if (!e || !enc || a.stages < 1 || a.stages > kTmaMaxStages) return -9;
+  if (e < 0 || !enc || a.stages < 1 || a.stages > kTmaMaxStages) return -9;
   int *fault = nullptr;
   if (fault_word(&fault)) return -9;
   int rc = opt_in(e);
@@ -1427,7 +1076,7 @@ int launch_tma_group(const GroupPlan &p, cudaStream_t s) {
     grid = (int)(gr < 1 ? 1 : gr);
   }
   grid = grid_knob(grid, a.ntiles);
-  e->fn<<<grid, p.threads, smem, s>>>(map, t);
+  tma_entry(e).fn<<<grid, p.threads, smem, s>>>(map, t);
   CC_CK(cudaGetLastError());
   return 0;
 }

@@ -199,3 +199,44 @@ def test_three_axis_rounds_in_the_eight_axis_group(monkeypatch, axes, R, mu,
             assert np.array_equal(b.map_all(), o.map), step
         plan = b.plan(1, 1)
         assert [int(r[1]) for r in plan[:2]] == [12, 8], plan
+
+
+@pytest.mark.parametrize("problem,q,ns", [
+    ("hamming", 4, (7, 9)), ("hamming", 5, (5, 7)), ("hamming", 6, (5, 7)),
+    ("lee", 4, (7, 9)), ("lee", 5, (5, 7)), ("lee", 6, (5, 6)),
+    ("lee", 7, (5, 6))])
+@pytest.mark.parametrize("R,mu", [(1, 1), (2, 2), (3, 1), (4, 1)])
+def test_streamed_groups_of_larger_axes_match_the_oracle(monkeypatch, problem,
+                                                         q, ns, R, mu):
+    """The padded plan of Hamming q = 4..6 and Lee q = 4..7: one and two later
+    groups of one to four axes, rows that end in padding and rows that do not,
+    tile budgets that move the split.  (At R = 1 the 16-bit planes fill their
+    region, so only rows without padding stream.)"""
+    from oracle.cport import CPortCell
+    monkeypatch.setenv("CC_TMA", "1")
+    monkeypatch.setenv("CC_TUNE", "0")
+    used = 0
+    for n in ns:
+        axes = [q] * n
+        size = q ** n
+        rng = np.random.default_rng(size % 997 + R)
+        code = rng.integers(0, size, size=max(4, size // 300))
+        code = np.concatenate([code, code[:2]])
+        o = CPortCell(axes, R, problem, mu=mu)
+        o.recount(code)
+        cnt = o.cnt.copy()
+        o.gain_map()
+        gain = o.map.copy()
+        o.loss_map()
+        for kb in (20, 40, 100):
+            monkeypatch.setenv("CC_SMEM_BUDGET_KB", str(kb))
+            with GpuBackend(axes, R, problem=problem, mu=mu) as b:
+                b.recount(code)
+                assert np.array_equal(b.read_cnt(), cnt), (n, kb)
+                b.gain_map()
+                assert np.array_equal(b.map_all(), gain), (n, kb)
+                b.loss_map()
+                assert np.array_equal(b.map_all(), o.map), (n, kb)
+                used += sum(int(np.count_nonzero(b.plan_forms(im, om) & TMA))
+                            for im, om in ((0, 2), (1, 1), (2, 1)))
+    assert used > 0 or R == 1, "no launch took the streamed form"
