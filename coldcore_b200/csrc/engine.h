@@ -220,8 +220,8 @@ size_t tma_first_smem_bytes(int kk, int r1, int stages);
 bool tma_first_ok(const GroupArgs &a, int r1, int stages);
 GroupPlan tma_first_variant(const GroupPlan &p, int stages, int threads);
 // the first group of a ternary Hamming cell over row pairs, a.tma == 3
-bool tern_first_ok(const GroupArgs &a, int r1);
-GroupPlan tern_first_variant(const GroupPlan &p, int threads);
+bool rows_first_ok(const GroupArgs &a, int r1);
+GroupPlan rows_first_variant(const GroupPlan &p, int threads);
 int launch_tma_group(const GroupPlan &p, cudaStream_t s);
 int tma_prepare(const GroupPlan &p);
 int tma_blocks_per_sm(const GroupPlan &p);

@@ -242,12 +242,12 @@ std::vector<GroupPlan> group_variants(const GroupPlan &p, int R1,
   // group qualifies: 32 or 64-word rows, 2 or 3 stages, 256 or 512 threads
   const char *tma_env = getenv("CC_TMA");
   const bool tma_off = tma_env && atoi(tma_env) == 0;
-  // a ternary first group over packed row pairs (its tiles are the pairs
+  // a first group over packed row pairs (its tiles are the pairs
   // the group already has, so a recount's code bounds stay valid)
   for (int th : {256, 512}) {
     if (tma_off || (p.a.tma == 3 && p.threads == th)) continue;
-    GroupPlan v = tern_first_variant(p, th);
-    if (!tern_first_ok(v.a, R1)) continue;
+    GroupPlan v = rows_first_variant(p, th);
+    if (!rows_first_ok(v.a, R1)) continue;
     v.grid = occupancy_grid(v);
     out.push_back(v);
   }
@@ -336,8 +336,8 @@ int pad_max_axes(int prob, int q) {
 // round_up(T0, 64) words a row, so every later group's rows start on 128-
 // byte boundaries and run as streamed launches over packed pairs; the last
 // writes the map or cnt back at the canonical index.  The axes after the
-// first group are split evenly into groups of at most pad_max_axes, and a
-// ternary first group takes the packed row-pair form where it applies.  false when the cell does not qualify or
+// first group are split evenly into groups of at most pad_max_axes, and the
+// first group takes the packed row-pair form where it applies.  false when the cell does not qualify or
 // the padded planes do not fit the room16 u16 words of the allocation.
 bool pad_plan(std::vector<GroupPlan> &groups, const Geometry &g,
               const PlanPtrs &ptr, int dst, int R1, long long room16) {
@@ -406,13 +406,13 @@ bool pad_plan(std::vector<GroupPlan> &groups, const Geometry &g,
   f.a.pitch = P0;
   f.a.t0 = T0;
   f.a.plane = plane16;
-  // row pairs as the first group's tiles: the packed ternary form runs on
-  // them (the register kernels take them as Bo = 2)
+  // row pairs as the first group's tiles: the packed form runs on them (the
+  // register kernels take them as Bo = 2)
   GroupPlan fv = f;
   fv.a.Bo = 2;
   fv.a.ntiles = (fv.a.outer + 1) / 2;
-  if (f.a.Bo == 1 && f.a.nchunk == 1 && tern_first_ok(fv.a, R1))
-    f = tern_first_variant(fv, 256);
+  if (f.a.nchunk == 1 && rows_first_ok(fv.a, R1))
+    f = rows_first_variant(fv, 256);
   groups.resize(1);
   groups.insert(groups.end(), later.begin(), later.end());
   size_streamed(groups);
