@@ -271,8 +271,10 @@ std::vector<GroupPlan> group_variants(const GroupPlan &p, int R1,
         }
       }
   // a padded plan's later groups run streamed only (the register kernels
-  // address the canonical layout)
-  if (p.a.pitch && p.a.tma == 1) return out;
+  // address the canonical layout), and its first group over row pairs has
+  // taken half the register kernels' time wherever both were timed (65 us
+  // against 31 on Lee 7^8), so those are not timed again
+  if (p.a.pitch && (p.a.tma == 1 || p.a.tma == 3)) return out;
   for (int stages : {0, 2, 3})
     if (!tma_off && tma_first_ok(p.a, R1, stages))
       for (int th : {128, 256, 512}) {

@@ -42,7 +42,18 @@ struct RowRound {
   static constexpr int A = I == 0 ? KK - BM : I == N - 1 ? LOW : BM * (I - 1);
   static constexpr int B = I == 0 ? BM : I == N - 1 ? KK - BM - LOW
                            : (LOW - A < BM ? LOW - A : BM);
+  // axes applied by the rounds before this one
+  static constexpr int DONE = I == 0 ? 0 : I == N - 1 ? BM + LOW
+                              : BM + BM * (I - 1);
 };
+// Distance layers that can be nonzero after `axes` axes of kind C: a Hamming
+// axis adds at most 1 to the distance, a Lee axis Q / 2.  The early rounds
+// neither write nor read the others.
+template <int C, int R1>
+__host__ __device__ constexpr int live_after(int axes) {
+  const int reach = axes * (axis_lee(C) ? axis_size(C) / 2 : 1);
+  return reach + 1 < R1 ? reach + 1 : R1;
+}
 
 template <int C, int KK, int R1, int SRC, int I>
 __device__ __forceinline__ void rows_round(uint32_t *work, const TmaArgs &a,
@@ -56,6 +67,8 @@ __device__ __forceinline__ void rows_round(uint32_t *work, const TmaArgs &a,
   constexpr int QA = P<Q, A>::v, QB = P<Q, B>::v;
   constexpr bool FIRST = I == 0, LAST = I == TR::N - 1;
   constexpr int NB = T0 / QB;
+  constexpr int LIN = live_after<C, R1>(TR::DONE);
+  constexpr int LOUT = live_after<C, R1>(TR::DONE + B);
   for (int blk = threadIdx.x; blk < NB; blk += blockDim.x) {
     const int pb = blk % QA + (blk / QA) * (QA * QB);
     uint32_t v[R1][QB];
@@ -79,12 +92,13 @@ __device__ __forceinline__ void rows_round(uint32_t *work, const TmaArgs &a,
 #pragma unroll
       for (int d = 0; d < R1; d++)
 #pragma unroll
-        for (int e = 0; e < QB; e++) v[d][e] = work[d * WS + pb + e * QA];
+        for (int e = 0; e < QB; e++)
+          v[d][e] = d < LIN ? work[d * WS + pb + e * QA] : 0u;
     }
     Axes<C, R1, B, 0>::run(v);
     if (!LAST) {
 #pragma unroll
-      for (int d = 0; d < R1; d++)
+      for (int d = 0; d < LOUT; d++)
 #pragma unroll
         for (int e = 0; e < QB; e++) work[d * WS + pb + e * QA] = v[d][e];
       continue;
@@ -129,36 +143,32 @@ struct RowRounds<C, KK, R1, SRC, N, N> {
                                              uint32_t) {}
 };
 
-// Wide stores of a tile's layers (a row pitch that is a multiple of 8
-// words and at least T0 rounded up to 8): each thread takes 8 positions of
-// one layer from the buffer (two 16-byte shared loads of packed lanes) and
-// stores each row's 8 words with one 16-byte store.  Positions from T0 to
-// the next multiple of 8 land in the row's padding.
+// Wide stores of a tile's layers (a row pitch that is a multiple of 8 words
+// and at least T0 rounded up to 8): each thread takes 4 positions of one layer
+// from the buffer (a 16-byte shared load of packed lanes, consecutive across
+// the warp, so free of bank conflicts) and stores each row's 4 words with one
+// 8-byte store.  Positions from T0 to the next multiple of 4 land in the
+// row's padding.
 template <int C, int KK, int R1>
 __device__ __forceinline__ void rows_copy_out(const uint32_t *work,
                                               const TmaArgs &a, long long r0,
                                               bool two) {
   constexpr int T0 = P<axis_size(C), KK>::v;
   constexpr int WS = (T0 + 31) / 32 * 32;
-  constexpr int C8 = (T0 + 7) / 8;
-  static_assert(C8 * 8 <= WS, "the buffer covers the rounded row");
-  const int n = a.lout * C8;
+  constexpr int C4 = (T0 + 3) / 4;
+  static_assert(C4 * 4 <= WS, "the buffer covers the rounded row");
+  const int n = a.lout * C4;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int d = i / C8, m = (i - d * C8) * 8;
+    const int d = i / C4, m = (i - d * C4) * 4;
     const uint4 x = *reinterpret_cast<const uint4 *>(work + d * WS + m);
-    const uint4 y = *reinterpret_cast<const uint4 *>(work + d * WS + m + 4);
     uint16_t *q = a.layers16 + d * a.plane + r0 * a.pitch + m;
-    __stcs(reinterpret_cast<uint4 *>(q),
-           make_uint4(__byte_perm(x.x, x.y, 0x5410),
-                      __byte_perm(x.z, x.w, 0x5410),
-                      __byte_perm(y.x, y.y, 0x5410),
-                      __byte_perm(y.z, y.w, 0x5410)));
+    __stcs(reinterpret_cast<uint2 *>(q),
+           make_uint2(__byte_perm(x.x, x.y, 0x5410),
+                      __byte_perm(x.z, x.w, 0x5410)));
     if (two)
-      __stcs(reinterpret_cast<uint4 *>(q + a.pitch),
-             make_uint4(__byte_perm(x.x, x.y, 0x7632),
-                        __byte_perm(x.z, x.w, 0x7632),
-                        __byte_perm(y.x, y.y, 0x7632),
-                        __byte_perm(y.z, y.w, 0x7632)));
+      __stcs(reinterpret_cast<uint2 *>(q + a.pitch),
+             make_uint2(__byte_perm(x.x, x.y, 0x7632),
+                        __byte_perm(x.z, x.w, 0x7632)));
   }
 }
 

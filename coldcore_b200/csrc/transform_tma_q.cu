@@ -1,5 +1,5 @@
-// transform_tma_q.cu — the streamed groups of Hamming axes of 4 to 6 and Lee
-// axes of 4 to 7 (tma_group.cuh), all in a padded plan's layout: OUT 0 writes
+// transform_tma_q.cu — the streamed groups of Hamming axes of 4 to 6, Lee axes
+// of 4 to 7 and ternary cells of R = 2 (tma_group.cuh), all in a padded plan's layout: OUT 0 writes
 // layers, 3 the map and 4 the cnt at their canonical index.
 //
 // A group takes as many axes as keep its tile's middle extent within 256, the
@@ -17,6 +17,8 @@ namespace {
 #define TQ(C, K, L)                                                         \
   TQ1(C, K, 2, L), TQ1(C, K, 3, L), TQ1(C, K, 4, L), TQ1(C, K, 5, L)
 const TmaEntry kTmaQ[] = {
+    // ternary cells of three layers (four and five: transform_tma.cu)
+    TQ1(3, 3, 3, 32), TQ1(3, 4, 3, 32), TQ1(3, 5, 3, 16),
     TQ(4, 1, 32), TQ(4, 2, 32), TQ(4, 3, 32), TQ(4, 4, 16),
     TQ(5, 1, 32), TQ(5, 2, 32), TQ(5, 3, 16),
     TQ(6, 1, 32), TQ(6, 2, 32), TQ(6, 3, 16),

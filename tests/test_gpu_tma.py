@@ -240,3 +240,26 @@ def test_streamed_groups_of_larger_axes_match_the_oracle(monkeypatch, problem,
                 used += sum(int(np.count_nonzero(b.plan_forms(im, om) & TMA))
                             for im, om in ((0, 2), (1, 1), (2, 1)))
     assert used > 0 or R == 1, "no launch took the streamed form"
+
+
+@pytest.mark.parametrize("n,mu,kb", [(12, 2, 100), (13, 1, 64), (11, 1, 64),
+                                     (10, 2, 100)])
+def test_padded_ternary_plan_of_three_layers(monkeypatch, n, mu, kb):
+    """R = 2 ternary cells: seven and eight axes in the first group over row
+    pairs, an odd number of rows, then one streamed group or two."""
+    from oracle.cport import CPortCell
+    monkeypatch.setenv("CC_TMA", "1")
+    monkeypatch.setenv("CC_TUNE", "0")
+    monkeypatch.setenv("CC_SMEM_BUDGET_KB", str(kb))
+    axes, size = [3] * n, 3 ** n
+    code = np.random.default_rng(n).integers(0, size, size=size // 90)
+    o = CPortCell(axes, 2, "hamming", mu=mu)
+    o.recount(code)
+    with GpuBackend(axes, 2, mu=mu) as b:
+        b.recount(code)
+        assert np.array_equal(b.read_cnt(), o.cnt)
+        for field in ("gain_map", "loss_map"):
+            getattr(b, field)()
+            getattr(o, field)()
+            assert np.array_equal(b.map_all(), o.map), field
+        assert b.plan_forms(1, 1)[0] & TMA
