@@ -59,6 +59,7 @@ struct Cell {
   int noff = 0;
   int slots = 0;
   long long tlen = 0;
+  bool ball_ok = false;              // the table is exactly the metric ball
 };
 
 // one cell's code slices per first-group tile, computed on the device from
@@ -732,14 +733,17 @@ int launch_items(Batch *b, const Group &gr, const int *active) {
 }
 
 // the gain map of every cell with active[i] again (d_active: the same flags
-// on the device), on the streams the step uses
+// on the device), on the streams the step uses; `beside` puts on the main
+// stream what runs at the same time
+template <class Beside>
 int rebuild_gains(Batch *b, const std::vector<int> &active,
-                  const int *d_active) {
+                  const int *d_active, Beside beside) {
   const size_t np = std::max<size_t>(1, b->passes.size());
   CC_CK(cudaMemsetAsync(b->d_next, 0, std::max<size_t>(1, b->nnext) * 8,
                         b->stream));
   CC_CK(cudaMemsetAsync(b->d_done, 0, np * sizeof(unsigned), b->stream));
   CC_CK(cudaEventRecord(b->fork, b->stream));
+  int rc = beside();
   bool used[kSideStreams] = {false};
   auto fork = [&](int k) -> int {
     if (used[k]) return 0;
@@ -747,7 +751,6 @@ int rebuild_gains(Batch *b, const std::vector<int> &active,
     CC_CK(cudaStreamWaitEvent(b->side[k], b->fork, 0));
     return 0;
   };
-  int rc = 0;
   for (size_t i = 0; i < b->cells.size() && !rc; i++) {
     const Cell &c = b->cells[i];
     if (!c.big || !active[i]) continue;
@@ -1180,6 +1183,7 @@ int dct_batch_set_table(long long h, int cell, const int32_t *tbl, int slots,
   c.noff = (int)ent.size();
   c.slots = slots;
   c.tlen = len;
+  c.ball_ok = metric_ball_table(c.g, soa, slots, len);
   return 0;
 }
 
@@ -1339,8 +1343,8 @@ int dct_batch_greedy(long long h, const int *cells, int n, const int *max_add,
     steps = std::max<long long>(steps, std::min<long long>(
         max_add[k], sc[3 * cells[k]]));
   }
-  // workspace: per cell its table entry, state, placed words, chunk keys and
-  // dirty flags; the rebuild flags of the listed cells and of the batch's
+  // workspace: per cell its table entry, state, placed words and chunk keys;
+  // the rebuild flags of the listed cells and of the batch's
   // cells; the jobs of the two launches of a step
   auto pad = [](size_t x) { return (x + 63) / 64 * 64; };
   const size_t st_b = (size_t)n * kGreedyStateBytes;
@@ -1365,7 +1369,7 @@ int dct_batch_greedy(long long h, const int *cells, int n, const int *max_add,
                                   return o; };
   const size_t o_tab = take((size_t)n * sizeof(BatchGreedyCell));
   const size_t o_st = take(st_b), o_pl = take(pl_b);
-  const size_t o_key = take(chunks * 8), o_dirty = take(chunks);
+  const size_t o_key = take(chunks * 8);
   const size_t o_fresh = take(fresh_words * 8);
   const size_t o_flag = take((size_t)n * 4);
   const size_t o_act = take(b->cells.size() * 4);
@@ -1403,7 +1407,6 @@ int dct_batch_greedy(long long h, const int *cells, int n, const int *max_add,
       g.placed = reinterpret_cast<long long *>(ws + o_pl) +
                  (size_t)k * std::max(cap, 1);
       g.ckey = reinterpret_cast<unsigned long long *>(ws + o_key) + co;
-      g.dirty = reinterpret_cast<uint8_t *>(ws + o_dirty) + co;
       g.code = c.dcode;
       g.ncode = (long long)c.code.size();
       g.max_add = max_add[k];
@@ -1458,7 +1461,7 @@ int dct_batch_greedy(long long h, const int *cells, int n, const int *max_add,
     const int par = (int)(issued & 1);
     if (follow) {
       rc = launch_greedy_argmax(dtab, d_jam, (int)jam.size(), par,
-                                issued == 0, d_flag, b->stream);
+                                issued == 0, b->stream);
       read_states(par);
       const GreedyHost *h = ring[par ^ 1];
       if (issued) ck(cudaEventSynchronize(b->ev_greedy[par ^ 1]));
@@ -1469,7 +1472,8 @@ int dct_batch_greedy(long long h, const int *cells, int n, const int *max_add,
         const bool done = issued ? h[k].done != 0 : st0[k].done != 0;
         const long long gain = issued ? h[k].gain(par ^ 1)
                                       : sc[3 * cells[k] + 1];
-        const int want = !done && greedy_rebuild_pays(gain, c.tlen, c.gain_us);
+        const int want = !done && c.ball_ok &&
+                         greedy_rebuild_pays(gain, c.tlen, c.gain_us);
         live = live || !done;
         any = any || want;
         changed = changed || want != flag[k];
@@ -1483,9 +1487,11 @@ int dct_batch_greedy(long long h, const int *cells, int n, const int *max_add,
       if (!rc)
         rc = launch_greedy_place(dtab, d_jpl, (int)jpl.size(), par, kExcluded,
                                  b->stream);
-      if (!rc)
-        rc = launch_greedy_refresh(dtab, n, ball_blocks, d_flag, b->stream);
-      if (any && !rc) rc = rebuild_gains(b, act, d_act);
+      // the other cells' refresh runs while the side streams rebuild
+      auto refresh = [&] {
+        return launch_greedy_refresh(dtab, n, ball_blocks, d_flag, b->stream);
+      };
+      if (!rc) rc = any ? rebuild_gains(b, act, d_act, refresh) : refresh();
       if (any && !rc)
         rc = launch_greedy_exclude(dtab, n, d_flag, kExcluded, b->stream);
       follow = any;
@@ -1495,7 +1501,7 @@ int dct_batch_greedy(long long h, const int *cells, int n, const int *max_add,
     const long long m = std::min(chunk, steps - issued);
     for (long long i = 0; i < m && !rc; i++, issued++) {
       const int p2 = (int)(issued & 1);
-      rc = launch_greedy_argmax(dtab, d_jam, (int)jam.size(), p2, 0, d_flag,
+      rc = launch_greedy_argmax(dtab, d_jam, (int)jam.size(), p2, 0,
                                 b->stream);
       if (!rc) rc = launch_greedy_place(dtab, d_jpl, (int)jpl.size(), p2,
                                         kExcluded, b->stream);

@@ -286,6 +286,11 @@ struct WalkArgs {
   int noff = 0;
 };
 constexpr int kMaxPackOff = 255;
+// Is the table exactly the metric ball: distinct patterns, each moving
+// distinct axes by admissible shifts within radius R, as many as the ball
+// has?  Only then do a transform and walks over the table agree.
+bool metric_ball_table(const Geometry &g, const std::vector<int32_t> &soa,
+                       int slots, long long len);
 // Packs a validated SoA table; false when the cell does not qualify: the
 // open grid (it rejects patterns), 2^31 words or more, more than four slots
 // or more than 255 (position, shift) entries.
@@ -318,7 +323,7 @@ int launch_gather_set(const Geometry &g, const long long *dcand, int nc,
 // argmax over chunk keys and a placement that lowers the gains it changes
 constexpr int kGreedyStateBytes = 48;
 constexpr int kGreedyChunk = 1024;        // map words per kept key
-constexpr int kGreedyBlockChunks = 8;     // chunks per argmax block: a warp each
+constexpr int kGreedyBlockChunks = 32;    // chunks per argmax block
 constexpr int kGreedyMaxPat = 1024;       // ball patterns per place block
 // host view of one cell's state (GreedyState)
 struct GreedyHost {
@@ -341,7 +346,6 @@ struct BatchGreedyCell {
   long long *placed;
   long long *fresh;         // |B| words: those the last placement satisfied
   unsigned long long *ckey; // best key of each chunk of kGreedyChunk words
-  uint8_t *dirty;           // its key is stale
   const long long *code;    // words that are never placed (device)
   long long ncode;
   int max_add;
@@ -368,11 +372,10 @@ int launch_greedy_exclude(const BatchGreedyCell *dcells, int ncells,
                           const int *rebuild, int32_t exclude,
                           cudaStream_t s);
 // jobs: (cell, block of the cell) per block, or nullptr for one cell; par:
-// parity of the step; all / rebuilt[cell]: read every chunk; rebuild[cell]:
-// its gain map is left to a transform
+// parity of the step; all: read every chunk (a greedy's first step);
+// rebuild[cell]: its gain map is left to a transform
 int launch_greedy_argmax(const BatchGreedyCell *dcells, const int2 *jobs,
-                         int njobs, int par, int all, const int *rebuilt,
-                         cudaStream_t s);
+                         int njobs, int par, int all, cudaStream_t s);
 int launch_greedy_place(const BatchGreedyCell *dcells, const int2 *jobs,
                         int njobs, int par, int32_t exclude, cudaStream_t s);
 // the gains after a placement: `blocks` blocks per cell share its new words

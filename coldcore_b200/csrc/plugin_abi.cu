@@ -135,7 +135,8 @@ struct State {
   unsigned long long dd_last = 0;
   bool layered_out = false;        // last transform left N_0..N_R
   // set side (setside.cu): the listed predicate set Z, cached per cnt state
-  bool ball_ok = false;            // support table proven == metric ball
+  bool metric_table = false;       // support table proven == metric ball
+  bool ball_ok = false;            // ... on a cell the set side takes
   bool set_ok = false;             // ... and the set side is on
   int set_policy = 1;              // DCT_SET_GATHER: 0 off, 1 auto, 2 force
   long long set_min = -1;          // DCT_SET_MIN: walk size that tries it
@@ -152,7 +153,7 @@ struct State {
   long long *d_list = nullptr;
   long long lcap = 0;
   // device greedy: state, placed words, words satisfied per placement
-  // [the cell's BatchGreedyCell][its state][chunk keys][fresh words][dirty]
+  // [the cell's BatchGreedyCell][its state][chunk keys][fresh words]
   char *d_greedy = nullptr;
   GreedyHost *h_greedy = nullptr;  // pinned ring of kGreedyRing states
   cudaEvent_t ev_greedy[kGreedyRing] = {nullptr};
@@ -966,65 +967,14 @@ int finish_init(long long *bytes) {
   return 0;
 }
 
-// Is the support table exactly the metric ball?  Every pattern must move
-// distinct axes by admissible deltas within radius R, the patterns must be
-// distinct, and their number must equal the ball's cardinality (coldcore
-// dct_hc.cu:158-204 states the same test).  Only then may a gather count
-// listed words by distance instead of walking the table.
-bool table_is_ball(const std::vector<int32_t> &soa, int slots, long long len) {
-  const int n = S.g.n, R = S.g.R, prob = S.g.prob;
-  if (n > 16) return false;
-  for (int i = 0; i < n; i++)
+// May a gather count listed words by distance instead of walking the table?
+// Only where the table is exactly the metric ball (coldcore dct_hc.cu:158-204
+// states the same test), on at most 16 axes of at most 16 values.
+bool table_is_ball() {
+  if (S.g.n > 16) return false;
+  for (int i = 0; i < S.g.n; i++)
     if (S.g.ax[i] > 16) return false;
-  auto weight = [&](int pos, int d) -> int {      // -1: inadmissible
-    const int a = S.g.ax[pos];
-    if (d < 1 || d >= a) return -1;
-    const int c = std::min(d, a - d);
-    if (prob == kHamming) return 1;
-    if (prob == kLee) return c <= R ? c : -1;
-    return c <= R ? 0 : -1;                        // L-infinity
-  };
-  std::vector<unsigned long long> keys;
-  keys.reserve((size_t)len);
-  for (long long t = 0; t < len; t++) {
-    unsigned seen = 0;
-    unsigned long long key = 0;
-    int w = 0;
-    for (int k = 0; k < slots; k++) {
-      const int32_t c = soa[(size_t)k * len + t];
-      if (!c) continue;
-      const int pos = c >> 24, d = c & 0xFFFFFF;
-      if (pos >= n || ((seen >> pos) & 1u)) return false;
-      seen |= 1u << pos;
-      const int e = weight(pos, d);
-      if (e < 0) return false;
-      w += e;
-      key |= (unsigned long long)d << (4 * pos);
-    }
-    if (w > R) return false;
-    keys.push_back(key);
-  }
-  std::sort(keys.begin(), keys.end());
-  if (std::adjacent_find(keys.begin(), keys.end()) != keys.end()) return false;
-  // cardinality: coefficients 0..W of prod_i (1 + sum_d t^weight(i, d))
-  const int W = (prob == kHamming || prob == kLee) ? R : 0;
-  std::vector<long double> poly(W + 1, 0.0L);
-  poly[0] = 1.0L;
-  for (int i = 0; i < n; i++) {
-    std::vector<long double> nx(W + 1, 0.0L);
-    for (int w = 0; w <= W; w++) {
-      if (poly[w] == 0) continue;
-      nx[w] += poly[w];
-      for (int d = 1; d < S.g.ax[i]; d++) {
-        const int e = weight(i, d);
-        if (e >= 0 && w + e <= W) nx[w + e] += poly[w];
-      }
-    }
-    poly.swap(nx);
-  }
-  long double tot = 0;
-  for (int w = 0; w <= W; w++) tot += poly[w];
-  return tot == (long double)len;
+  return S.metric_table;
 }
 
 void set_side_init(const std::vector<int32_t> &soa, int slots) {
@@ -1034,7 +984,8 @@ void set_side_init(const std::vector<int32_t> &soa, int slots) {
   S.set_policy = sp ? atoi(sp) : 1;
   S.set_min = sm ? atoll(sm) : -1;
   S.set_ratio = sr ? std::max(1LL, atoll(sr)) : 2;
-  S.ball_ok = table_is_ball(soa, slots, S.len);
+  S.metric_table = metric_ball_table(S.g, soa, slots, S.len);
+  S.ball_ok = table_is_ball();
   S.set_ok = S.set_policy != 0 && S.ball_ok;
   S.zcap_max = std::min<long long>(S.g.space, 1LL << 27);
   S.z_mode = -1;
@@ -1607,9 +1558,8 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
   const size_t o_key = o_run + kGreedyRunBytes;
   static_assert(kGreedyStateBytes <= 64, "greedy state");
   const size_t o_fresh = o_key + (size_t)nch * 8;
-  const size_t o_dirty = o_fresh + (size_t)S.len * 8;
   if (!S.d_greedy) {
-    CC_CK(cudaMalloc(&S.d_greedy, o_dirty + (size_t)nch));
+    CC_CK(cudaMalloc(&S.d_greedy, o_fresh + (size_t)S.len * 8));
     CC_CK(cudaHostAlloc((void **)&S.h_greedy, kGreedyRing * kGreedyStateBytes,
                         cudaHostAllocDefault));
     for (auto &ev : S.ev_greedy)
@@ -1664,7 +1614,6 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
   gc.placed = S.d_placed;
   gc.fresh = reinterpret_cast<long long *>(S.d_greedy + o_fresh);
   gc.ckey = reinterpret_cast<unsigned long long *>(S.d_greedy + o_key);
-  gc.dirty = reinterpret_cast<uint8_t *>(S.d_greedy + o_dirty);
   gc.code = S.d_active;
   gc.ncode = (long long)code.size();
   gc.max_add = max_add;
@@ -1689,7 +1638,8 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
   const int npl = (int)((S.len + gc.pats - 1) / gc.pats);
   const int nrf = sm_count() * 4;
   // the time of a gain transform: measured by the autotuner, else launches
-  // and bytes at a small cell's rate; a streamed cell is never rebuilt
+  // and bytes at a small cell's rate; a streamed cell is never rebuilt, nor
+  // one whose table is not the ball that the transform sums over
   double rebuild_us = S.tune_ms[1][1] * 1e3;
   if (rebuild_us <= 0) {
     const Plan &P = plan_for(1, 1);
@@ -1698,7 +1648,7 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
     for (size_t i = 0; i < P.passes.size(); i++)
       rebuild_us += 6.0 * S.g.space / 1.0e6;
   }
-  if (S.streamed) rebuild_us = 1e30;
+  if (S.streamed || !S.metric_table || S.fmt != 0) rebuild_us = 1e30;
   auto read_state = [&](int slot) -> int {
     CC_CK(cudaMemcpyAsync(S.h_greedy + slot, gc.st, sizeof(st),
                           cudaMemcpyDeviceToHost, g_stream));
@@ -1712,11 +1662,11 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
   // out in chunks with one look at the state between them.
   const long long steps = std::min<long long>(max_add, d0);
   long long issued = 0, chunk = 32;
-  bool follow = true, rebuilt = true;
+  bool follow = true;
   while (issued < steps) {
     if (follow) {
       const int par = (int)(issued & 1);
-      rc = launch_greedy_argmax(dcell, nullptr, nam, par, rebuilt, nullptr,
+      rc = launch_greedy_argmax(dcell, nullptr, nam, par, issued == 0,
                                 g_stream);
       if (rc || (rc = read_state(par))) return rc;
       const int look = issued ? par ^ 1 : par;
@@ -1730,7 +1680,6 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
       rc = rebuild ? build_map()
                    : launch_greedy_refresh(dcell, 1, nrf, nullptr, g_stream);
       if (rc) return rc;
-      rebuilt = rebuild;
       follow = rebuild;
       issued++;
       continue;

@@ -16,6 +16,7 @@
 // word's digits, axis sizes and strides sit in shared memory, and each
 // thread resolves one pattern at a time with a few integer ops per slot.
 #include <algorithm>
+#include <array>
 #include <cstdlib>
 
 #include "engine.h"
@@ -93,6 +94,54 @@ __device__ __forceinline__ long long walk_word(const WalkArgs &a, long long w,
     x += (long long)sh * s.pw[p];
   }
   return x;
+}
+
+bool metric_ball_table(const Geometry &g, const std::vector<int32_t> &soa,
+                       int slots, long long len) {
+  const bool sum = g.prob == kHamming || g.prob == kLee;
+  auto weight = [&](int pos, int d) -> int {      // -1: inadmissible
+    const int a = g.ax[pos], c = std::min(d, a - d);
+    if (d < 1 || d >= a) return -1;
+    if (g.prob == kHamming) return 1;
+    return c > g.R ? -1 : sum ? c : 0;
+  };
+  std::vector<std::array<int32_t, kMaxSlots>> rows((size_t)len);
+  for (long long t = 0; t < len; t++) {
+    auto &row = rows[(size_t)t];
+    row.fill(0);
+    int w = 0, m = 0;
+    for (int k = 0; k < slots; k++) {
+      const int32_t c = soa[(size_t)k * len + t];
+      if (!c) continue;
+      if (m < k || (c >> 24) >= g.n) return false;   // a walk stops at a gap
+      const int e = weight(c >> 24, c & 0xFFFFFF);
+      if (e < 0) return false;
+      w += e;
+      row[m++] = c;
+    }
+    if (w > g.R) return false;
+    std::sort(row.begin(), row.begin() + m);
+    for (int k = 1; k < m; k++)
+      if (row[k] >> 24 == row[k - 1] >> 24) return false;
+  }
+  std::sort(rows.begin(), rows.end());
+  if (std::adjacent_find(rows.begin(), rows.end()) != rows.end()) return false;
+  // |B|: coefficients 0..W of prod_j (1 + sum_d t^weight(j, d))
+  const int W = sum ? g.R : 0;
+  std::vector<long double> poly(W + 1, 0.0L);
+  poly[0] = 1.0L;
+  for (int j = 0; j < g.n; j++) {
+    std::vector<long double> nx(poly);
+    for (int w = 0; w <= W; w++)
+      for (int d = 1; d < g.ax[j]; d++) {
+        const int e = weight(j, d);
+        if (e >= 0 && w + e <= W) nx[w + e] += poly[w];
+      }
+    poly.swap(nx);
+  }
+  long double tot = 0;
+  for (long double v : poly) tot += v;
+  return tot == (long double)len;
 }
 
 bool pack_walk(const Geometry &g, const std::vector<int32_t> &soa, int slots,
@@ -342,8 +391,13 @@ int launch_drop_walks(const WalkArgs &w, const long long *ddrops, int k,
 // batched engine's campaign repair), three launches a step:
 //
 //   k_greedy_argmax   the word of largest gain (ties: the smallest index).
-//     The map is cut into chunks of kChunk words whose best keys are kept; a
-//     step reads only the chunks whose best word lost gain (dirty).
+//     The map is cut into chunks of kChunk words whose best keys are kept.
+//     Gains never grow, so a kept key holds until its own word loses gain: a
+//     step looks at that one word of each chunk and reads only the chunks
+//     where it did, after a transform of the map too.  (A flag set by the
+//     refresh where an updated word's gain equals its chunk's best costs a
+//     second random read for each of the |fresh| x |B| updates, and ties
+//     flag chunks for nothing: 14.0 us a step on K_3(14,3), 12.4 us this way.)
 //   k_greedy_place    the word's ball, split over many blocks: cnt += 1 with
 //     pair atomics; the words it satisfies (old count mu - 1) are listed.
 //   k_greedy_refresh  lowers the gain of every candidate whose ball holds a
@@ -378,6 +432,7 @@ constexpr int kChunk = kGreedyChunk;
 // on K_3(14,3)), against a transform of the cell
 constexpr double kGreedyUpdatesPerUs = 36000.0;
 constexpr int kBlockChunks = kGreedyBlockChunks;
+constexpr int kArgmaxWarps = 8;
 
 __device__ __forceinline__ unsigned long long greedy_key(int32_t v,
                                                          long long x) {
@@ -386,6 +441,13 @@ __device__ __forceinline__ unsigned long long greedy_key(int32_t v,
 }
 __device__ __forceinline__ int32_t key_gain(unsigned long long k) {
   return (int32_t)((uint32_t)(k >> 32) ^ 0x80000000u);
+}
+
+// a chunk's kept key, or 0 if its word has lost gain since
+__device__ __forceinline__ unsigned long long fresh_key(
+    const BatchGreedyCell &c, long long ch) {
+  const unsigned long long k = __ldcg(c.ckey + ch);
+  return __ldcg(c.map + (uint32_t)~(uint32_t)k) == key_gain(k) ? k : 0;
 }
 
 // map[x] = exclude for a cell's code and placed words (they never re-enter);
@@ -428,19 +490,15 @@ __device__ __forceinline__ unsigned long long read_chunk(
   }
   for (int o = 16; o > 0; o >>= 1)
     m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if (lane == 0) {
-    c.ckey[ch] = m;
-    c.dirty[ch] = 0;
-  }
+  if (lane == 0) c.ckey[ch] = m;
   return m;
 }
 
 // jobs: (cell, block of the cell), or nullptr for cell 0 and blockIdx.x;
 // block 0 of a cell also commits its last placement
-__global__ void __launch_bounds__(32 * kBlockChunks)
+__global__ void __launch_bounds__(32 * kArgmaxWarps)
 k_greedy_argmax(const BatchGreedyCell *__restrict__ cells,
-                const int2 *__restrict__ jobs, int par, int all,
-                const int *__restrict__ rebuilt) {
+                const int2 *__restrict__ jobs, int par, int all) {
   const int2 job = jobs ? jobs[blockIdx.x] : make_int2(0, (int)blockIdx.x);
   const BatchGreedyCell &c = cells[job.x];
   GreedyState *st = reinterpret_cast<GreedyState *>(c.st);
@@ -455,13 +513,23 @@ k_greedy_argmax(const BatchGreedyCell *__restrict__ cells,
     st->nnew = 0;
     st->best[par ^ 1] = 0;
   }
-  const long long ch = (long long)job.y * kBlockChunks + (threadIdx.x >> 5);
-  if (ch * kChunk >= c.w.g.space) return;           // a whole warp
-  const unsigned long long m =
-      all || (rebuilt && rebuilt[job.x]) || c.dirty[ch] ? read_chunk(c, ch)
-                                                        : c.ckey[ch];
+  // lane j looks at the warp's chunk j, the warp reads the stale ones
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long first = (long long)job.y * kBlockChunks + warp;
+  const long long mine = first + (long long)kArgmaxWarps * lane;
+  unsigned long long m = 0;
+  bool stale = false;
+  if (lane < kBlockChunks / kArgmaxWarps && mine * kChunk < c.w.g.space) {
+    if (!all) m = fresh_key(c, mine);
+    stale = m == 0;
+  }
+  for (unsigned todo = __ballot_sync(0xffffffffu, stale); todo;
+       todo &= todo - 1)
+    m = max(m, read_chunk(c, first + kArgmaxWarps * (__ffs(todo) - 1)));
+  for (int o = 16; o > 0; o >>= 1)
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
   // one atomic a warp; most warps see a larger key already there
-  if ((threadIdx.x & 31) == 0 && m > __ldcg(&st->best[par]))
+  if (lane == 0 && m > __ldcg(&st->best[par]))
     atomicMax(&st->best[par], m);
 }
 
@@ -491,7 +559,6 @@ __device__ __forceinline__ void greedy_place(const BatchGreedyCell &c,
         c.placed[placed] = x;
         st->pend = 1;
         c.map[x] = exclude;
-        c.dirty[x / kChunk] = 1;
       }
     }
   }
@@ -550,22 +617,13 @@ __device__ __forceinline__ void greedy_refresh(const BatchGreedyCell &c) {
     __syncthreads();                      // s is reused across words
     word_setup<WALK>(a, x0, s);
     long long y[4];
-    int32_t old[4];
-    unsigned long long key[4];
     const long long tt = t0 + threadIdx.x;
 #pragma unroll
     for (int j = 0; j < 4; j++)
       y[j] = tt + 256 * j < t1 ? walk_word<WALK>(a, x0, tt + 256 * j, s) : -1;
 #pragma unroll
     for (int j = 0; j < 4; j++)
-      if (y[j] >= 0) old[j] = atomicSub(&c.map[y[j]], 1);
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-      if (y[j] >= 0) key[j] = c.ckey[y[j] / kChunk];
-    // the chunk's best loses gain (or ties with it): its key is stale
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-      if (y[j] >= 0 && old[j] == key_gain(key[j])) c.dirty[y[j] / kChunk] = 1;
+      if (y[j] >= 0) atomicSub(&c.map[y[j]], 1);
   }
 }
 
@@ -584,7 +642,7 @@ k_greedy_refresh(const BatchGreedyCell *__restrict__ cells,
 // (1.2 us) between the phases.  Near a cover a phase is a few microseconds of
 // dependent L2 round trips, so what does not change is kept close: the cell
 // is a kernel parameter, the packed table and its entries sit in shared
-// memory.  On K_3(14,3) a step takes 11 us at gains of 5 and 17 us at 150;
+// memory.  On K_3(14,3) a step takes 9 us at gains of 50 and 14 us at 160;
 // the whole-map argmax, one-block place and refresh launches this replaces
 // took 49 us, the three launches above 25 us (9 of them gaps).  The grid is
 // resident as a whole (a cooperative launch) and every wait is bounded: a
@@ -659,10 +717,11 @@ __device__ __forceinline__ void warp_setup(const WalkArgs &a, const int4 *ent,
   __syncwarp();
 }
 
-// Each phase is shared out over the warps of the grid and needs no block
-// barrier: argmax by chunks, place by patterns (interleaved), refresh by
-// pieces of kRunPat patterns of one new word, whose updates are all in
-// flight together.  (A block refreshing its own new words saves a barrier,
+// Argmax is shared out by chunks, whose stale ones a block's warps read side
+// by side; place by whole warps of patterns (three lanes of every warp of the
+// grid instead meant 2,368 atomics on two addresses, 1.5 us); refresh by
+// pieces of kRunPat patterns of one new word, whose updates are all in flight
+// together.  (A block refreshing its own new words saves a barrier,
 // 1.4 us, but a word's 2,969 updates by one block take 8 us.)
 template <int WALK>
 __global__ void __launch_bounds__(kRunThreads)
@@ -672,6 +731,7 @@ k_greedy_run(const __grid_constant__ BatchGreedyCell c, int table_words,
   __shared__ int4 ent[WALK == kPack ? kMaxPackOff : 1];
   __shared__ WalkSmem smem[kRunWarps];
   __shared__ unsigned long long wbest[kRunWarps];
+  __shared__ int stale[kRunThreads], nstale;
   GreedyState *st = reinterpret_cast<GreedyState *>(c.st);
   const WalkArgs &a = c.w;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -706,19 +766,22 @@ k_greedy_run(const __grid_constant__ BatchGreedyCell c, int table_words,
       st->nnew = 0;
       st->best[par ^ 1] = 0;
     }
+    // a thread looks at each of the block's chunks, its warps share the
+    // stale ones
     unsigned long long k = 0;
-    for (long long b = gw; b < nch; b += 32 * W) {
-      // 32 of the warp's chunks: a lane looks at each, the warp reads the
-      // stale ones
-      const long long ch = b + lane * W;
-      bool stale = false;
+    for (long long b = blockIdx.x; b < nch; b += kRunThreads * gridDim.x) {
+      const long long ch = b + (long long)tid * gridDim.x;
+      __syncthreads();                  // the last round's list is read
+      if (tid == 0) nstale = 0;
+      __syncthreads();
       if (ch < nch) {
-        const unsigned long long key = __ldcg(c.ckey + ch);
-        stale = __ldcg(c.dirty + ch);
-        if (!stale) k = max(k, key);
+        const unsigned long long key = fresh_key(c, ch);
+        if (key == 0) stale[atomicAdd(&nstale, 1)] = (int)ch;
+        k = max(k, key);
       }
-      for (unsigned m = __ballot_sync(0xffffffffu, stale); m; m &= m - 1)
-        k = max(k, read_chunk(c, b + (__ffs(m) - 1) * W));
+      __syncthreads();
+      for (int q = warp; q < nstale; q += kRunWarps)
+        k = max(k, read_chunk(c, stale[q]));
     }
     for (int o = 16; o > 0; o >>= 1)
       k = max(k, __shfl_xor_sync(0xffffffffu, k, o));
@@ -743,12 +806,11 @@ k_greedy_run(const __grid_constant__ BatchGreedyCell c, int table_words,
       c.placed[placed] = x0;
       st->pend = 1;
       c.map[x0] = exclude;
-      c.dirty[x0 / kChunk] = 1;
     }
-    if (gw < a.len) {
+    if (32 * gw < a.len) {
       warp_setup<WALK>(a, ent, x0, s);
-      for (long long b = gw; b < a.len; b += 32 * W) {
-        const long long t = b + lane * W;
+      for (long long b = 32 * gw; b < a.len; b += 32 * W) {
+        const long long t = b + lane;
         const long long x = t < a.len ? walk(x0, t) : -1;
         int cv = 0x10000;
         if (x >= 0) {
@@ -771,27 +833,24 @@ k_greedy_run(const __grid_constant__ BatchGreedyCell c, int table_words,
     if (!grid_barrier(run, ++bar)) return;
     // -------- refresh
     const long long n = __ldcg(&st->nnew) * nseg;
-    for (long long p = gw; p < n; p += W) {
-      const long long u = __ldcg(c.fresh + p / nseg);
-      const long long t0 = p % nseg * kRunPat + lane;
-      warp_setup<WALK>(a, ent, u, s);
-      long long y[kRunPat / 32];
-      int32_t old[kRunPat / 32];
-      unsigned long long key[kRunPat / 32];
+    for (long long p0 = gw; p0 < n; p0 += 32 * W) {
+      // the words of the warp's next 32 pieces in one read
+      const long long pl = p0 + lane * W;
+      const long long ul = pl < n ? __ldcg(c.fresh + pl / nseg) : 0;
+      const int sl = (int)(pl % nseg);
+      for (int r = 0; r < 32 && p0 + r * W < n; r++) {
+        const long long u = __shfl_sync(0xffffffffu, ul, r);
+        const long long t0 =
+            (long long)__shfl_sync(0xffffffffu, sl, r) * kRunPat + lane;
+        warp_setup<WALK>(a, ent, u, s);
+        long long y[kRunPat / 32];
 #pragma unroll
-      for (int j = 0; j < kRunPat / 32; j++)
-        y[j] = t0 + 32 * j < a.len ? walk(u, t0 + 32 * j) : -1;
+        for (int j = 0; j < kRunPat / 32; j++)
+          y[j] = t0 + 32 * j < a.len ? walk(u, t0 + 32 * j) : -1;
 #pragma unroll
-      for (int j = 0; j < kRunPat / 32; j++)
-        if (y[j] >= 0) old[j] = atomicSub(&c.map[y[j]], 1);
-#pragma unroll
-      for (int j = 0; j < kRunPat / 32; j++)
-        if (y[j] >= 0) key[j] = __ldcg(c.ckey + y[j] / kChunk);
-      // the chunk's best loses gain (or ties with it): its key is stale
-#pragma unroll
-      for (int j = 0; j < kRunPat / 32; j++)
-        if (y[j] >= 0 && old[j] == key_gain(key[j]))
-          c.dirty[y[j] / kChunk] = 1;
+        for (int j = 0; j < kRunPat / 32; j++)
+          if (y[j] >= 0) atomicSub(&c.map[y[j]], 1);
+      }
     }
     if (!grid_barrier(run, ++bar)) return;
   }
@@ -826,10 +885,9 @@ int launch_greedy_refresh(const BatchGreedyCell *dcells, int ncells,
 }
 
 int launch_greedy_argmax(const BatchGreedyCell *dcells, const int2 *jobs,
-                         int njobs, int par, int all, const int *rebuilt,
-                         cudaStream_t s) {
-  k_greedy_argmax<<<(unsigned)njobs, 32 * kBlockChunks, 0, s>>>(
-      dcells, jobs, par, all, rebuilt);
+                         int njobs, int par, int all, cudaStream_t s) {
+  k_greedy_argmax<<<(unsigned)njobs, 32 * kArgmaxWarps, 0, s>>>(
+      dcells, jobs, par, all);
   CC_CK(cudaGetLastError());
   return 0;
 }

@@ -135,3 +135,52 @@ def test_batched_greedy_by_updates_and_by_rebuilds(steps, rebuild,
             assert got[i][0].tolist() == want.tolist(), (i, p, a)
             assert got[i][1] == wdef
             assert np.array_equal(e.cnt(i), ob.cnt.astype(np.uint16))
+
+
+def test_a_table_that_is_not_the_ball_is_never_rebuilt(monkeypatch):
+    """A cell whose table lacks some of the ball's patterns: its greedy stays
+    with the table's updates, whatever the rule on rebuilds says."""
+    from coldcore_b200.batch import BatchEngine
+    from coldcore_b200.patterns import wide_table
+    monkeypatch.setenv("CC_GREEDY_REBUILD", "1")
+    axes, R, steps = (3,) * 6, 2, 12
+    size = 3 ** 6
+    table = wide_table(axes, R, "hamming")
+    cells = [table, table[:-7], np.concatenate([table, table[-1:]])]
+    code = np.random.default_rng(8).integers(0, size, 9)
+    with BatchEngine() as e:
+        for _ in cells:
+            e.add("hamming", axes, R, code)
+        e.build(0)
+        for i, tbl in enumerate(cells):
+            e.set_table(i, tbl)
+        e.run()
+        starts = [(e.cnt(i).astype(int), e.gain(i).astype(int))
+                  for i in range(len(cells))]
+        got = e.greedy(np.arange(len(cells)), [steps] * len(cells))
+        for i, tbl in enumerate(cells):
+            cnt, gain = starts[i]
+            gain[code] = -1
+            strides = [3 ** j for j in range(len(axes))]
+            for step, w in enumerate(got[i][0]):
+                assert w == np.argmax(gain) and gain[w] > 0, (i, step)
+                gain[w] = -1 << 20
+
+                def ball(x):
+                    for row in tbl:
+                        y = int(x)
+                        for s in row[row != 0]:
+                            pw = strides[int(s) >> 24]
+                            d = y // pw % 3
+                            y += ((d + (int(s) & 0xFFFFFF)) % 3 - d) * pw
+                        yield y
+                fresh = []
+                for x in ball(w):
+                    if cnt[x] == 0:
+                        fresh.append(x)
+                    cnt[x] += 1
+                for u in fresh:
+                    for y in ball(u):
+                        gain[y] -= 1
+            assert len(got[i][0]) == steps
+            assert np.array_equal(e.cnt(i), cnt.astype(np.uint16)), i
