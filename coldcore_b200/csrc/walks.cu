@@ -428,8 +428,10 @@ struct GreedyState {
 static_assert(sizeof(GreedyState) == kGreedyStateBytes, "state layout");
 
 constexpr int kChunk = kGreedyChunk;
-// updates a refresh makes in a microsecond: 36,000 (445 K of them in 12 us
-// on K_3(14,3)), against a transform of the cell
+// updates a refresh makes in a microsecond, against a transform of the cell:
+// 90,000 on K_3(14,3) (487 K of them in 5.4 us), fewer on maps that pass the
+// L2.  64 mixed cells of up to 16.8 M words take 14.9 ms at any line from
+// 36,000 to 90,000, and 24.7 ms at 130,000.
 constexpr double kGreedyUpdatesPerUs = 36000.0;
 constexpr int kBlockChunks = kGreedyBlockChunks;
 constexpr int kArgmaxWarps = 8;
@@ -443,10 +445,9 @@ __device__ __forceinline__ int32_t key_gain(unsigned long long k) {
   return (int32_t)((uint32_t)(k >> 32) ^ 0x80000000u);
 }
 
-// a chunk's kept key, or 0 if its word has lost gain since
+// a chunk's kept key k, or 0 if its word has lost gain since
 __device__ __forceinline__ unsigned long long fresh_key(
-    const BatchGreedyCell &c, long long ch) {
-  const unsigned long long k = __ldcg(c.ckey + ch);
+    const BatchGreedyCell &c, unsigned long long k) {
   return __ldcg(c.map + (uint32_t)~(uint32_t)k) == key_gain(k) ? k : 0;
 }
 
@@ -520,7 +521,7 @@ k_greedy_argmax(const BatchGreedyCell *__restrict__ cells,
   unsigned long long m = 0;
   bool stale = false;
   if (lane < kBlockChunks / kArgmaxWarps && mine * kChunk < c.w.g.space) {
-    if (!all) m = fresh_key(c, mine);
+    if (!all) m = fresh_key(c, __ldcg(c.ckey + mine));
     stale = m == 0;
   }
   for (unsigned todo = __ballot_sync(0xffffffffu, stale); todo;
@@ -642,7 +643,8 @@ k_greedy_refresh(const BatchGreedyCell *__restrict__ cells,
 // (1.2 us) between the phases.  Near a cover a phase is a few microseconds of
 // dependent L2 round trips, so what does not change is kept close: the cell
 // is a kernel parameter, the packed table and its entries sit in shared
-// memory.  On K_3(14,3) a step takes 9 us at gains of 50 and 14 us at 160;
+// memory, the keys of its chunks beside them (7,500 -> 7,380 us for 640
+// steps).  On K_3(14,3) a step takes 9 us at gains of 50 and 14 us at 160;
 // the whole-map argmax, one-block place and refresh launches this replaces
 // took 49 us, the three launches above 25 us (9 of them gaps).  The grid is
 // resident as a whole (a cooperative launch) and every wait is bounded: a
@@ -730,7 +732,7 @@ k_greedy_run(const __grid_constant__ BatchGreedyCell c, int table_words,
   extern __shared__ uint32_t table[];
   __shared__ int4 ent[WALK == kPack ? kMaxPackOff : 1];
   __shared__ WalkSmem smem[kRunWarps];
-  __shared__ unsigned long long wbest[kRunWarps];
+  __shared__ unsigned long long wbest[kRunWarps], keys[kRunThreads];
   __shared__ int stale[kRunThreads], nstale;
   GreedyState *st = reinterpret_cast<GreedyState *>(c.st);
   const WalkArgs &a = c.w;
@@ -752,6 +754,9 @@ k_greedy_run(const __grid_constant__ BatchGreedyCell c, int table_words,
            s.off[(p >> 16) & 255u] + s.off[p >> 24];
   };
   const long long nch = (a.g.space + kChunk - 1) / kChunk;
+  // the first kRunThreads of the block's chunks keep their keys here
+  if (blockIdx.x + (long long)tid * gridDim.x < nch)
+    keys[tid] = __ldcg(c.ckey + blockIdx.x + (long long)tid * gridDim.x);
   const long long nseg = (a.len + kRunPat - 1) / kRunPat;
   unsigned bar = 0;
   for (int i = 0; i < steps; i++, par ^= 1) {
@@ -775,13 +780,19 @@ k_greedy_run(const __grid_constant__ BatchGreedyCell c, int table_words,
       if (tid == 0) nstale = 0;
       __syncthreads();
       if (ch < nch) {
-        const unsigned long long key = fresh_key(c, ch);
-        if (key == 0) stale[atomicAdd(&nstale, 1)] = (int)ch;
+        const unsigned long long key = fresh_key(
+            c, b == blockIdx.x ? keys[tid] : __ldcg(c.ckey + ch));
+        if (key == 0) stale[atomicAdd(&nstale, 1)] = tid;
         k = max(k, key);
       }
       __syncthreads();
-      for (int q = warp; q < nstale; q += kRunWarps)
-        k = max(k, read_chunk(c, stale[q]));
+      for (int q = warp; q < nstale; q += kRunWarps) {
+        const int own = stale[q];
+        const unsigned long long key =
+            read_chunk(c, b + (long long)own * gridDim.x);
+        if (lane == 0 && b == blockIdx.x) keys[own] = key;
+        k = max(k, key);
+      }
     }
     for (int o = 16; o > 0; o >>= 1)
       k = max(k, __shfl_xor_sync(0xffffffffu, k, o));
