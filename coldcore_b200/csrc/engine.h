@@ -127,7 +127,7 @@ struct TmaArgs {
   // padded planes (GroupArgs::pitch): the canonical inner stride, the
   // pitch and the valid words of each padded run
   long long inner_c, pitch, t0;
-  // ternary first group (tern_first): the rows of the cell
+  // first group over row pairs (rows_first): the rows of the cell
   long long rows;
   // 8-bit layer planes (tma_first OUT 5): their byte offset from layers16
   long long off8;

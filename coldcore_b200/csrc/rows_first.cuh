@@ -27,6 +27,11 @@ namespace {
 // padded layout, or T0); the low axes run in between.  No waits: plain loads,
 // one CTA buffer, a barrier between rounds.
 //
+// Bound by the rounds' shared-memory traffic: H3(16,4)'s axes 0..6 take 164 us
+// in a recount and 176 in a gain (183 and 190 with every layer in every round
+// and 4-byte copies out), where their bytes alone would take 66 and 79; Lee
+// 7^8's axes 0..3 take 28.5 us (31; the register kernel 65).
+//
 // Axes a round: two for Q = 3 (9-word blocks), and for Q = 4 up to four
 // layers (64 registers); one otherwise.
 template <int C, int R1>

@@ -1,6 +1,6 @@
 // transform_first_q.cu — the first groups over row pairs of Hamming axes of 4
-// to 6, Lee axes of 4 to 7 and ternary cells of R = 2 (rows_first.cuh): rows of up to 4,096 words, so
-// that two to four CTAs of R1 x T0 lanes share an SM.
+// to 6, Lee axes of 4 to 7 and ternary cells of R = 2 (rows_first.cuh): rows
+// of up to 4,096 words, so that two to four CTAs of R1 x T0 lanes share an SM.
 #include "rows_first.cuh"
 
 namespace cc {

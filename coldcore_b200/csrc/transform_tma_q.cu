@@ -1,6 +1,8 @@
 // transform_tma_q.cu — the streamed groups of Hamming axes of 4 to 6, Lee axes
-// of 4 to 7 and ternary cells of R = 2 (tma_group.cuh), all in a padded plan's layout: OUT 0 writes
-// layers, 3 the map and 4 the cnt at their canonical index.
+// of 4 to 7 and ternary cells of R = 2 (tma_group.cuh), all in a padded plan's
+// layout: OUT 0 writes layers, 3 the map and 4 the cnt at their canonical
+// index.  Lee 7^8's two strided launches take 16 us each, 45 and 41 with the
+// register kernels.
 //
 // A group takes as many axes as keep its tile's middle extent within 256, the
 // tensor map's box limit, and two stages within shared memory; tiles of up to
