@@ -16,7 +16,6 @@
 // word's digits, axis sizes and strides sit in shared memory, and each
 // thread resolves one pattern at a time with a few integer ops per slot.
 #include <algorithm>
-#include <array>
 #include <cstdlib>
 
 #include "engine.h"
@@ -105,27 +104,31 @@ bool metric_ball_table(const Geometry &g, const std::vector<int32_t> &soa,
     if (g.prob == kHamming) return 1;
     return c > g.R ? -1 : sum ? c : 0;
   };
-  std::vector<std::array<int32_t, kMaxSlots>> rows((size_t)len);
+  static_assert(kMaxAxes <= 64, "one bit an axis");
+  std::vector<long long> words((size_t)len);        // around word 0
   for (long long t = 0; t < len; t++) {
-    auto &row = rows[(size_t)t];
-    row.fill(0);
-    int w = 0, m = 0;
+    unsigned long long moved = 0;
+    long long x = 0;
+    int w = 0;
+    bool open = true;
     for (int k = 0; k < slots; k++) {
       const int32_t c = soa[(size_t)k * len + t];
-      if (!c) continue;
-      if (m < k || (c >> 24) >= g.n) return false;   // a walk stops at a gap
-      const int e = weight(c >> 24, c & 0xFFFFFF);
+      if (!c) { open = false; continue; }
+      const int pos = c >> 24, d = c & 0xFFFFFF;
+      // a walk stops at a gap
+      if (!open || pos >= g.n || (moved >> pos & 1)) return false;
+      moved |= 1ULL << pos;
+      const int e = weight(pos, d);
       if (e < 0) return false;
       w += e;
-      row[m++] = c;
+      x += d * g.pw[pos];
     }
     if (w > g.R) return false;
-    std::sort(row.begin(), row.begin() + m);
-    for (int k = 1; k < m; k++)
-      if (row[k] >> 24 == row[k - 1] >> 24) return false;
+    words[(size_t)t] = x;
   }
-  std::sort(rows.begin(), rows.end());
-  if (std::adjacent_find(rows.begin(), rows.end()) != rows.end()) return false;
+  std::sort(words.begin(), words.end());
+  if (std::adjacent_find(words.begin(), words.end()) != words.end())
+    return false;
   // |B|: coefficients 0..W of prod_j (1 + sum_d t^weight(j, d))
   const int W = sum ? g.R : 0;
   std::vector<long double> poly(W + 1, 0.0L);
