@@ -225,8 +225,14 @@ GroupPlan rows_first_variant(const GroupPlan &p, int threads);
 int launch_tma_group(const GroupPlan &p, cudaStream_t s);
 int tma_prepare(const GroupPlan &p);
 int tma_blocks_per_sm(const GroupPlan &p);
-int tma_fault_pending();
-void tma_fault_clear();
+// A streamed launch that gave up waiting for its loads leaves its output
+// unfinished: -8 (and a message) when one has since the last look, else 0.
+// To be asked once the launches in question have drained.
+int tma_fault_take();
+// Failures made on the host, for tests of the paths behind them
+// (dct_b200_fault_inject): true when this event of `kind` is the armed one.
+enum FaultKind { kFaultStreamed = 0, kFaultKinds = 1 };
+bool fault_due(int kind);
 int launch_code_bounds(const long long *code, long long ncode,
                        long long tile_words, long long ntiles,
                        long long *bounds, cudaStream_t s);

@@ -593,13 +593,7 @@ int run_streamed(int init_mode, int out_mode) {
 }
 
 int run_transform(int init_mode, int out_mode) {
-  if (tma_fault_pending()) {
-    // an earlier streamed launch gave up waiting for its tile loads
-    tma_fault_clear();
-    fprintf(stderr, "coldcore_b200: a streamed group launch timed out "
-            "waiting for its tensor loads\n");
-    return -8;
-  }
+  if (const int rc = tma_fault_take()) return rc;   // a tuning launch's
   if (S.streamed) return run_streamed(init_mode, out_mode);
   Plan &P = plan_for(init_mode, out_mode);
   int pm, pt;
@@ -1124,12 +1118,6 @@ bool gather_transform_pays(const Plan &P, long long nw) {
 }
 
 int run_gather_transform(const Plan &P, int mode, int target) {
-  if (tma_fault_pending()) {
-    tma_fault_clear();
-    fprintf(stderr, "coldcore_b200: a streamed group launch timed out "
-            "waiting for its tensor loads\n");
-    return -8;
-  }
   for (const auto &gp : P.groups) {
     GroupPlan p = gp;
     p.a.pmode = mode;
@@ -1163,10 +1151,12 @@ int gather_impl(const long long *words, int nwords, int mode, int target,
   }
   if (counts) {
     S.stats[1] += (nwords + kStageCap - 1) / kStageCap;
-    return staged_words(words, nwords, out,
-                        [&](const long long *w, int nb, int32_t *o) {
-                          return launch_read_at(counts, w, nb, o, g_stream);
-                        });
+    const int rc = staged_words(
+        words, nwords, out, [&](const long long *w, int nb, int32_t *o) {
+          return launch_read_at(counts, w, nb, o, g_stream);
+        });
+    // the streams have drained: a launch that timed out is this call's
+    return rc ? rc : tma_fault_take();
   }
   for (long long off = 0; off < nwords; off += kStageCap) {
     const int nb = (int)std::min<long long>(kStageCap, nwords - off);
@@ -1405,6 +1395,7 @@ int dct_transform(int init_mode, int out_mode) {
   rc = run_transform(init_mode, out_mode);
   if (rc) return rc;
   CC_CK(cudaStreamSynchronize(g_stream));
+  if ((rc = tma_fault_take())) return rc;
   S.code_in_flight = false;
   S.layered_out = out_mode == 3;
   if (out_mode == 2) {

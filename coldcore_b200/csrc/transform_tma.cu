@@ -30,10 +30,13 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <atomic>
+#include <cstdio>
 #include <cstring>
 #include <mutex>
 #include <unordered_map>
 
+#include "../../include/coldcore_b200/plugin.h"
 #include "engine.h"
 #include "rows_first.cuh"
 #include "tma_group.cuh"
@@ -590,12 +593,20 @@ GroupPlan rows_first_variant(const GroupPlan &p, int threads) {
   return v;
 }
 
-int tma_fault_pending() {
-  return g_fault_host && *(volatile int *)g_fault_host ? 1 : 0;
+int tma_fault_take() {
+  volatile int *f = g_fault_host;
+  if (!f || !*f) return 0;
+  *f = 0;
+  fprintf(stderr, "coldcore_b200: a streamed group launch timed out "
+          "waiting for its tensor loads\n");
+  return -8;
 }
 
-void tma_fault_clear() {
-  if (g_fault_host) *(volatile int *)g_fault_host = 0;
+static std::atomic<int> g_inject[kFaultKinds];
+
+bool fault_due(int kind) {
+  std::atomic<int> &c = g_inject[kind];
+  return c.load() > 0 && c.fetch_sub(1) == 1;
 }
 
 namespace {
@@ -910,7 +921,14 @@ int launch_tma_group(const GroupPlan &p, cudaStream_t s) {
   grid = grid_knob(grid, a.ntiles);
   tma_entry(e).fn<<<grid, p.threads, smem, s>>>(map, t);
   CC_CK(cudaGetLastError());
+  if (fault_due(kFaultStreamed)) *(volatile int *)g_fault_host = 1;
   return 0;
 }
 
 }  // namespace cc
+
+extern "C" int dct_b200_fault_inject(int kind, int nth) {
+  if (kind < 0 || kind >= cc::kFaultKinds || nth < 0) return -1;
+  cc::g_inject[kind] = nth;
+  return 0;
+}

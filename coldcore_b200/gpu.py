@@ -101,6 +101,7 @@ def _bind(path):
         "dct_b200_ball_hist": (I, [_LLP, I, I, I, _I32P]),
         "dct_b200_layers_at": (I, [_LLP, I, _I32P]),
         "dct_b200_greedy_fill": (I, [I, _LLP, _LLP]),
+        "dct_b200_fault_inject": (I, [I, I]),
         "dct_b200_last_timings": (I, [ctypes.POINTER(ctypes.c_float), I]),
         "dct_b200_ooc_plan": (I, [I, I, ctypes.POINTER(I), I, I, I, _LL, _LL,
                                   _LL, I, _LLP, I]),

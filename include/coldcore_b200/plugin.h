@@ -301,6 +301,11 @@ CCP_API int  dct_b200_layers_at(const long long *idx, int k, int32_t *out);
 CCP_API int  dct_b200_greedy_fill(int max_add, long long *placed,
                                   long long *deficit);
 CCP_API int  dct_b200_read_layer(int d, long long off, long long len, int32_t *out);
+/* Tests of the error paths: the nth event of `kind` from now fails as seen
+ * from the host (0 disarms; nothing fails on the device).  Kind 0: a streamed
+ * launch reports that it timed out waiting for its tensor loads, so the call
+ * that queued it returns -8. */
+CCP_API int  dct_b200_fault_inject(int kind, int nth);
 
 /* ---- out-of-core (ooc) cells: distance layers in host memory ----
  * Replaces the reference's host placement of the layer planes

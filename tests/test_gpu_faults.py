@@ -1,0 +1,59 @@
+"""Calls whose device work fails report it themselves and leave the cell in
+a state that the next calls answer from correctly.  The failures are made on
+the host (dct_b200_fault_inject); nothing fails on the device."""
+import numpy as np
+import pytest
+
+from coldcore_b200.gpu import GpuBackend
+from oracle.dp_oracle import OracleBackend
+
+pytestmark = pytest.mark.gpu
+
+STREAMED = 0                             # dct_b200_fault_inject kinds
+
+
+@pytest.fixture
+def streamed_cell(monkeypatch):
+    """A ternary cell whose plans stream, untuned, at a 60% cover."""
+    monkeypatch.setenv("CC_TMA", "1")
+    monkeypatch.setenv("CC_TUNE", "0")
+    monkeypatch.setenv("DCT_SET_GATHER", "0")
+    axes, R = [3] * 12, 4
+    size = 3 ** 12
+    code = np.random.default_rng(4).choice(size, 60, replace=False)
+    with GpuBackend(axes, R) as b:
+        yield b, code, OracleBackend(axes, R)
+        b._lib.dct_b200_fault_inject(STREAMED, 0)
+
+
+def test_a_streamed_time_out_is_the_failing_transforms_error(streamed_cell):
+    b, code, o = streamed_cell
+    b.recount(code)
+    o.recount(code)
+    b._lib.dct_b200_fault_inject(STREAMED, 1)
+    with pytest.raises(RuntimeError):
+        b.gain_map()
+    b.gain_map()                         # reported once, by that call
+    o.gain_map()
+    assert np.array_equal(b.map_all(), o.map)
+
+
+def test_a_streamed_time_out_is_the_failing_gathers_error(streamed_cell,
+                                                          monkeypatch):
+    """Untuned (straight after a recount) and with the plan of an earlier
+    gain map: the call answered by one transform reports, the next one and
+    the next transform are right."""
+    b, code, o = streamed_cell
+    monkeypatch.setenv("CC_GATHER_TRANSFORM", "1")
+    b.recount(code)
+    o.recount(code)
+    cands = np.random.default_rng(1).integers(0, 3 ** 12, 5000)
+    want = o.ball_gather(cands[:200], 0)
+    for _ in range(2):
+        b._lib.dct_b200_fault_inject(STREAMED, 1)
+        with pytest.raises(RuntimeError):
+            b.ball_gather(cands, 0)
+        assert np.array_equal(b.ball_gather(cands, 0)[:200], want)
+        b.gain_map()
+    o.gain_map()
+    assert np.array_equal(b.map_all(), o.map)
