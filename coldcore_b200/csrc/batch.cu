@@ -1022,8 +1022,11 @@ int dct_batch_build(long long h, int tile_kb) {
 int dct_batch_run(long long h, int mode) {
   Batch *b = get(h);
   if (!b || !b->built) return -1;
-  if (mode == 0) return run_persistent(b);
-  if (mode == 1) return run_per_pass(b);
+  if (mode == 0 || mode == 1) {
+    const int rc = mode == 0 ? run_persistent(b) : run_per_pass(b);
+    const int late = tma_fault_take();   // the launches have drained
+    return rc ? rc : late;
+  }
   if (mode == 2) {
     // self-test of the bounded dependency wait: one launch in which the
     // first pass needs one more tile than it has, so its dependents time
@@ -1547,7 +1550,8 @@ int dct_batch_greedy(long long h, const int *cells, int n, const int *max_add,
     if (!rc && err) rc = -7;
   }
   cudaStreamSynchronize(b->stream);
-  return rc;
+  const int late = tma_fault_take();     // a rebuild's streamed launch
+  return rc ? rc : late;
 }
 
 // mode 0: #{x : cnt[x] == target}; 1: the deficit sum max(0, mu - cnt)

@@ -194,7 +194,8 @@ CCP_API int  dct_batch_add(long long h, int problem, int n, const int *ax,
 CCP_API int  dct_batch_build(long long h, int tile_kb);
 /* mode 0: the persistent graph launch; 1: one launch per pass per cell
  * (same kernels and streams, no graph); 2: self-test of the bounded
- * dependency wait (returns -7, no hang) */
+ * dependency wait (returns -7, no hang).  -7 / -8: a bounded wait of the
+ * step ran out; the next run computes every field afresh. */
 CCP_API int  dct_batch_run(long long h, int mode);
 /* field 0 cnt (uint16), 1 gain map (int32), 2 loss map (int32) */
 CCP_API int  dct_batch_read(long long h, int cell, int field, long long off,

@@ -57,3 +57,36 @@ def test_a_streamed_time_out_is_the_failing_gathers_error(streamed_cell,
         b.gain_map()
     o.gain_map()
     assert np.array_equal(b.map_all(), o.map)
+
+
+def test_a_streamed_time_out_is_the_failing_batch_calls_error(monkeypatch):
+    """A step of one launch per pass and a greedy whose gain rebuilds stream:
+    each reports, and the next step and greedy are the oracle's."""
+    from coldcore_b200.batch import BatchEngine
+    from coldcore_b200.patterns import wide_table
+    monkeypatch.setenv("CC_TUNE", "0")
+    monkeypatch.setenv("CC_GREEDY_REBUILD", "1")
+    axes, R = (3,) * 11, 3
+    code = np.random.default_rng(6).choice(3 ** 11, 80, replace=False)
+    o = OracleBackend(list(axes), R)
+    o.recount(code)
+    with BatchEngine() as e:
+        e.add("hamming", axes, R, code)
+        e.build(48)
+        e.set_table(0, wide_table(axes, R, "hamming"))
+        lib = e._lib
+        for mode in (0, 1):
+            lib.dct_b200_fault_inject(STREAMED, 1)
+            assert e.run_rc(1) == -8
+            e.run(mode)
+            assert np.array_equal(e.cnt(0), o.read_cnt())
+            lib.dct_b200_fault_inject(STREAMED, 1)
+            with pytest.raises(RuntimeError):
+                e.greedy([0], [4])
+        lib.dct_b200_fault_inject(STREAMED, 0)
+        e.run(0)
+        assert e.scalars()[0, 0] == o.uncovered()
+        (placed, deficit), = e.greedy([0], [4])
+        o.ball_update(placed, 1)
+        assert deficit == o.uncovered()
+        assert np.array_equal(e.cnt(0), o.read_cnt())
