@@ -76,6 +76,14 @@ inline int max_mult(const MultHist &h) {
   return h.empty() ? 0 : h.rbegin()->first;
 }
 
+// a greedy's state and its launches' barrier state as they lie on the device
+struct GreedySlot {
+  GreedyHost st;
+  char pad[64 - kGreedyStateBytes];
+  int run[kGreedyRunBytes / 4];    // [1]: a barrier timed out
+};
+static_assert(sizeof(GreedySlot) == 64 + kGreedyRunBytes, "greedy slot");
+
 struct State {
   bool live = false;
   Geometry g{};
@@ -133,6 +141,7 @@ struct State {
   long long stats[8] = {0};
   long long bytes_dev = 0, bytes_host = 0;
   unsigned long long dd_last = 0;
+  bool torn = false;               // a call failed while it changed cnt
   bool layered_out = false;        // last transform left N_0..N_R
   // set side (setside.cu): the listed predicate set Z, cached per cnt state
   bool metric_table = false;       // support table proven == metric ball
@@ -155,7 +164,7 @@ struct State {
   // device greedy: state, placed words, words satisfied per placement
   // [the cell's BatchGreedyCell][its state][chunk keys][fresh words]
   char *d_greedy = nullptr;
-  GreedyHost *h_greedy = nullptr;  // pinned ring of kGreedyRing states
+  GreedySlot *h_greedy = nullptr;  // pinned ring of kGreedyRing states
   cudaEvent_t ev_greedy[kGreedyRing] = {nullptr};
   long long *d_placed = nullptr, *h_placed = nullptr;
   long long placed_cap = 0;
@@ -300,6 +309,16 @@ int check_update(const long long *words, int nw, int delta, Batch1 &batch) {
     if (!within_counter(S.active_size + nw, mx)) return -1;
   }
   return 0;
+}
+
+// 0 where cnt is the counters of the active multiset; -1 without a cell, -8
+// after a call that failed while it changed cnt, until a recount
+int cnt_ready() {
+  if (!S.live) return -1;
+  if (!S.torn) return 0;
+  fprintf(stderr, "coldcore_b200: an earlier call failed while it changed "
+          "the counters; recount first\n");
+  return -8;
 }
 
 int fetch_scalar(long long *r, int slot = 0) {
@@ -594,11 +613,19 @@ int run_streamed(int init_mode, int out_mode) {
 
 int run_transform(int init_mode, int out_mode) {
   if (const int rc = tma_fault_take()) return rc;   // a tuning launch's
-  if (S.streamed) return run_streamed(init_mode, out_mode);
+  if (S.streamed) {
+    const int rc = run_streamed(init_mode, out_mode);
+    // begun: neither refused (arguments, no split, host planes too few) nor
+    // out of device memory for its pieces
+    S.torn = S.torn || (out_mode == 2 && rc < -5 &&
+                        rc != -(100 + (int)cudaErrorMemoryAllocation));
+    return rc;
+  }
   Plan &P = plan_for(init_mode, out_mode);
   int pm, pt;
   set_predicate(init_mode, &pm, &pt);
   int nt = 0, rc = 0;
+  if (!P.window && P.groups.empty()) return -1;   // the planner found no tile
   if (P.window) {
     if (init_mode == 0) {
       int32_t *pl = S.layers + P.scatter_plane * S.plane;
@@ -606,6 +633,7 @@ int run_transform(int init_mode, int out_mode) {
       rc = launch_scatter(pl, S.d_code, S.codeM, g_stream);
       if (rc) return rc;
     }
+    S.torn = S.torn || out_mode == 2;    // until the recount has drained
     if ((rc = timing_mark(nt))) return rc;
     for (auto &w : P.passes) {
       WindowArgs x = w;
@@ -616,7 +644,6 @@ int run_transform(int init_mode, int out_mode) {
       if ((rc = timing_mark(++nt))) return rc;
     }
   } else {
-    if (P.groups.empty()) return -1;           // the planner found no tile
     if (init_mode == 0) {
       const GroupArgs &a0 = P.groups[0].a;
       const long long need = a0.ntiles + 1;
@@ -632,6 +659,7 @@ int run_transform(int init_mode, int out_mode) {
                               S.d_bounds, g_stream);
       if (rc) return rc;
     }
+    S.torn = S.torn || out_mode == 2;
     if ((rc = timing_mark(nt))) return rc;
     for (auto &gp : P.groups) {
       GroupPlan p = gp;
@@ -1390,12 +1418,17 @@ int dct_transform(int init_mode, int out_mode) {
       (out_mode == 2 && init_mode != 0))
     return -1;
   if (out_mode == 3 && S.R1 == 1) return -1;
-  int rc = autotune(init_mode, out_mode);
+  int rc = init_mode ? cnt_ready() : 0;
+  if (rc) return rc;
+  rc = autotune(init_mode, out_mode);
   if (rc) return rc;
   rc = run_transform(init_mode, out_mode);
   if (rc) return rc;
   CC_CK(cudaStreamSynchronize(g_stream));
-  if ((rc = tma_fault_take())) return rc;
+  if ((rc = tma_fault_take())) {
+    S.torn = S.torn || out_mode == 2;
+    return rc;
+  }
   S.code_in_flight = false;
   S.layered_out = out_mode == 3;
   if (out_mode == 2) {
@@ -1405,16 +1438,18 @@ int dct_transform(int init_mode, int out_mode) {
     S.active_size = S.codeM;
     S.act_hist = S.up_hist;
     S.cnt_ver++;
+    S.torn = false;
   }
   return 0;
 }
 
 int dct_ball_update(const long long *words, int nwords, int delta) {
-  if (!S.live) return -1;
+  int rc = cnt_ready();
+  if (rc) return rc;
   Batch1 batch;
   if (check_update(words, nwords, delta, batch)) return -1;
   if (nwords == 0) return 0;
-  int rc = update_impl(words, nwords, delta, nullptr);
+  rc = update_impl(words, nwords, delta, nullptr);
   if (rc) return rc;
   apply_active(batch, delta, nwords);
   return 0;
@@ -1424,12 +1459,13 @@ int dct_ball_update_delta(const long long *words, int nwords, int delta,
                           long long *dd) {
   if (!dd) return -1;
   *dd = 0;
-  if (!S.live) return -1;
+  int rc = cnt_ready();
+  if (rc) return rc;
   Batch1 batch;
   if (check_update(words, nwords, delta, batch)) return -1;
   if (nwords == 0) return 0;
   auto *trans = reinterpret_cast<unsigned long long *>(S.d_scalar + 2);
-  int rc = update_impl(words, nwords, delta, trans);
+  rc = update_impl(words, nwords, delta, trans);
   if (rc) return rc;
   long long now;
   rc = fetch_scalar(&now, 2);
@@ -1443,13 +1479,13 @@ int dct_ball_update_delta(const long long *words, int nwords, int delta,
 
 int dct_ball_gather(const long long *words, int nwords, int target,
                     int32_t *out) {
-  if (!S.live) return -1;
+  if (const int rc = cnt_ready()) return rc;
   return gather_impl(words, nwords, kPredEq, target, out);
 }
 
 int dct_ball_gather_mu(const long long *words, int nwords, int role,
                        int32_t *out) {
-  if (!S.live) return -1;
+  if (const int rc = cnt_ready()) return rc;
   if (nwords <= 0) return 0;
   if (role < 0 || role > 1) return -1;
   return gather_impl(words, nwords, role == 0 ? kPredDef : kPredCrit, 0, out);
@@ -1538,6 +1574,7 @@ int swap_eval_fast(const long long *drops, int k, const long long *cand,
 // Returns the number placed, or a negative error.  The map is clobbered.
 int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
   if (!S.live || max_add < 0 || (max_add && !placed) || !deficit) return -1;
+  if (const int rc = cnt_ready()) return rc;
   if (S.g.space >= (1LL << 32)) return -1;    // 32-bit index in the key
   // placed words are new (multiplicity 1): the counters stay within uint16
   if (!within_counter(S.active_size + max_add, std::max(max_mult(S.act_hist), 1)))
@@ -1551,7 +1588,7 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
   const size_t o_fresh = o_key + (size_t)nch * 8;
   if (!S.d_greedy) {
     CC_CK(cudaMalloc(&S.d_greedy, o_fresh + (size_t)S.len * 8));
-    CC_CK(cudaHostAlloc((void **)&S.h_greedy, kGreedyRing * kGreedyStateBytes,
+    CC_CK(cudaHostAlloc((void **)&S.h_greedy, kGreedyRing * sizeof(GreedySlot),
                         cudaHostAllocDefault));
     for (auto &ev : S.ev_greedy)
       CC_CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
@@ -1641,7 +1678,7 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
   }
   if (S.streamed || !S.metric_table || S.fmt != 0) rebuild_us = 1e30;
   auto read_state = [&](int slot) -> int {
-    CC_CK(cudaMemcpyAsync(S.h_greedy + slot, gc.st, sizeof(st),
+    CC_CK(cudaMemcpyAsync(S.h_greedy + slot, gc.st, sizeof(GreedySlot),
                           cudaMemcpyDeviceToHost, g_stream));
     CC_CK(cudaEventRecord(S.ev_greedy[slot], g_stream));
     return 0;
@@ -1654,6 +1691,8 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
   const long long steps = std::min<long long>(max_add, d0);
   long long issued = 0, chunk = 32;
   bool follow = true;
+  S.cnt_ver++;
+  S.torn = true;                   // until every step has been accounted for
   while (issued < steps) {
     if (follow) {
       const int par = (int)(issued & 1);
@@ -1662,7 +1701,7 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
       if (rc || (rc = read_state(par))) return rc;
       const int look = issued ? par ^ 1 : par;
       CC_CK(cudaEventSynchronize(S.ev_greedy[look]));
-      const GreedyHost &h = S.h_greedy[look];
+      const GreedyHost &h = S.h_greedy[look].st;
       if (h.done) break;
       const bool rebuild = greedy_rebuild_pays(h.gain(look), S.len,
                                                rebuild_us);
@@ -1680,22 +1719,22 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
                            g_stream);
     if (rc) return rc;
     issued += n;
+    if (fault_due(kFaultBarrier))
+      CC_CK(cudaMemsetAsync(reinterpret_cast<int *>(run) + 1, 1, 1, g_stream));
     if ((rc = read_state(0))) return rc;
     CC_CK(cudaEventSynchronize(S.ev_greedy[0]));
-    if (S.h_greedy[0].done) break;
+    if (S.h_greedy[0].run[1]) {    // no further launch on a half-done step
+      fprintf(stderr, "coldcore_b200: a greedy launch timed out at its grid "
+              "barrier\n");
+      return -8;
+    }
+    if (S.h_greedy[0].st.done) break;
     chunk = std::min<long long>(chunk * 2, 512);
   }
   if ((rc = read_state(0))) return rc;
-  int tail[kGreedyRunBytes / 4] = {0};
-  CC_CK(cudaMemcpyAsync(tail, run, kGreedyRunBytes, cudaMemcpyDeviceToHost,
-                        g_stream));
   CC_CK(cudaStreamSynchronize(g_stream));
-  if (tail[1]) {
-    fprintf(stderr, "coldcore_b200: a greedy launch timed out at its grid "
-            "barrier\n");
-    return -8;
-  }
-  st = S.h_greedy[0];
+  if ((rc = tma_fault_take())) return rc;      // a rebuild's streamed launch
+  st = S.h_greedy[0].st;
   const int n = st.placed_now();
   if (n) {
     CC_CK(cudaMemcpyAsync(S.h_placed, S.d_placed, (size_t)n * 8,
@@ -1706,7 +1745,7 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
     count_words(placed, n, batch);
     apply_active(batch, +1, n);
   }
-  S.cnt_ver++;
+  S.torn = false;
   *deficit = st.deficit_now();
   return n;
 }
@@ -1717,7 +1756,7 @@ int dct_b200_greedy_fill(int max_add, long long *placed, long long *deficit) {
 
 int dct_swap_eval(const long long *drops, int k, const long long *cand,
                   const long long *off, int32_t *gain, int32_t *loss) {
-  if (!S.live) return -1;
+  if (const int rc = cnt_ready()) return rc;
   if (k <= 0) return 0;
   if (k > 65535 || !off || off[0] != 0 || !drops || !loss) return -1;
   for (int i = 0; i < k; i++)
@@ -1763,6 +1802,7 @@ int dct_loss_owner(const long long *words, int M, int32_t *out) {
   // hold the staged code
   const int to = S.act == S.up ? 1 - S.up : S.act;
   if (S.code_buf[to].reserve(M)) return -2;
+  S.torn = true;
   CC_CK(cudaMemsetAsync(S.cnt, 0, (size_t)S.cnt_len * 2, g_stream));
   int rc = update_impl(words, M, +1, nullptr);
   if (rc) return rc;
@@ -1774,6 +1814,7 @@ int dct_loss_owner(const long long *words, int M, int32_t *out) {
   S.delta.clear();
   S.active_size = M;
   S.act_hist.swap(hist);
+  S.torn = false;
   if (M == 0) return 0;
   int lm, lt;
   mode_role(1, &lm, &lt);
@@ -1787,7 +1828,7 @@ int dct_stats(long long *out, int n) {
 }
 
 long long dct_count_eq(int target) {
-  if (!S.live) return -1;
+  if (const int rc = cnt_ready()) return rc;
   // the zero-word list of a set-side gather already counted them
   if (target == 0 && S.z_valid && S.z_ver == S.cnt_ver &&
       (S.z_mode == kPredEq ? S.z_target == 0
@@ -1804,8 +1845,9 @@ long long dct_count_eq(int target) {
 }
 
 long long dct_count_deficit(void) {
-  if (!S.live) return -1;
-  int rc = launch_cnt_reduce(S.cnt, S.g.space, kPredDef, 0, g_mu,
+  int rc = cnt_ready();
+  if (rc) return rc;
+  rc = launch_cnt_reduce(S.cnt, S.g.space, kPredDef, 0, g_mu,
                              S.d_scalar + kQuerySlot, g_stream, red_out());
   if (rc) return rc;
   long long r;
@@ -1902,6 +1944,7 @@ int dct_read_cnt(long long off, long long len, uint16_t *out) {
   if (!S.live || off < 0 || len < 0 || off + len > S.g.space ||
       (len && !out))
     return -1;
+  if (const int rc = cnt_ready()) return rc;
   if (len)
     CC_CK(cudaMemcpyAsync(out, S.cnt + off, (size_t)len * 2,
                           cudaMemcpyDefault, g_stream));
@@ -2040,6 +2083,7 @@ int dct_b200_ball_hist(const long long *words, int nw, int src, int nbins,
     return -1;
   if (nw <= 0) return 0;
   if (!valid_words(words, nw)) return -1;
+  if (const int rc = src == 1 ? cnt_ready() : 0) return rc;
   const WalkArgs w = walk_args();
   const long long cap = kStageCap / nbins;   // nb * nbins fits d_out
   for (long long off = 0; off < nw; off += cap) {

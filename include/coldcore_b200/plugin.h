@@ -298,14 +298,19 @@ CCP_API int  dct_b200_layers_at(const long long *idx, int k, int32_t *out);
  * positive gain, or max_add words are placed.  placed (capacity max_add)
  * receives the words in placement order and joins the active multiset;
  * *deficit receives the total deficit left.  Returns the number placed or a
- * negative code.  The map (plane 0) is overwritten.  |X| < 2^32. */
+ * negative code.  The map (plane 0) is overwritten.  |X| < 2^32.
+ *
+ * A recount or a greedy that fails once its launches have begun leaves cnt
+ * between two states: every call that reads cnt then returns -8 until a
+ * recount (or dct_loss_owner, or dct_free) has set it. */
 CCP_API int  dct_b200_greedy_fill(int max_add, long long *placed,
                                   long long *deficit);
 CCP_API int  dct_b200_read_layer(int d, long long off, long long len, int32_t *out);
 /* Tests of the error paths: the nth event of `kind` from now fails as seen
  * from the host (0 disarms; nothing fails on the device).  Kind 0: a streamed
  * launch reports that it timed out waiting for its tensor loads, so the call
- * that queued it returns -8. */
+ * that queued it returns -8.  Kind 1: a launch of dct_b200_greedy_fill reports
+ * a time-out at its grid barrier. */
 CCP_API int  dct_b200_fault_inject(int kind, int nth);
 
 /* ---- out-of-core (ooc) cells: distance layers in host memory ----

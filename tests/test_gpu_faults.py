@@ -9,7 +9,7 @@ from oracle.dp_oracle import OracleBackend
 
 pytestmark = pytest.mark.gpu
 
-STREAMED = 0                             # dct_b200_fault_inject kinds
+STREAMED, BARRIER = 0, 1                 # dct_b200_fault_inject kinds
 
 
 @pytest.fixture
@@ -90,3 +90,78 @@ def test_a_streamed_time_out_is_the_failing_batch_calls_error(monkeypatch):
         o.ball_update(placed, 1)
         assert deficit == o.uncovered()
         assert np.array_equal(e.cnt(0), o.read_cnt())
+
+
+def refuses(b, w):
+    """Every call that reads cnt is refused."""
+    calls = [lambda: b.gain_map(), lambda: b.loss_map(), lambda: b.uncovered(),
+             lambda: b.ball_gather(w, 0), lambda: b.ball_update(w, 1),
+             lambda: b.ball_update_delta(w, 1), lambda: b.read_cnt(),
+             lambda: b.swap_eval(w, w), lambda: b.greedy_fill_device(1)]
+    for i, call in enumerate(calls):
+        with pytest.raises(RuntimeError):
+            call()
+            raise AssertionError(f"call {i} answered")
+
+
+@pytest.mark.parametrize("axes,R", [([2] * 14, 2), ([3] * 9, 2)])
+def test_a_greedy_that_times_out_stops_and_asks_for_a_recount(axes, R,
+                                                              monkeypatch):
+    """A barrier time-out ends the greedy at that launch: the launch after it
+    would start on a half-done step.  cnt then lies between two states: no
+    call answers from it, nor from a list of the deficient words made before
+    the greedy, until a recount."""
+    monkeypatch.setenv("CC_GREEDY_REBUILD", "0")
+    monkeypatch.setenv("DCT_SET_GATHER", "2")
+    size = int(np.prod(axes))
+    code = np.random.default_rng(2).choice(size, 20, replace=False)
+    o = OracleBackend(axes, R)
+    o.recount(code)
+    cands = np.arange(0, size, 7)
+    with GpuBackend(axes, R) as b:
+        b.recount(code)
+        before = b.uncovered()
+        assert np.array_equal(b.ball_gather(cands, 0), o.ball_gather(cands, 0))
+        b._lib.dct_b200_fault_inject(BARRIER, 1)
+        with pytest.raises(RuntimeError):
+            b.greedy_fill_device(60)
+        refuses(b, code[:3])
+        b.recount(code)
+        assert b.uncovered() == before == o.uncovered()
+        placed, deficit = b.greedy_fill_device(60)
+        o.ball_update(placed, 1)
+        assert deficit == o.uncovered() == b.uncovered()
+        b.ball_update(placed, -1)        # they are active words
+        assert b.uncovered() == before
+
+
+def test_a_recount_that_times_out_asks_for_a_recount(streamed_cell):
+    b, code, o = streamed_cell
+    b.recount(code)
+    b._lib.dct_b200_fault_inject(STREAMED, 1)
+    with pytest.raises(RuntimeError):
+        b.recount(code[:40])
+    refuses(b, code[:2])
+    b.recount(code[:40])
+    o.recount(code[:40])
+    assert np.array_equal(b.read_cnt(), o.read_cnt())
+    b.ball_update(code[:2], -1)
+    o.ball_update(code[:2], -1)
+    assert b.uncovered() == o.uncovered()
+
+
+def test_a_greedy_rebuild_that_times_out_is_the_greedys_error(streamed_cell,
+                                                              monkeypatch):
+    b, code, o = streamed_cell
+    monkeypatch.setenv("CC_GREEDY_REBUILD", "1")
+    b.recount(code)
+    b.gain_map()
+    b._lib.dct_b200_fault_inject(STREAMED, 2)
+    with pytest.raises(RuntimeError):
+        b.greedy_fill_device(3)
+    refuses(b, code[:2])
+    b.recount(code)
+    o.recount(code)
+    placed, deficit = b.greedy_fill_device(3)
+    o.ball_update(placed, 1)
+    assert deficit == o.uncovered()
