@@ -1444,6 +1444,8 @@ int dct_batch_greedy(long long h, const int *cells, int n, const int *max_add,
   up(o_jam, jam.data(), jam.size() * 8);
   up(o_jpl, jpl.data(), jpl.size() * 8);
   up(o_flag, flag.data(), (size_t)n * 4);
+  // the rebuilds' error word: an earlier step's is not this call's
+  ck(cudaMemsetAsync(b->d_err, 0, 4, b->stream));
   // incumbents never re-enter
   if (!rc) rc = launch_greedy_exclude(dtab, n, nullptr, kExcluded, b->stream);
   GreedyHost *ring[2] = {

@@ -165,3 +165,27 @@ def test_a_greedy_rebuild_that_times_out_is_the_greedys_error(streamed_cell,
     placed, deficit = b.greedy_fill_device(3)
     o.ball_update(placed, 1)
     assert deficit == o.uncovered()
+
+
+@pytest.mark.parametrize("rebuild", ["0", "1"])
+def test_an_error_of_an_earlier_step_is_not_a_greedys(rebuild, monkeypatch):
+    """The dependency-wait self-test leaves its error word; the step of one
+    launch per pass after it is right, and so is the greedy from that step."""
+    from coldcore_b200.batch import BatchEngine
+    from coldcore_b200.patterns import wide_table
+    monkeypatch.setenv("CC_GREEDY_REBUILD", rebuild)
+    axes, R = (2,) * 13, 1
+    code = np.random.default_rng(7).choice(2 ** 13, 30, replace=False)
+    o = OracleBackend(list(axes), R)
+    o.recount(code)
+    with BatchEngine() as e:
+        e.add("hamming", axes, R, code)
+        e.build(16)
+        e.set_table(0, wide_table(axes, R, "hamming"))
+        assert e.run_rc(2) == -7
+        e.run(1)
+        (placed, deficit), = e.greedy([0], [5])
+        assert len(placed) == 5
+        o.ball_update(placed, 1)
+        assert deficit == o.uncovered()
+        assert np.array_equal(e.cnt(0), o.read_cnt())
