@@ -60,6 +60,7 @@ struct Cell {
   int slots = 0;
   long long tlen = 0;
   bool ball_ok = false;              // the table is exactly the metric ball
+  bool moved = false;                // cnt or gain changed since the last step
 };
 
 // one cell's code slices per first-group tile, computed on the device from
@@ -1023,6 +1024,7 @@ int dct_batch_run(long long h, int mode) {
   Batch *b = get(h);
   if (!b || !b->built) return -1;
   if (mode == 0 || mode == 1) {
+    for (Cell &c : b->cells) c.moved = false;
     const int rc = mode == 0 ? run_persistent(b) : run_per_pass(b);
     const int late = tma_fault_take();   // the launches have drained
     return rc ? rc : late;
@@ -1240,6 +1242,7 @@ int dct_batch_update(long long h, int cell, const long long *words, int nw,
   if (!c || !c->dtbl || (delta != 1 && delta != -1)) return -1;
   int rc = stage_cell_words(b, *c, words, nw);
   if (rc || !nw) return rc;
+  c->moved = true;
   rc = launch_update(cell_walk(*c), b->d_words, nullptr, nw, delta, nullptr,
                      b->stream);
   if (rc) return rc;
@@ -1456,6 +1459,9 @@ int dct_batch_greedy(long long h, const int *cells, int n, const int *max_add,
                        b->stream));
     ck(cudaEventRecord(b->ev_greedy[slot], b->stream));
   };
+  // A map that updates or an earlier greedy have left behind or ahead of cnt
+  // is never rebuilt: a transform would raise gains that the keys kept of its
+  // chunks bound, and bring back words that an earlier greedy took out.
   // While a placement of some cell may be worth a rebuild of its map, the
   // host follows the gains one step behind (the first step knows them from
   // the last launch) and the device stays busy; gains never grow, so after
@@ -1477,7 +1483,7 @@ int dct_batch_greedy(long long h, const int *cells, int n, const int *max_add,
         const bool done = issued ? h[k].done != 0 : st0[k].done != 0;
         const long long gain = issued ? h[k].gain(par ^ 1)
                                       : sc[3 * cells[k] + 1];
-        const int want = !done && c.ball_ok &&
+        const int want = !done && c.ball_ok && !c.moved &&
                          greedy_rebuild_pays(gain, c.tlen, c.gain_us);
         live = live || !done;
         any = any || want;
@@ -1520,6 +1526,7 @@ int dct_batch_greedy(long long h, const int *cells, int n, const int *max_add,
     if (all) break;
     chunk = std::min<long long>(chunk * 2, 512);
   }
+  for (int k = 0; k < n; k++) b->cells[cells[k]].moved = true;
   if (!rc) {
     read_states(0);
     ck(cudaStreamSynchronize(b->stream));

@@ -184,3 +184,36 @@ def test_a_table_that_is_not_the_ball_is_never_rebuilt(monkeypatch):
                         gain[y] -= 1
             assert len(got[i][0]) == steps
             assert np.array_equal(e.cnt(i), cnt.astype(np.uint16)), i
+
+
+@pytest.mark.parametrize("axes,R,mu", [((2,) * 11, 1, 2), ((3,) * 11, 2, 2),
+                                       ((2,) * 17, 2, 1)])
+def test_batched_greedy_from_a_moved_map_is_never_rebuilt(axes, R, mu,
+                                                          monkeypatch):
+    """A second greedy without a step between, and a greedy after words were
+    taken out: the gain map stays the last step's with the updates since, as
+    it is without rebuilds, and no word is placed twice."""
+    from coldcore_b200.batch import BatchEngine
+    from coldcore_b200.patterns import wide_table
+    size = int(np.prod(axes))
+    code = np.random.default_rng(size).choice(size, 40, replace=False)
+    got = []
+    for rebuild in ("0", "1"):
+        monkeypatch.setenv("CC_GREEDY_REBUILD", rebuild)
+        with BatchEngine() as e:
+            for _ in range(2):
+                e.add("hamming", axes, R, code, mu)
+            e.build(48)
+            for i in range(2):
+                e.set_table(i, wide_table(axes, R, "hamming"))
+            e.run()
+            e.update(1, code[:12], -1)
+            out = e.greedy([0, 1], [6, 6]) + e.greedy([0, 1], [5, 5])
+            words = np.concatenate([out[0][0], out[2][0]])
+            assert len(np.unique(words)) == len(words)
+            got.append([w.tolist() for w, _d in out] +
+                       [e.cnt(i).tolist() for i in range(2)])
+            e.run()                      # every field afresh: rebuilt again
+            (w0, _), = e.greedy([0], [6])
+            got[-1].append(w0.tolist())
+    assert got[0] == got[1]
