@@ -147,6 +147,7 @@ struct State {
   bool metric_table = false;       // support table proven == metric ball
   bool ball_ok = false;            // ... on a cell the set side takes
   bool set_ok = false;             // ... and the set side is on
+  bool metric_tbl2 = false;        // dct_set_tbl2's table is the ball too
   int set_policy = 1;              // DCT_SET_GATHER: 0 off, 1 auto, 2 force
   long long set_min = -1;          // DCT_SET_MIN: walk size that tries it
   long long set_ratio = 2;         // DCT_SET_RATIO: set side while |Z| <= r|B|
@@ -1099,12 +1100,14 @@ int gather_launch(int mode, int target, int nb, const long long *dw,
 // leave plane 0, the map, alone, and by the last launch they end before the
 // last plane.  So: a layered cell in device memory with R >= 3, a table that
 // is the metric ball (the walk's answer), 16-bit exactness, and no exact
-// layers of an earlier call in the planes.  Returns the plan, or nullptr.
+// layers of an earlier call in the planes.  (The table in use: dct_use_fmt's
+// second one may hold other patterns.)  Returns the plan, or nullptr.
 // An untuned cell takes the streamed forms without tuning (a tuning run
 // costs hundreds of such calls, and would write the map).
 Plan *gather_transform_plan() {
   if (S.streamed || S.layers_mode != 0 || S.cnt_mode != 0 || !S.ball_ok ||
-      S.layered_out || S.R1 < 4 || !half_planes_ok(kSrcCnt, kDstMap))
+      (S.fmt == 1 && !S.metric_tbl2) || S.layered_out || S.R1 < 4 ||
+      !half_planes_ok(kSrcCnt, kDstMap))
     return nullptr;
   Plan *P = nullptr;
   if (S.tuned[1][1] && S.plan_ok[1][1]) {
@@ -1342,6 +1345,7 @@ int dct_set_tbl2(const uint16_t *mask, const uint64_t *offs, long long len) {
   }
   if (S.tbl2) { cudaFree(S.tbl2); S.tbl2 = nullptr; }
   if (S.pk2) { cudaFree(S.pk2); S.pk2 = nullptr; }
+  S.metric_tbl2 = metric_ball_table(S.g, soa, w, S.len);
   return upload_table(soa, w, &S.tbl2, &S.slots2, &S.pk2);
 }
 
@@ -1618,8 +1622,10 @@ int greedy_fill_impl(int max_add, long long *placed, long long *deficit) {
   constexpr int32_t kExcluded = INT_MIN / 2;
   // At mu = 1, with a table that is the metric ball, an active word's whole
   // ball is covered: its gain is 0 and it is never placed.  Otherwise the
-  // active words are taken out of the map, after every transform of it.
-  const bool exclude = mu > 1 || !S.set_ok || S.fmt != 0;
+  // active words are taken out of the map, after every transform of it.  (A
+  // second table that is not the ball may have placed some of them.)
+  const bool exclude = mu > 1 || !S.set_ok || S.fmt != 0 ||
+                       (S.tbl2 && !S.metric_tbl2);
   std::vector<long long> code;
   if (exclude) {
     each_active([&](long long w, int) { code.push_back(w); });

@@ -2,10 +2,13 @@
 of candidates), with and without the predicate bit plane, against the
 oracle and against the per-word walk, for Hamming, Lee, torus and
 mixed-radix cells, mu = 1 and 2, every role."""
+import ctypes
+
 import numpy as np
 import pytest
 
 from coldcore_b200.gpu import GpuBackend
+from coldcore_b200.patterns import wide_table
 from oracle.dp_oracle import OracleBackend
 
 pytestmark = pytest.mark.gpu
@@ -71,3 +74,59 @@ def test_gather_by_transform_matches(monkeypatch, problem, axes, R, mu):
         at = b.layers_at(some)
         b.ball_gather(cands, 0)
         assert np.array_equal(b.layers_at(some), at)
+
+
+def second_table(b, tbl):
+    """dct_set_tbl2 from the rows of a wide table."""
+    mask = np.zeros(len(tbl), dtype=np.uint16)
+    offs = np.zeros(len(tbl), dtype=np.uint64)
+    for k in range(tbl.shape[1]):
+        pos, dl = tbl[:, k] >> 24, tbl[:, k] & 0xFFFFFF
+        used = dl > 0
+        mask[used] |= (1 << pos[used]).astype(np.uint16)
+        offs[used] |= dl[used].astype(np.uint64) << (
+            4 * pos[used]).astype(np.uint64)
+    p = ctypes.POINTER
+    assert b._lib.dct_set_tbl2(
+        mask.ctypes.data_as(p(ctypes.c_uint16)),
+        offs.ctypes.data_as(p(ctypes.c_uint64)), len(tbl)) == 0
+
+
+def test_second_table_of_other_patterns(monkeypatch):
+    """dct_use_fmt(1) with a table that is not the ball: large gathers answer
+    from that table as small ones do, and a greedy never places a word that
+    is active although the table did not cover it."""
+    monkeypatch.setenv("DCT_SET_GATHER", "0")
+    monkeypatch.setenv("CC_GATHER_TRANSFORM", "1")
+    axes, R = [3] * 9, 3
+    size = 3 ** 9
+    tbl = wide_table(axes, R, "hamming")
+    other = tbl.copy()
+    other[::3] = tbl[2]                  # pattern 0, the centre, too
+    rng = np.random.default_rng(9)
+    cands = rng.integers(0, size, 30000)
+    with GpuBackend(axes, R) as b:
+        second_table(b, other)
+        b.recount(rng.choice(size, 40, replace=False))
+        assert b._lib.dct_use_fmt(1) == 0
+        small = np.concatenate([b.ball_gather(cands[i:i + 6000], 0)
+                                for i in range(0, len(cands), 6000)])
+        assert np.array_equal(b.ball_gather(cands, 0), small)
+        assert b._lib.dct_use_fmt(0) == 0
+        assert not np.array_equal(b.ball_gather(cands, 0), small)
+    # word 0 is active, yet all but one word of its ball is uncovered
+    monkeypatch.setenv("DCT_SET_GATHER", "1")
+    axes, R = [3] * 6, 1
+    tbl = wide_table(axes, R, "hamming")
+    tbl[:] = tbl[2]
+    x = np.arange(3 ** 6)
+    weight = sum((x // 3 ** j % 3 != 0).astype(int) for j in range(6))
+    with GpuBackend(axes, R) as b:
+        second_table(b, tbl)
+        b.recount(x[weight >= 3])
+        assert b._lib.dct_use_fmt(1) == 0
+        b.ball_update([0], +1)
+        assert b._lib.dct_use_fmt(0) == 0
+        assert b.uncovered() == 12 == b.ball_gather([0], 0)[0]
+        placed, _ = b.greedy_fill_device(12)
+        assert len(placed) and 0 not in placed
