@@ -231,7 +231,8 @@ int tma_blocks_per_sm(const GroupPlan &p);
 int tma_fault_take();
 // Failures made on the host, for tests of the paths behind them
 // (dct_b200_fault_inject): true when this event of `kind` is the armed one.
-enum FaultKind { kFaultStreamed = 0, kFaultBarrier = 1, kFaultKinds = 2 };
+enum FaultKind { kFaultStreamed = 0, kFaultBarrier = 1, kFaultPinned = 2,
+                 kFaultKinds = 3 };
 bool fault_due(int kind);
 int launch_code_bounds(const long long *code, long long ncode,
                        long long tile_words, long long ntiles,

@@ -55,14 +55,18 @@ struct Plan {
 struct WordBuf {
   long long *p = nullptr;
   long long cap = 0, n = 0;
+  // room for m words; a refusal leaves the words that are there
   int reserve(long long m) {
     if (m <= cap) return 0;
-    if (p) cudaFreeHost(p);
-    p = nullptr;
     const long long want = std::max<long long>(m + m / 2, 1024);
-    cap = n = 0;
-    CC_CK(cudaHostAlloc((void **)&p, (size_t)want * 8, cudaHostAllocDefault));
+    if (fault_due(kFaultPinned))
+      return -(100 + (int)cudaErrorMemoryAllocation);
+    void *q = nullptr;
+    CC_CK(cudaHostAlloc(&q, (size_t)want * 8, cudaHostAllocDefault));
+    if (p) cudaFreeHost(p);
+    p = static_cast<long long *>(q);
     cap = want;
+    n = 0;
     return 0;
   }
   long long count(long long w) const {
@@ -1387,22 +1391,32 @@ int dct_set_code(const long long *idx, int M) {
     hist[1] = M;
   }
   if (!within_counter(M, max_mult(hist))) return -1;
-  if (M > S.code_cap) {
-    if (S.d_code) cudaFree(S.d_code);
-    S.d_code = nullptr;
-    const long long cap = std::max<long long>(M, 1024);
-    CC_CK(cudaMalloc(&S.d_code, (size_t)cap * 8));
-    S.code_cap = cap;
-  }
+  // all the room first: a call that is refused leaves the staged code, on the
+  // device and here, as it was
+  long long *room = nullptr;
+  const long long cap = std::max<long long>(M, 1024);
+  if (M > S.code_cap) CC_CK(cudaMalloc(&room, (size_t)cap * 8));
   // the buffer that does not hold the active multiset; a copy out of it may
   // still be on its way when the last call staged a code that no transform
   // has used since
-  if (S.code_in_flight) CC_CK(cudaStreamSynchronize(g_stream));
-  S.code_in_flight = false;
   const int to = S.act == S.up ? 1 - S.up : S.up;
   WordBuf &b = S.code_buf[to];
-  int rc = b.reserve(M);
-  if (rc) return rc;
+  int rc = 0;
+  if (S.code_in_flight) {
+    const cudaError_t e = cudaStreamSynchronize(g_stream);
+    if (e != cudaSuccess) rc = -(100 + (int)e);
+  }
+  if (!rc) rc = b.reserve(M);
+  if (rc) {
+    if (room) cudaFree(room);
+    return rc;
+  }
+  S.code_in_flight = false;
+  if (room) {
+    if (S.d_code) cudaFree(S.d_code);
+    S.d_code = room;
+    S.code_cap = cap;
+  }
   if (M) {
     memcpy(b.p, src, (size_t)M * 8);
     CC_CK(cudaMemcpyAsync(S.d_code, b.p, (size_t)M * 8,

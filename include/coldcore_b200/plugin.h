@@ -310,7 +310,8 @@ CCP_API int  dct_b200_read_layer(int d, long long off, long long len, int32_t *o
  * from the host (0 disarms; nothing fails on the device).  Kind 0: a streamed
  * launch reports that it timed out waiting for its tensor loads, so the call
  * that queued it returns -8.  Kind 1: a launch of dct_b200_greedy_fill reports
- * a time-out at its grid barrier. */
+ * a time-out at its grid barrier.  Kind 2: the pinned memory that a code is
+ * staged in is refused. */
 CCP_API int  dct_b200_fault_inject(int kind, int nth);
 
 /* ---- out-of-core (ooc) cells: distance layers in host memory ----

@@ -9,7 +9,7 @@ from oracle.dp_oracle import OracleBackend
 
 pytestmark = pytest.mark.gpu
 
-STREAMED, BARRIER = 0, 1                 # dct_b200_fault_inject kinds
+STREAMED, BARRIER, PINNED = 0, 1, 2      # dct_b200_fault_inject kinds
 
 
 @pytest.fixture
@@ -189,3 +189,29 @@ def test_an_error_of_an_earlier_step_is_not_a_greedys(rebuild, monkeypatch):
         o.ball_update(placed, 1)
         assert deficit == o.uncovered()
         assert np.array_equal(e.cnt(0), o.read_cnt())
+
+
+def test_a_code_that_is_refused_room_leaves_the_staged_one():
+    """A second, larger code whose pinned room is refused: the recount is of
+    the code staged before it, whose words can then be taken out."""
+    axes, R = [3] * 9, 2
+    rng = np.random.default_rng(3)
+    first, large = (rng.choice(3 ** 9, m, replace=False) for m in (30, 9000))
+    o = OracleBackend(axes, R)
+    with GpuBackend(axes, R) as b:
+        b.recount(rng.choice(3 ** 9, 50, replace=False))
+        b.stage_code(first)
+        b._lib.dct_b200_fault_inject(PINNED, 1)
+        with pytest.raises(RuntimeError):
+            b.stage_code(large)
+        assert b._lib.dct_transform(0, 2) == 0
+        o.recount(first)
+        assert np.array_equal(b.read_cnt(), o.read_cnt())
+        b.ball_update(first[:5], -1)
+        o.ball_update(first[:5], -1)
+        assert np.array_equal(b.read_cnt(), o.read_cnt())
+        with pytest.raises(RuntimeError):
+            b.ball_update(first[:1], -1)
+        b.recount(large)                 # with room it is staged
+        o.recount(large)
+        assert np.array_equal(b.read_cnt(), o.read_cnt())
