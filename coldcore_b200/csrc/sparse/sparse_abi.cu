@@ -707,20 +707,26 @@ double binom_d(int n, int r) {
   return x;
 }
 
-// Whether the design's fields run by levels: every rank and binomial of the
-// levels below 2^32, level values within 16 bits, and less work than the
-// rows.  A row entry costs 1.8 ps (C(30,8,4): 410 M entries in 738 us) and
-// a level read 1.0 ps, a level launch about 3 us more.
-bool use_levels() {
+// Whether the design's fields can run by levels: every rank and binomial of
+// the levels below 2^32, level values within 16 bits.
+bool levels_fit() {
   if (!C.dv || C.dt >= C.dk || C.dk > kLevelMaxK || C.lev_refused)
     return false;
+  for (int j = C.dt; j <= C.dk; j++)
+    if (binom_d(C.dv, j) >= 4.0e9) return false;
+  return binom_d(C.dk - 1, C.dt) <= 65535;
+}
+
+// ... and whether they are less work than the rows.  A row entry costs 1.8 ps
+// (C(30,8,4): 410 M entries in 738 us) and a level read 1.0 ps, a level
+// launch about 3 us more.  (CC_SPARSE_LEVELS: 0 the rows, 1 the levels
+// wherever they fit)
+bool use_levels() {
+  if (!levels_fit()) return false;
+  const char *e = getenv("CC_SPARSE_LEVELS");
+  if (e) return atoi(e) != 0;
   double reads = 0;
-  for (int j = C.dt; j <= C.dk; j++) {
-    const double n = binom_d(C.dv, j);
-    if (n >= 4.0e9) return false;
-    if (j > C.dt) reads += n * j;
-  }
-  if (binom_d(C.dk - 1, C.dt) > 65535) return false;
+  for (int j = C.dt + 1; j <= C.dk; j++) reads += binom_d(C.dv, j) * j;
   const double rows = (double)C.ncand * C.d;
   return 1.0e-6 * reads + 3.0 * (C.dk - C.dt) < 1.8e-6 * rows + 2.0;
 }

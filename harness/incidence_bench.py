@@ -1,21 +1,22 @@
 """Field throughput of the explicit-incidence engine on a covering design.
 
 One step = a gain field and a loss field over every candidate of C(v,k,t)
-(default C(30,8,4): 5,852,925 blocks x 70 triples, a 1.64 GB incidence,
-27,405 universe elements) after a recount of a seeded solution, the
-incidence built on the device.  Reported per field: milliseconds, and GB/s
-of its algorithmic bytes (the incidence read once, the map written once,
-cnt read once).  Given another ABI-2 library (``--ref PATH``, e.g. the
-reference's own ``src/plugins/sparse/sparse.cu`` built for sm_100a), its
+(default C(30,8,4): 5,852,925 blocks x 70 of the 27,405 four-subsets, a
+1.64 GB incidence) after a recount of a seeded solution, the incidence built
+on the device.  A design's fields run by subset-size levels and read no row,
+so ``GBps`` counts what a field cannot do without (cnt read once, the map
+written once).  The row form (``CC_SPARSE_LEVELS=0``, which reads the
+incidence) is timed beside it, under ``row_form``, and its gain field checked
+against the default form's.  Given another ABI-2 library (``--ref PATH``, e.g.
+the reference's own ``src/plugins/sparse/sparse.cu`` built for sm_100a), its
 kernels are timed in alternation on the same incidence.
 
     python -m harness.incidence_bench [--v 30 --k 8 --t 4 --reps 20]
                                             [--ref PATH] [--bits]
 
-The default row form tests one role bit per universe element in shared
-memory; ``--bits`` also times the counter form (``CC_SPARSE_BITS=0``: one
-counter read per row entry) and checks its gain field against the default
-form's (reported under ``counter_form``).
+The row form tests one role bit per universe element in shared memory;
+``--bits`` also times its counter form (``CC_SPARSE_BITS=0``: one counter read
+per row entry), under ``counter_form``.
 """
 import argparse
 import json
@@ -83,30 +84,33 @@ def measure(v=30, k=8, t=4, reps=20, rounds=3, ref_path=None,
                 if ref is not None:
                     theirs.append(_time_fields(ref, torch.cuda.default_stream(),
                                                reps))
-            # the same engine with one CTA wave per SM instead of four
-            os.environ["CC_SPARSE_BLOCKS_PER_SM"] = "8"
-            try:
-                _warm(b, 0.1)
-                one_wave = [_time_fields(b, stream, reps)
-                            for _ in range(rounds)]
-            finally:
-                os.environ.pop("CC_SPARSE_BLOCKS_PER_SM", None)
             b.gain_map()
             sample = np.arange(0, n_cand, 997)
             gain = b.map_read_at(sample)
-            bit_rounds = bits_same = None
-            if bits:
-                # the other row form: a counter read per row entry
-                os.environ["CC_SPARSE_BITS"] = "0"
+
+            def form(knobs):
+                """Rounds of the fields under `knobs`, and whether the gain
+                field is the default form's."""
+                os.environ.update(knobs)
                 try:
                     _warm(b, 0.1)
-                    bit_rounds = [_time_fields(b, stream, reps)
-                                  for _ in range(rounds)]
+                    times = [_time_fields(b, stream, reps)
+                             for _ in range(rounds)]
                     b.gain_map()
-                    bits_same = bool(np.array_equal(b.map_read_at(sample),
-                                                    gain))
+                    return times, bool(np.array_equal(b.map_read_at(sample),
+                                                      gain))
                 finally:
-                    os.environ.pop("CC_SPARSE_BITS", None)
+                    for k in knobs:
+                        os.environ.pop(k)
+
+            by_rows = {"CC_SPARSE_LEVELS": "0"}
+            row_rounds, row_same = form(by_rows)
+            # the row form with one CTA wave per SM instead of four
+            one_wave, _ = form({**by_rows, "CC_SPARSE_BLOCKS_PER_SM": "8"})
+            bit_rounds = bits_same = None
+            if bits:
+                bit_rounds, bits_same = form({**by_rows,
+                                              "CC_SPARSE_BITS": "0"})
             same = None
             if ref is not None:
                 ref.gain_map()
@@ -124,36 +128,39 @@ def measure(v=30, k=8, t=4, reps=20, rounds=3, ref_path=None,
         cpu_ms = (time.perf_counter() - t0) / 3 * 1e3
         cpu_same = bool(np.array_equal(out_map[sample], gain))
     ms = statistics.median(ours)
-    by = n_cand * (d + 1) * 4 + n_univ * 4
+    by = n_cand * 4 + n_univ * 4         # what a field cannot do without
+    row_by = by + n_cand * d * 4         # ... by rows: the incidence too
+
+    def row_line(times, same):
+        m = statistics.median(times)
+        return {"ms_per_field": round(m, 4),
+                "ms_rounds": [round(x, 4) for x in times],
+                "GBps": round(row_by / (m * 1e-3) / 1e9, 1),
+                "same_gain_sample": same}
+
     out.update({"n_cand": n_cand, "d": d, "n_univ": n_univ,
                 "incidence_gb": round(n_cand * d * 4 / 1e9, 3),
                 "solution": len(sol), "ms_per_field": round(ms, 4),
                 "ms_rounds": [round(x, 4) for x in ours],
-                "ms_rounds_8_ctas_per_sm": [round(x, 4) for x in one_wave],
                 "GBps": round(by / (ms * 1e-3) / 1e9, 1),
-                "algorithmic_bytes_per_field": by})
+                "algorithmic_bytes_per_field": by,
+                "row_form": row_line(row_rounds, row_same)})
+    out["row_form"]["bytes_per_field"] = row_by
+    out["row_form"]["ms_rounds_8_ctas_per_sm"] = [round(x, 4)
+                                                  for x in one_wave]
     if bit_rounds is not None:
-        bms = statistics.median(bit_rounds)
-        out["counter_form"] = {"ms_per_field": round(bms, 4),
-                            "ms_rounds": [round(x, 4) for x in bit_rounds],
-                            "GBps": round(by / (bms * 1e-3) / 1e9, 1),
-                            "same_gain_sample": bits_same}
+        out["counter_form"] = row_line(bit_rounds, bits_same)
     if cpu_ms is not None:
         out["cpu_baseline"] = {
-            "value": round(by / (cpu_ms * 1e-3) / 1e9, 2), "unit": "GB/s",
+            "value": round(row_by / (cpu_ms * 1e-3) / 1e9, 2), "unit": "GB/s",
             "cores": os.cpu_count(), "kind": "port",
             "sample": f"3 gain fields of {out['design']}, C restatement on "
                       f"all host threads, {cpu_ms:.1f} ms each",
             "same_gain_sample": cpu_same}
     if theirs:
-        rms = statistics.median(theirs)
         out["reference_plugin"] = {
-            "library": os.path.basename(ref_path),
-            "ms_per_field": round(rms, 4),
-            "ms_rounds": [round(x, 4) for x in theirs],
-            "GBps": round(by / (rms * 1e-3) / 1e9, 1),
-            "same_gain_sample": same,
-            "speedup": round(rms / ms, 2)}
+            "library": os.path.basename(ref_path), **row_line(theirs, same),
+            "speedup": round(statistics.median(theirs) / ms, 2)}
     return out
 
 
@@ -166,7 +173,7 @@ def main():
     ap.add_argument("--ref", default=None,
                     help="another ABI-2 library to time beside the engine")
     ap.add_argument("--bits", action="store_true",
-                    help="also time the counter form (CC_SPARSE_BITS=0)")
+                    help="also time the counter row form (CC_SPARSE_BITS=0)")
     a = ap.parse_args()
     print(json.dumps(measure(a.v, a.k, a.t, a.reps, ref_path=a.ref,
                              bits=a.bits)))

@@ -337,3 +337,41 @@ def test_design_fields_by_levels_against_the_rows(v, k, t):
             want.append(o.map.copy())
     for a, w in zip(got, want):
         assert np.array_equal(a, w)
+
+
+@pytest.mark.parametrize("v,k,t", [
+    (24, 6, 3), (18, 9, 4), (20, 12, 2), (23, 4, 3), (17, 16, 5), (26, 7, 1),
+    (12, 2, 1), (9, 8, 7), (40, 4, 2), (128, 2, 1), (128, 3, 2), (20, 13, 9),
+    (28, 6, 3)])
+def test_design_levels_where_they_fit(v, k, t, monkeypatch):
+    """CC_SPARSE_LEVELS=1 runs a design's fields by levels at sizes the rule
+    leaves to the rows (=0): one level to eleven, byte values and, above 255,
+    16-bit ones, last runs of every length, one level's sets in one thread."""
+    from coldcore_b200.incidence import GpuCoveringDesignBackend
+    rng = np.random.default_rng(v * k + t)
+    with GpuCoveringDesignBackend(v, k, t, mu=2) as b:
+        for m in (0, 1, max(2, b.n_univ // (2 * b.d)), b.n_cand // 3):
+            b.recount(rng.choice(b.n_cand, m, replace=False))
+            for fld in (b.gain_map, b.loss_map):
+                got = []
+                for form in ("1", "0"):
+                    monkeypatch.setenv("CC_SPARSE_LEVELS", form)
+                    fld()
+                    got.append(b.map_all())
+                assert np.array_equal(*got), (m, fld)
+
+
+def test_incidence_bench_times_the_forms_it_names():
+    """The bench's row and counter forms read the rows (the levels do not),
+    agree with the default form, and each rate is of its own bytes."""
+    from harness.incidence_bench import measure
+    r = measure(28, 6, 3, reps=2, rounds=1, bits=True)
+    n_cand, n_univ, d = 376740, 3276, 20
+    assert r["algorithmic_bytes_per_field"] == 4 * (n_cand + n_univ)
+    assert r["row_form"]["bytes_per_field"] == 4 * (n_cand * (d + 1) + n_univ)
+    for form in ("row_form", "counter_form"):
+        assert r[form]["same_gain_sample"]
+        assert r[form]["GBps"] * r[form]["ms_per_field"] == pytest.approx(
+            4 * (n_cand * (d + 1) + n_univ) / 1e6, rel=0.02)
+    assert r["GBps"] * r["ms_per_field"] == pytest.approx(
+        4 * (n_cand + n_univ) / 1e6, rel=0.02)
