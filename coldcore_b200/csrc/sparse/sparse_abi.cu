@@ -68,8 +68,8 @@ struct Cell {
   int32_t *xval = nullptr;
   int xcap = 0;
   uint32_t *bits = nullptr;        // role bit per universe element
-  // covering designs: C(v,k,t), the level form's binomials and its two level
-  // buffers (allocated by the first field that runs by levels)
+  // covering designs: C(v,k,t), and where its fields run by levels the
+  // binomials and two level buffers
   int dv = 0, dk = 0, dt = 0;
   uint32_t *binom32 = nullptr;
   void *lev[2] = {nullptr, nullptr};
@@ -776,42 +776,50 @@ int run_levels(int target, int32_t *out) {
   return 0;
 }
 
-// the design's field into the map by levels; 1 when its buffers do not fit
-// (the caller reads the rows instead)
-int field_levels(int target) {
-  const bool wide = binom_d(C.dk - 1, C.dt) > 255;
-  if (!C.lev[0]) {
-    double most = 0;
-    for (int j = C.dt; j < C.dk; j++) most = std::max(most, binom_d(C.dv, j));
-    const size_t bytes = ((size_t)(most + 0.5) * (wide ? 2 : 1) + 31) / 16 * 16;
-    const int V1 = C.dv + 1, K1 = C.dk + 1;
-    std::vector<uint32_t> B((size_t)V1 * K1, 0);
-    for (int b = 0; b < K1; b++)
-      for (int a = b; a < V1; a++) {
-        const double x = binom_d(a, b);
-        B[(size_t)b * V1 + a] = x >= 4294967295.0 ? 0xffffffffu
-                                                  : (uint32_t)(x + 0.5);
-      }
-    void *p = nullptr, *q = nullptr, *r = nullptr;
-    if (cudaMalloc(&p, bytes) != cudaSuccess ||
-        cudaMalloc(&q, bytes) != cudaSuccess ||
-        cudaMalloc(&r, B.size() * 4) != cudaSuccess) {
-      cudaGetLastError();
-      if (p) cudaFree(p);
-      if (q) cudaFree(q);
-      C.lev_refused = true;
-      return 1;
+// whether the level values need 16 bits
+bool wide_levels() { return binom_d(C.dk - 1, C.dt) > 255; }
+
+// The level buffers and the binomials of a design whose fields run by
+// levels: got at init, with the cell's other memory, so that its count is
+// whole.  Where they do not fit the fields read the rows.
+int alloc_levels() {
+  if (C.lev[0] || !use_levels()) return 0;
+  double most = 0;
+  for (int j = C.dt; j < C.dk; j++) most = std::max(most, binom_d(C.dv, j));
+  const size_t bytes =
+      ((size_t)(most + 0.5) * (wide_levels() ? 2 : 1) + 31) / 16 * 16;
+  const int V1 = C.dv + 1, K1 = C.dk + 1;
+  std::vector<uint32_t> B((size_t)V1 * K1, 0);
+  for (int b = 0; b < K1; b++)
+    for (int a = b; a < V1; a++) {
+      const double x = binom_d(a, b);
+      B[(size_t)b * V1 + a] = x >= 4294967295.0 ? 0xffffffffu
+                                                : (uint32_t)(x + 0.5);
     }
-    C.lev[0] = p;
-    C.lev[1] = q;
-    C.binom32 = static_cast<uint32_t *>(r);
-    C.dev_bytes += 2 * (long long)bytes + (long long)B.size() * 4;
-    SK(cudaMemcpyAsync(C.binom32, B.data(), B.size() * 4,
-                       cudaMemcpyHostToDevice, g_s));
-    SK(cudaStreamSynchronize(g_s));          // B lives on this frame
+  void *p = nullptr, *q = nullptr, *r = nullptr;
+  if (cudaMalloc(&p, bytes) != cudaSuccess ||
+      cudaMalloc(&q, bytes) != cudaSuccess ||
+      cudaMalloc(&r, B.size() * 4) != cudaSuccess) {
+    cudaGetLastError();
+    if (p) cudaFree(p);
+    if (q) cudaFree(q);
+    C.lev_refused = true;
+    return 0;
   }
-  return wide ? run_levels<uint16_t>(target, C.map)
-              : run_levels<uint8_t>(target, C.map);
+  C.lev[0] = p;
+  C.lev[1] = q;
+  C.binom32 = static_cast<uint32_t *>(r);
+  C.dev_bytes += 2 * (long long)bytes + (long long)B.size() * 4;
+  SK(cudaMemcpyAsync(C.binom32, B.data(), B.size() * 4,
+                     cudaMemcpyHostToDevice, g_s));
+  SK(cudaStreamSynchronize(g_s));            // B lives on this frame
+  return 0;
+}
+
+// the design's field into the map by levels
+int field_levels(int target) {
+  return wide_levels() ? run_levels<uint16_t>(target, C.map)
+                       : run_levels<uint8_t>(target, C.map);
 }
 
 }  // namespace
@@ -970,6 +978,7 @@ int sparse_b200_init_design(int v, int k, int t, int inc_mode,
   C.dv = v;
   C.dk = k;
   C.dt = t;
+  if ((rc = alloc_levels())) goto fail;
   if (bytes_dev) *bytes_dev = C.dev_bytes;
   if (bytes_host) *bytes_host = C.host_bytes;
   return 0;
@@ -1019,8 +1028,11 @@ int sparse_recount(const long long *idx, long long m) {
 
 int sparse_field(int target) {
   if (!C.live) return -1;
-  int rc = use_levels() ? field_levels(target) : 1;
-  if (rc == 1) rc = launch_rows(nullptr, C.ncand, target, C.map);
+  int rc = alloc_levels();           // CC_SPARSE_LEVELS=1 set since init
+  if (rc) return rc;
+  rc = C.lev[0] && use_levels()
+           ? field_levels(target)
+           : launch_rows(nullptr, C.ncand, target, C.map);
   if (rc) return rc;
   SK(cudaStreamSynchronize(g_s));
   return 0;

@@ -375,3 +375,18 @@ def test_incidence_bench_times_the_forms_it_names():
             4 * (n_cand * (d + 1) + n_univ) / 1e6, rel=0.02)
     assert r["GBps"] * r["ms_per_field"] == pytest.approx(
         4 * (n_cand + n_univ) / 1e6, rel=0.02)
+
+
+@pytest.mark.parametrize("v,k,t", [(24, 6, 3), (20, 12, 2), (28, 6, 3)])
+def test_a_designs_device_bytes_are_whole_after_init(v, k, t, monkeypatch):
+    """What init reports holds the buffers its fields run on: a field by
+    levels allocates nothing more."""
+    from coldcore_b200.incidence import GpuCoveringDesignBackend
+    if (v, k, t) != (28, 6, 3):          # that one runs by levels unasked
+        monkeypatch.setenv("CC_SPARSE_LEVELS", "1")
+    with GpuCoveringDesignBackend(v, k, t) as b:
+        total = b._lib.sparse_dev_bytes()
+        assert total > 4 * b.n_cand * (b.d + 1)
+        for fld in (b.gain_map, b.loss_map):
+            fld()
+            assert b._lib.sparse_dev_bytes() == total
