@@ -695,6 +695,14 @@ constexpr int kRunThreads = 256;
 constexpr int kRunWarps = kRunThreads / 32;
 constexpr int kRunPat = 128;            // patterns of one refresh piece
 constexpr int kRunTable = 8192;         // packed patterns kept in shared memory
+// k_greedy_run's static shared memory (rounded up) with the longest table: it
+// runs without an opt-in, so the sum stays within what every launch may use
+constexpr size_t kRunStatic = kMaxPackOff * sizeof(int4) +
+                              kRunWarps * sizeof(WalkSmem) +
+                              (kRunWarps + kRunThreads) * 8 +
+                              (kRunThreads + 1) * 4 + 128;
+static_assert(kRunStatic + kRunTable * 4 <= 48 * 1024,
+              "the persistent greedy's shared memory");
 
 // one warp's form of word_setup
 template <int WALK>
