@@ -217,3 +217,28 @@ def test_batched_greedy_from_a_moved_map_is_never_rebuilt(axes, R, mu,
             (w0, _), = e.greedy([0], [6])
             got[-1].append(w0.tolist())
     assert got[0] == got[1]
+
+
+@pytest.mark.parametrize("axes,R,mu", [((3,) * 11, 2, 2), ((4,) * 8, 2, 2),
+                                       ((2,) * 17, 3, 3)])
+def test_batched_rebuilds_of_a_large_cell(axes, R, mu, monkeypatch):
+    """Cells with launches of their own, mu above 1: a rebuild after every
+    placement, incumbents and placed words with gains left to them."""
+    from coldcore_b200.batch import BatchEngine
+    from coldcore_b200.patterns import wide_table
+    monkeypatch.setenv("CC_GREEDY_REBUILD", "1")
+    size = int(np.prod(axes))
+    code = np.random.default_rng(size).choice(size, size // 900,
+                                              replace=False)
+    ob = OracleBackend(list(axes), R, mu=mu)
+    ob.recount(code)
+    want, wdef = exact_greedy(ob, code, 6)
+    with BatchEngine() as e:
+        e.add("hamming", axes, R, code, mu)
+        e.build(48)
+        e.set_table(0, wide_table(axes, R, "hamming"))
+        e.run()
+        (placed, deficit), = e.greedy([0], [6])
+        assert placed.tolist() == want.tolist()
+        assert deficit == wdef
+        assert np.array_equal(e.cnt(0), ob.cnt.astype(np.uint16))

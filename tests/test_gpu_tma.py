@@ -263,3 +263,51 @@ def test_padded_ternary_plan_of_three_layers(monkeypatch, n, mu, kb):
             getattr(o, field)()
             assert np.array_equal(b.map_all(), o.map), field
         assert b.plan_forms(1, 1)[0] & TMA
+
+
+@pytest.mark.parametrize("axes,R,kb", [
+    ([4] * 11, 3, 0), ([4] * 11, 3, 100), ([5] * 10, 2, 0), ([6] * 9, 3, 0),
+    ([3] * 14, 3, 0), ([3] * 15, 2, 0)])
+def test_repeated_recounts_and_gains_of_row_pair_groups(monkeypatch, axes, R,
+                                                        kb):
+    """Tuned plans (kb 0) and one pinned to six-axis rows, in one process:
+    every recount and gain of two alternating codes is the oracle's, time
+    after time, with another transform between."""
+    from oracle.cport import CPortCell
+    if kb:
+        monkeypatch.setenv("CC_TMA", "1")
+        monkeypatch.setenv("CC_SMEM_BUDGET_KB", str(kb))
+    size = int(np.prod(axes))
+    rng = np.random.default_rng(size % 1009)
+    codes = [rng.choice(size, size // d, replace=False) for d in (900, 250)]
+    want = []
+    for code in codes:
+        o = CPortCell(axes, R)
+        o.recount(code)
+        o.gain_map()
+        want.append((o.cnt.copy(), o.map.copy()))
+    with GpuBackend(axes, R) as b:
+        for i in range(12):
+            cnt, gain = want[i & 1]
+            b.recount(codes[i & 1])
+            if i % 3 == 2:
+                b.loss_map()
+            assert np.array_equal(b.read_cnt(), cnt), i
+            b.gain_map()
+            assert np.array_equal(b.map_all(), gain), i
+
+
+@pytest.mark.parametrize("problem,q,n,R", [
+    ("hamming", 4, 9, 2), ("hamming", 5, 7, 3), ("hamming", 6, 7, 4),
+    ("lee", 4, 9, 3), ("lee", 5, 7, 2), ("lee", 6, 6, 4), ("lee", 7, 6, 3),
+    ("hamming", 4, 9, 1), ("lee", 4, 9, 1)])
+def test_cells_of_larger_axes_that_stream(monkeypatch, problem, q, n, R):
+    """Which of these cells' plans stream, each for itself: all, also at
+    R = 1 where the rows (4^5 or 4^6 words) need no padding."""
+    monkeypatch.setenv("CC_TMA", "1")
+    monkeypatch.setenv("CC_TUNE", "0")
+    monkeypatch.setenv("CC_SMEM_BUDGET_KB", "100")
+    with GpuBackend([q] * n, R, problem=problem) as b:
+        for im, om in ((0, 2), (1, 1), (2, 1)):
+            forms = b.plan_forms(im, om)
+            assert np.count_nonzero(forms & TMA) >= 1, (im, om, forms)
