@@ -41,7 +41,13 @@ namespace {
 
 constexpr long long kCounterMax = 65535;    // uint16 cnt
 constexpr long long kStageCap = 1 << 16;    // words per staged chunk
-constexpr long long kExtFirst = 1 << 15;    // extracted entries in one go
+// Extracted entries that come back with their count, through pinned memory;
+// the rest take a second wait and a copy into the caller's pageable arrays.
+// On K_3(14,3)'s map (4.8 M words), us a call with room for 2^12 / 2^15 /
+// 2^16 entries: one found 47 / 51 / 55, 10,097 found 98 / 68 / 74, 30,290
+// found 153 / 96 / 101, 60,076 found 282 / 241 / 178.  A doubling from 2^15
+// costs every small answer as much again as all the room up to there.
+constexpr long long kExtFirst = 1 << 15;
 constexpr int kGreedyRing = 2;              // steps whose states are in flight
 
 struct Plan {
