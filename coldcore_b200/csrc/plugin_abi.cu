@@ -148,7 +148,7 @@ struct State {
   std::unordered_map<long long, int> delta;
   long long active_size = 0;
   MultHist up_hist, act_hist;      // distinct words per multiplicity
-  long long stats[8] = {0};
+  long long stats[9] = {0};
   long long bytes_dev = 0, bytes_host = 0;
   unsigned long long dd_last = 0;
   bool torn = false;               // a call failed while it changed cnt
@@ -1192,6 +1192,7 @@ int gather_impl(const long long *words, int nwords, int mode, int target,
   }
   if (counts) {
     S.stats[1] += (nwords + kStageCap - 1) / kStageCap;
+    S.stats[8]++;
     const int rc = staged_words(
         words, nwords, out, [&](const long long *w, int nb, int32_t *o) {
           return launch_read_at(counts, w, nb, o, g_stream);
@@ -1848,7 +1849,7 @@ int dct_loss_owner(const long long *words, int M, int32_t *out) {
 }
 
 int dct_stats(long long *out, int n) {
-  if (n > 8) n = 8;
+  if (n > 9) n = 9;
   for (int i = 0; i < n; i++) out[i] = S.stats[i];
   return n < 0 ? 0 : n;
 }

@@ -516,11 +516,11 @@ class GpuBackend:
         return out
 
     def gpu_stats(self):
-        buf = (_LL * 8)()
-        self._lib.dct_stats(buf, 8)
+        buf = (_LL * 9)()
+        self._lib.dct_stats(buf, 9)
         keys = ("gather_set_side", "gather_walk", "set_scans",
                 "set_overflows", "swap_eval_fast", "swap_eval_fallback",
-                "count_eq0_listed", "gather_set_tiled")
+                "count_eq0_listed", "gather_set_tiled", "gather_transform")
         return {k: int(v) for k, v in zip(keys, buf)}
 
     # ---------------- queries

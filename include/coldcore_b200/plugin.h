@@ -106,7 +106,9 @@ CCP_API int  dct_swap_eval(const long long *drops, int k, const long long *cand,
 /* plugin.h:116; dct_hc.cu:779-783 — counters: [0] gathers served by the
  * set side, [1] by the walk, [2] predicate-set scans, [3] scans that
  * overflowed, [4] swap_eval fast path, [5] swap_eval fallback, [6]
- * count_eq(0) answered by the listing pass, [7] tiled set gathers */
+ * count_eq(0) answered by the listing pass, [7] tiled set gathers.
+ * Additive: [8] calls, counted under [1], that one transform answered in
+ * place of the walk */
 CCP_API int  dct_stats(long long *out, int n);
 
 /* ---- reductions / map queries ---- */

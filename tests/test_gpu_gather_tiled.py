@@ -130,3 +130,48 @@ def test_second_table_of_other_patterns(monkeypatch):
         assert b.uncovered() == 12 == b.ball_gather([0], 0)[0]
         placed, _ = b.greedy_fill_device(12)
         assert len(placed) and 0 not in placed
+
+
+@pytest.mark.parametrize("problem,axes,R,mu,tuned,transform", [
+    ("hamming", [3] * 12, 4, 1, False, True),      # padded, streamed
+    ("hamming", [3] * 13, 4, 2, False, True),
+    ("hamming", [4] * 9, 4, 1, False, True),
+    ("hamming", [5] * 8, 4, 2, False, True),
+    ("lee", [7] * 6, 4, 1, False, True),
+    ("hamming", [2] * 16, 3, 1, False, True),      # streamed, unpadded
+    ("hamming", [2] * 18, 3, 1, False, False),     # more than 16 axes
+    ("hamming", [3] * 14, 4, 1, True, True),       # tuned, its map redirected
+    ("hamming", [4] * 11, 3, 2, True, None),       # whichever plan won
+    ("hamming", [3] * 11, 3, 1, False, False),     # pitched planes too wide
+    ("hamming", [3] * 12, 2, 1, False, False),     # three layers: no room
+])
+def test_which_large_gathers_one_transform_answers(monkeypatch, problem, axes,
+                                                   R, mu, tuned, transform):
+    """The route of a large gather (gpu_stats) and its counts: straight after
+    a recount, on the plan made for it, or on the tuned plan of an earlier
+    gain map, which stays as it was."""
+    from oracle.cport import CPortCell
+    monkeypatch.setenv("CC_GATHER_TRANSFORM", "1")
+    monkeypatch.setenv("DCT_SET_GATHER", "0")
+    size = int(np.prod(axes))
+    rng = np.random.default_rng(len(axes) + R)
+    code = rng.choice(size, size // 700, replace=False)
+    o = CPortCell(axes, R, problem, mu=mu)
+    o.recount(code)
+    o.gain_map()
+    gain = o.map.copy()
+    o.loss_map()
+    cands = rng.integers(0, size, 70001)
+    with GpuBackend(axes, R, problem=problem, mu=mu) as b:
+        b.recount(code)
+        if tuned:
+            b.gain_map()
+        for role, want in ((0, gain), (1, o.map)):
+            before = b.gpu_stats()["gather_transform"]
+            assert np.array_equal(b.ball_gather(cands, role), want[cands])
+            if transform is not None:
+                used = b.gpu_stats()["gather_transform"] - before
+                assert used == (1 if transform else 0)
+        if tuned:
+            assert np.array_equal(b.map_all(), gain)
+        assert np.array_equal(b.read_cnt(), o.cnt)
