@@ -1,6 +1,6 @@
 // batch.cu — the batched campaign engine: many independent cells (Hamming,
 // Lee, torus, grid; any sizes) resident at once, and their count, gain and
-// loss transforms run as ONE persistent launch captured in a CUDA graph.
+// loss transforms run as one graph of persistent launches.
 //
 // The reference runs a campaign as one process per cell, each with its own
 // singleton plugin context (coldcore src/coldcore/campaign.py:186-221,
@@ -9,9 +9,11 @@
 // each cell's transforms are split into passes (one per axis group) and
 // passes into tiles, and the whole step — for every cell: recount from its
 // code, the uncovered/deficit count, gain map + maximum, loss map + maximum
-// — is one launch of batch_kernel (transform_group.cu) over a level-ordered
-// work table.  Handles, not the v1 singleton: batches never touch the
-// dct_* cell.
+// — is one CUDA graph: a persistent launch per register kernel over a
+// level-ordered work table (batch_groups.cu), one of batch_kernel
+// (transform_group.cu) for the cells without such a kernel, and the big
+// cells' own launches, on forked streams.  Handles, not the v1 singleton:
+// batches never touch the dct_* cell.
 //
 // Tile size is the one schedule knob (shared memory per tile); the
 // autotuner times a few and keeps the fastest.
@@ -299,7 +301,6 @@ void release(Batch *b) {
   b->built = false;
 }
 
-// passes + level-ordered work table for the current tile budget
 // Per-launch tuning of the cells with their own launches, as the singleton
 // tunes its plan: every variant group_variants offers for a launch (register
 // block, row width, prefetching, streamed form, CTA width) is timed on the
@@ -368,6 +369,7 @@ int tune_big_cells(Batch *b) {
   return rc;
 }
 
+// passes + level-ordered work table for the current tile budget
 int make_schedule(Batch *b) {
   b->passes.clear();
   b->dep.clear();
@@ -838,7 +840,7 @@ int run_persistent(Batch *b) {
 }
 
 // The same step as one launch per pass: every big cell's own launches on
-// the same four side streams as the graph, every small cell's passes as
+// the same side streams as the graph, every small cell's passes as
 // one launch each of the same tile code on the main stream, no host wait
 // until the end.  Only the launch structure differs from the persistent
 // graph launch, which is what the comparison measures.

@@ -50,7 +50,7 @@ struct MlpSmem {
   __nv_bfloat16 h1[kRows * kLdH];    // then dz1
   __nv_bfloat16 h2[kRows * kLdH];    // then dz2
   float b1[kHid], b2[kHid], w3[kHid];
-  float y[kRows], dy[kRows];
+  float dy[kRows];
   float b3;
 };
 

@@ -339,8 +339,9 @@ int pad_max_axes(int prob, int q) {
 // byte boundaries and run as streamed launches over packed pairs; the last
 // writes the map or cnt back at the canonical index.  The axes after the
 // first group are split evenly into groups of at most pad_max_axes, and the
-// first group takes the packed row-pair form where it applies.  false when the cell does not qualify or
-// the padded planes do not fit the room16 u16 words of the allocation.
+// first group takes the packed row-pair form where it applies.  false when
+// the cell does not qualify or the padded planes do not fit the room16 u16
+// words of the allocation.
 bool pad_plan(std::vector<GroupPlan> &groups, const Geometry &g,
               const PlanPtrs &ptr, int dst, int R1, long long room16) {
   if (groups.size() < 2 || (g.prob != kHamming && g.prob != kLee))

@@ -471,10 +471,11 @@ size_t tma_smem_bytes(int q, int k, int r1, int lanes, int stages,
   return (size_t)stages * words * 4 + 1024 + kTmaMaxStages * 8 + 16;
 }
 
-// The groups the streamed form serves: Hamming (q <= 6) and Lee (q <= 7) groups
-// over 16-bit planes in packed pairs (an even inner stride), 16-bit planes, the
-// map or cnt out, one tile per W inner words x the whole group, an instantiated (q, k,
-// layers, lanes) and its stages within 227 KB of shared memory.
+// The groups the streamed form serves: Hamming (q <= 6) and Lee (q <= 7)
+// groups over 16-bit planes in packed pairs (an even inner stride), 16-bit
+// planes, the map or cnt out, one tile per W inner words x the whole group, an
+// instantiated (q, k, layers, lanes) and its stages within 227 KB of shared
+// memory.
 bool tma_group_ok(const GroupArgs &a, int q, int r1, int lanes, int stages) {
   // one stage: a CTA small enough for two a SM, whose loads then overlap
   // the other CTA's rounds

@@ -431,9 +431,10 @@ struct GreedyState {
 static_assert(sizeof(GreedyState) == kGreedyStateBytes, "state layout");
 
 constexpr int kChunk = kGreedyChunk;
-// updates a refresh makes in a microsecond, against a transform of the cell:
-// 90,000 on K_3(14,3) (487 K of them in 5.4 us), fewer on maps that pass the
-// L2.  64 mixed cells of up to 16.8 M words take 14.9 ms at any line from
+// Updates a refresh makes in a microsecond, against a transform of the cell:
+// 90,000 on K_3(14,3) (487 K of them in 5.4 us), whose map stays in L2, fewer
+// on maps that pass it.  One line serves both because neither side is steep
+// there: 64 mixed cells of up to 16.8 M words take 14.9 ms at any line from
 // 36,000 to 90,000, and 24.7 ms at 130,000.
 constexpr double kGreedyUpdatesPerUs = 36000.0;
 constexpr int kBlockChunks = kGreedyBlockChunks;
@@ -936,7 +937,6 @@ int launch_greedy_exclude(const BatchGreedyCell *dcells, int ncells,
   return 0;
 }
 
-// blocks per word so that single-word walks still fill the GPU
 // ------------------------------------------------------------ tiled gather
 // Many candidates over a large ball: the per-word kernel above re-reads the
 // whole support table for every candidate (|B| x slots x 4 bytes, 546 KB a
@@ -1115,6 +1115,7 @@ bool gather_bits_pay(const WalkArgs &w, int nb) {
   return (double)nb * (double)w.len >= (double)w.g.space;
 }
 
+// blocks per word so that single-word walks still fill the GPU
 int pick_split(long long len, int nb) {
   long long cover = (len + 255) / 256;
   long long split = (long long)sm_count() * 64 / (nb > 0 ? nb : 1);

@@ -186,7 +186,7 @@ CCP_API int  dct_b200_read_map(long long off, long long len, int32_t *out);
  * uint16 bound min(occurrences, max multiplicity x |B|) <= 65,535) and
  * computes, for every cell, cnt from its code, the deficit
  * sum max(0, mu - cnt), the gain map and its maximum and the loss map and
- * its maximum in ONE persistent launch replayed from a CUDA graph.  Handles
+ * its maximum, as persistent launches replayed from one CUDA graph.  Handles
  * are independent of the dct_* singleton cell. ---- */
 CCP_API long long dct_batch_create(void);
 /* returns the cell index, or a negative error */
@@ -230,7 +230,8 @@ CCP_API long long dct_batch_extract(long long h, int cell, int field,
                                    int cap);
 /* Exact greedy on n listed cells at once, one argmax / place / refresh
  * launch per step for all of them: from each cell's gain map as the last
- * launch left it (no update since), code words excluded, place the word of
+ * launch left it (updates and greedies since then leave it behind cnt: it is
+ * taken as it is), code words excluded, place the word of
  * largest gain (ties: smallest index) until the deficit is 0, nothing
  * gains, or max_add[k] (<= cap) words are placed; the same rule as
  * dct_b200_greedy_fill.  placed_out: cap words per listed cell. */
