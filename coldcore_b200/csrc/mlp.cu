@@ -374,10 +374,10 @@ long long dct_mlp_create(unsigned long long seed) {
   for (int i = 0; i < kIn * kHid; i++) p[kW1 + i] = uni(sqrtf(6.f / kIn));
   for (int i = 0; i < kHid * kHid; i++) p[kW2 + i] = uni(sqrtf(6.f / kHid));
   for (int i = 0; i < kHid; i++) p[kW3 + i] = uni(sqrtf(6.f / kHid) * 0.5f);
-  cudaMemcpy(m->P, p.data(), kParams * 4, cudaMemcpyHostToDevice);
-  cudaMemset(m->G, 0, kParams * 4);
-  cudaMemset(m->M, 0, kParams * 4);
-  cudaMemset(m->V, 0, kParams * 4);
+  // on the net's own stream, which does not wait for the default one
+  cudaMemcpyAsync(m->P, p.data(), kParams * 4, cudaMemcpyHostToDevice, m->s);
+  for (float *z : {m->G, m->M, m->V})
+    cudaMemsetAsync(z, 0, kParams * 4, m->s);
   k_refresh_bf16<<<(kHid * kHid + 255) / 256, 256, 0, m->s>>>(m->P, m->w1b,
                                                              m->w2b);
   cudaStreamSynchronize(m->s);

@@ -45,3 +45,20 @@ def test_training_fits_a_rule():
         l1 = mo.loss(m.params(), Xv, Tv)
         acc = ((m.predict(Xv) > 0) == (Tv > 0.5)).mean()
     assert l1 < 0.5 * l0 and acc > 0.9, (l0, l1, acc)
+
+
+def test_fresh_nets_score_and_step_from_their_own_weights():
+    """Nets made one after another: the scores of each are those of its
+    parameters set again, and a first Adam step starts from zero moments."""
+    rng = np.random.default_rng(5)
+    X = rng.random((64, 32)).astype(np.float32)
+    T = (rng.random(64) < 0.3).astype(np.float32)
+    for seed in range(20):
+        with GpuMlp(seed=seed) as a, GpuMlp(seed=99) as b:
+            first = a.predict(X)
+            p = a.params()
+            b.set_params(p)
+            assert np.array_equal(first, b.predict(X))
+            a.train(X, T, epochs=1, batch=64, lr=1e-3)
+            # m / c1 over sqrt(v / c2) is the gradient's sign: at most lr
+            assert np.abs(a.params() - p).max() <= 1e-3 * (1 + 1e-3)
